@@ -148,20 +148,13 @@ int zc_reserve(zc_ctx *ctx, uint32_t block_log, uint32_t nb);
  *                   (11..15), so a match nearer than that reads shared instead of global memory
  *   fill_warps      decoder fill: blocks (warps) per CTA, 1, 2, 4 or 8; fill_warps * (2^fill_ring_log +
  *                   1408 * fill_words) bytes of shared memory per CTA, at most 227 KiB
- *   match_cap       encoder match pass: bytes compared per candidate before the match is left to the
- *                   parse to finish, 8..32
- *   match_tile      encoder match pass: sorted positions per CTA of 256 threads (256, 512 or 1024)
  *   fill_words      decoder fill: output words each lane fills per round (1, 2 or 4: rounds of 128,
  *                   256 or 512 bytes, whose loads are in flight together)
- *   match_dense     encoder match pass: a tile with at least this many positions that their nearest
- *                   candidate does not decide scans a lane per position, a tile with fewer a 16-lane group
- *                   per position, a candidate a lane (0..1025; 1025: always groups, except at level 1)
- *   match_defer     encoder match pass: a position whose nearest candidate's match also covers the
- *                   match_defer bytes before it lies inside a longer match and is left to the parse to
- *                   finish only if it lands there (0..4; 0: never; 3 by default: 2 is faster on data
- *                   with long matches, 3-4 on text-like data whose parse lands on such positions more)
+ *   match_cap (8..32), match_tile (256, 512 or 1024), match_dense (0..1025), match_defer (0..4)
+ *                   kept and checked, without effect: they shaped a match pass that compared every position's
+ *                   candidates; the parse now computes matches where it needs them
  * The decoder uses the shape of the level last given to zc_prepare (5 by default).  zc_autotune times
- * the candidates on a host sample (its whole blocks, up to one encoder launch) and keeps the fastest for
+ * the fill's candidates on a host sample (its whole blocks, up to one encoder launch) and keeps the fastest for
  * (block_log, level); it allocates its own device buffers for the duration of the call. */
 typedef struct zc_shape {
   uint32_t fill_ring_log, fill_warps, match_cap, match_tile, fill_words, match_dense, match_defer;

@@ -1,0 +1,79 @@
+"""The parse's finishing of matches (warp_finish) and its split into segments and walks, at the sizes where they can
+go wrong: match lengths on both sides of the 16- and 32-byte compares, the 64-byte extension steps and the longest
+match, equal lengths at several distances, chains longer than the depth, and launches that take each segment
+count.  Every comparison is of whole payloads, byte for byte."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def codec():
+    import zero_cuda as Z
+    with Z.CudaCodec(level=5) as c:
+        yield c
+
+
+def lengths(rng):
+    """Copies of one source cut to every length where a compare ends, each followed by fresh bytes."""
+    src = rng.integers(0, 256, 9000, dtype=np.uint8)
+    parts = []
+    for n in (3, 4, 5, 15, 16, 17, 31, 32, 33, 47, 48, 63, 64, 65, 95, 96, 97, 127, 128, 129, 160, 4095, 4096, 4097, 8192):
+        parts += [src[:n], rng.integers(0, 256, 7, dtype=np.uint8)]
+    return np.concatenate([src] + parts * 2)
+
+
+def rows(rng):
+    """Lines that share long prefixes and differ late: many long candidates, equal lengths at several distances."""
+    base = rng.integers(97, 123, 500, dtype=np.uint8)
+    out = []
+    for _ in range(260):
+        b = base[: int(rng.integers(5, 500))].copy()
+        b[int(rng.integers(3, b.size)):][:1] ^= 1
+        out.append(b)
+    return np.concatenate(out)
+
+
+DATA = {
+    "lengths": lengths,
+    "rows": rows,
+    "runs": lambda r: np.repeat(r.integers(0, 3, 60, dtype=np.uint8), r.integers(1, 5000, 60)),
+    "period_33": lambda r: np.resize(r.integers(0, 256, 33, dtype=np.uint8), 70001),
+    "two_symbols": lambda r: r.integers(0, 2, 65537, dtype=np.uint8),
+    "one_value": lambda r: np.full(66000, 7, np.uint8),
+    "tiny": lambda r: np.resize(r.integers(0, 256, 5, dtype=np.uint8), 11),
+}
+
+
+@pytest.mark.parametrize("level", [1, 5, 9])
+@pytest.mark.parametrize("name", sorted(DATA))
+def test_finished_matches(codec, name, level):
+    import oracle as O
+    data = DATA[name](np.random.default_rng(11))
+    for block_log in (16, 18):
+        B = 1 << block_log
+        methods, lens, _, pay, offs = codec.compress_arrays(data, block_log, level=level)
+        for b in range(len(methods)):
+            blk = data[b * B:(b + 1) * B].tobytes()
+            want = O.Port.compress_block(blk, O.depth_for_level(level))
+            got = pay[int(offs[b]): int(offs[b]) + int(lens[b])].tobytes() if methods[b] else blk
+            assert got == (want if len(want) < len(blk) else blk), f"block {b} of {name} at 2^{block_log}"
+
+
+@pytest.mark.parametrize("level", [1, 5])
+def test_segment_counts(codec, level):
+    """One launch of 2048 and one of 2560 blocks of 64 KiB (fewer segments a block, 32 and 64 a warp) against launches
+    of 64 blocks (1024 segments a block): the blocks repeat, so their payloads must."""
+    import datagen as G
+    block_log, nb, reps = 16, 512, 9
+    tile = G.lz_mix(nb << block_log, block_log, 3)
+    small = []
+    for k in range(0, nb, 64):
+        m, n, _, p, o = codec.compress_arrays(tile[k << block_log:(k + 64) << block_log], block_log, level=level)
+        small += [p[int(a): int(a) + int(b)].tobytes() for a, b in zip(o, n)]
+        assert m.all()
+    m, n, _, p, o = codec.compress_arrays(np.tile(tile, reps), block_log, level=level)
+    assert m.all()
+    for b in range(nb * reps):
+        assert p[int(o[b]): int(o[b]) + int(n[b])].tobytes() == small[b % nb], f"block {b}"

@@ -122,11 +122,10 @@ int ensure_enc(zc_ctx* c, uint32_t nb, uint32_t block_log) {
   const size_t B = (size_t)1 << block_log, TC = zc::tok_cap((uint32_t)B), EC = zc::ext_cap((uint32_t)B);
   const size_t N = (size_t)nb * B;
   Need need[] = {
-      {&c->e_tmp_pos, N * 4}, {&c->e_srt_pos, N * 4}, {&c->e_minfo, N * 4},
+      {&c->e_tmp, N * 4}, {&c->e_srt, N * 4}, {&c->e_minfo, N * 4},
       {&c->e_scnt, (size_t)nb * ((B + 4095) / 4096) * 256 * 4},
-      {&c->e_tk_seg, (size_t)nb * 3 * zc::seg_tok_cap((uint32_t)B) * 4},
-      {&c->e_tmp_h, N * 2}, {&c->e_srt_h, N * 2},
-      {&c->e_tk_i, nb * TC * 4}, {&c->e_tk_m, nb * TC * 4}, {&c->e_tk_d, nb * TC * 4},
+      {&c->e_tk_seg, (size_t)nb * 3 * zc::seg_tok_cap((uint32_t)B) * 4}, {&c->e_seg, (size_t)nb * zc::kMaxSegs * 4},
+      {&c->e_tmp_d, N}, {&c->e_tk_i, nb * TC * 4}, {&c->e_tk_m, nb * TC * 4}, {&c->e_tk_d, nb * TC * 4},
       {&c->e_bcnt, (size_t)nb * 8 * 4}, {&c->e_lit, N}, {&c->e_tok, nb * TC}, {&c->e_ext, nb * EC},
       {&c->e_sym, nb * TC}, {&c->e_grp, nb * TC}, {&c->e_bits, (size_t)nb * zc::bits_cap((uint32_t)B)},
       {&c->e_lanes, (size_t)nb * zc::lanes_per_block((uint32_t)B)}, {&c->e_freq, (size_t)nb * 5 * 256 * 2},
@@ -146,7 +145,7 @@ int ensure_dec(zc_ctx* c, uint32_t nb, uint32_t block_log) {
 
 bool bad_block_log(uint32_t bl) { return bl < zc::kMinBlockLog || bl > zc::kMaxBlockLog; }
 
-// blocks per encoder launch: 1 GiB of input (about 28 GiB of scratch: several waves of every stage on
+// blocks per encoder launch: 1 GiB of input (about 25 GiB of scratch: several waves of every stage on
 // 148 SMs), and the grid's y limit
 uint32_t enc_blocks_per_launch(uint32_t block_log) {
   return (uint32_t)std::min<size_t>(((size_t)1 << 30) >> block_log, 65535);
@@ -155,6 +154,16 @@ uint32_t enc_blocks_per_launch(uint32_t block_log) {
 // every SM busy; about 6 bytes of scratch per output byte)
 uint32_t dec_blocks_per_launch(uint32_t block_log) {
   return (uint32_t)std::min<size_t>(((size_t)4 << 30) >> block_log, 1u << 20);
+}
+
+// segments a block is parsed in: 1 KiB each, a lane's walk, where that fills the GPU (148 SMs x 1024 walks);
+// fewer blocks are cut finer, down to 1024 segments, so that the walks spread over more SMs
+// (64 MiB of text, 256 blocks of 256 KiB: the walks take 5.7 ms at 256 segments a block, 3.1 at 512, 1.7 at 1024;
+// 1 GiB of lz_mix: 14.3, 14.0, 15.0 ms with the parse, whose re-walks grow with the segments)
+uint32_t enc_segments(uint32_t nb, uint32_t block_log) {
+  uint32_t s = std::min(std::max((1u << block_log) / 1024u, 256u), zc::kMaxSegs);
+  while (s < zc::kMaxSegs && (uint64_t)nb * s < 148u * 1024u) s *= 2;
+  return s;
 }
 
 // The test injector (src/safe_codec.h:17 has the reference's): with ZC_FAIL_AFTER=n in the environment
@@ -188,15 +197,11 @@ int encode_device(zc_ctx* c, const uint8_t* d_in, const uint64_t* d_off, const u
   zc::EncArgs A{};
   A.in = d_in; A.in_off = d_off; A.in_len = d_len; A.nb = nb;
   A.B = 1u << block_log; A.block_log = block_log; A.depth = depth_for_level(level);
-  const Shape& sh = c->shape[block_log - zc::kMinBlockLog][level_class(level)];
-  A.cmp_cap = sh.cmp_cap;
-  A.match_tile = sh.match_tile;
-  A.match_dense = sh.match_dense;
-  A.match_defer = sh.match_defer;
-  A.tmp_pos = c->e_tmp_pos.as<uint32_t>(); A.srt_pos = c->e_srt_pos.as<uint32_t>();
+  A.tmp_e = c->e_tmp.as<uint32_t>(); A.tmp_d = c->e_tmp_d.as<uint8_t>(); A.srt = c->e_srt.as<uint32_t>();
   A.minfo = c->e_minfo.as<uint32_t>(); A.scnt = c->e_scnt.as<uint32_t>();
-  A.tk_seg = c->e_tk_seg.as<uint32_t>();
-  A.tmp_h = c->e_tmp_h.as<uint16_t>(); A.srt_h = c->e_srt_h.as<uint16_t>();
+  A.tk_seg = c->e_tk_seg.as<uint32_t>(); A.seg_exit = c->e_seg.as<uint32_t>();
+  A.nseg = enc_segments(nb, block_log);
+  A.walk_segs = (uint64_t)nb * A.nseg < 4 * 148u * 1024u ? 32 : 64;  // (64: two a lane, once they fill the GPU twice)
   A.tk_i = c->e_tk_i.as<uint32_t>(); A.tk_m = c->e_tk_m.as<uint32_t>(); A.tk_d = c->e_tk_d.as<uint32_t>();
   A.bcnt = c->e_bcnt.as<uint32_t>();
   A.s_lit = c->e_lit.as<uint8_t>(); A.s_tok = c->e_tok.as<uint8_t>(); A.s_ext = c->e_ext.as<uint8_t>();
@@ -440,7 +445,7 @@ void zc_close(zc_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   if (c->cstream) cudaStreamSynchronize(c->cstream);
   drop_graphs(c);
-  for (DevBuf* b : {&c->e_tmp_pos, &c->e_srt_pos, &c->e_minfo, &c->e_scnt, &c->e_tk_seg, &c->e_tmp_h, &c->e_srt_h, &c->e_tk_i,
+  for (DevBuf* b : {&c->e_tmp, &c->e_tmp_d, &c->e_srt, &c->e_minfo, &c->e_scnt, &c->e_tk_seg, &c->e_seg, &c->e_tk_i,
                     &c->e_tk_m, &c->e_tk_d, &c->e_bcnt, &c->e_lit, &c->e_tok, &c->e_ext, &c->e_sym, &c->e_grp,
                     &c->e_bits, &c->e_lanes, &c->e_freq, &c->e_lanelen, &c->e_sinfo, &c->e_slab, &c->d_lit, &c->d_tok,
                     &c->d_sym, &c->d_grp, &c->d_ext, &c->d_meta, &c->d_tks, &c->d_tkm, &c->d_tkd, &c->d_tkl, &c->s_in, &c->s_blk, &c->s_out, &c->s_meta, &c->work,
@@ -620,9 +625,9 @@ int zc_set_shape(zc_ctx* c, uint32_t block_log, int level, const zc_shape* in) {
   return ZC_OK;
 }
 
-// Times every candidate shape on the sample (whole blocks of it, up to one encoder launch) and keeps
-// the fastest for (block_log, level): the match cap by the encoder's time, the fill's shape by the
-// decoder's.  Each candidate runs once untimed and then `reps` times; its time is the smallest.
+// Times every candidate shape of the fill on the sample (whole blocks of it, up to one encoder launch) and
+// keeps the fastest for (block_log, level).  Each candidate runs once untimed and then `reps` times; its time
+// is the smallest.
 int zc_autotune(zc_ctx* c, const uint8_t* sample, size_t n, uint32_t block_log, int level, zc_shape* chosen) {
   if (!c || (!sample && n)) return ZC_E_ARG;
   ZC_GATE(c);
@@ -697,36 +702,7 @@ int zc_autotune(zc_ctx* c, const uint8_t* sample, size_t n, uint32_t block_log, 
     if (e != cudaSuccess) { r = cuda_fail(c, e, "autotune set-up"); break; }
     Shape best = saved;
     float best_ms = 1e30f;
-    for (uint32_t cap : {12u, 16u, 24u, 32u})
-      for (uint32_t tile : {256u, 512u, 1024u}) {
-        if (r) break;
-        cur = best;
-        cur.cmp_cap = cap;
-        cur.match_tile = tile;
-        float ms;
-        if ((r = timed(encode, ms))) break;
-        if (ms < best_ms) { best_ms = ms; best.cmp_cap = cap; best.match_tile = tile; }
-      }
-    for (uint32_t dense : {128u, 256u, 512u, 1025u}) {  // (with the best cap and tile; 1025: never a lane each)
-      if (r || dense == best.match_dense) continue;
-      cur = best;
-      cur.match_dense = dense;
-      float ms;
-      if ((r = timed(encode, ms))) break;
-      if (ms < best_ms) { best_ms = ms; best.match_dense = dense; }
-    }
-    for (uint32_t back : {2u, 3u, 4u}) {  // (the match pass's savings against the parse's extra finishes)
-      if (r || back == best.match_defer) continue;
-      cur = best;
-      cur.match_defer = back;
-      float ms;
-      if ((r = timed(encode, ms))) break;
-      if (ms < best_ms) { best_ms = ms; best.match_defer = back; }
-    }
-    if (r) break;
-    cur = best;
-    if ((r = encode())) break;  // (every cap writes the same payloads)
-    best_ms = 1e30f;
+    if ((r = encode())) break;  // (the sample's payloads, for the decoder)
     for (uint32_t rl = 11; rl <= 14 && !r; ++rl)
       for (uint32_t w : {1u, 2u, 4u, 8u})
         for (uint32_t wd : {1u, 2u, 4u}) {

@@ -7,16 +7,16 @@
 //
 //   k_sort_*       stable two-pass LSD radix sort of each block's positions by hash (8 + 8 bits), a
 //                  CTA per 4096-position tile: digit counts, per-block scan, ranked scatter (warp
-//                  match_any ranks, the tile reordered in shared memory, digit runs written together)
-//   k_enc_match    per sorted position: its nearest candidate, then, where that does not decide it, its
-//                  chain scanned (by a lane, or by a group of lanes a candidate each where the tile has few
-//                  such positions), comparing at most cmp_cap bytes; a match that reaches cmp_cap, or a
-//                  position that lies inside a longer match starting before it, is marked and finished
-//                  only if the parse visits it
-//   k_enc_parse    one CTA per block: the greedy + lazy parse as a chain 0 -> next(0) -> ..., walked
-//                  per segment in parallel from the segment start, then re-walked from the true entry
-//                  until it meets the first walk (rounds until no segment exit moves); a warp's walks
-//                  step together and finish capped matches as a warp
+//                  match_any ranks, the tile reordered in shared memory, digit runs written together).
+//                  An entry is one word: the position and 12 more bits of its 4 bytes' product
+//   k_enc_chain    per sorted entry: does its chain hold an entry with the same 12 bits (a candidate of 4
+//                  equal bytes)?  No: no match.  Yes: the position is marked with its place in the order
+//   k_enc_walk     the greedy + lazy parse as a chain 0 -> next(0) -> ..., walked in parallel from the start
+//                  of every segment of every block; a warp's walks step together, and the exact matches that
+//                  a step needs are computed by the warp for all its walks at once (warp_finish), only at
+//                  positions that a walk visits
+//   k_enc_parse    one CTA per block: segments re-walked from where the chain before them leaves until they
+//                  meet the first walk (rounds until no segment exit moves), then the tokens written
 //   k_enc_streams  one warp per block: group starts from a running maximum of per-token thresholds and a
 //                  next-start chain, recent offsets by shuffles from each group's start, tok / ext / sym /
 //                  group streams, offset bits packed by a word-segmented OR-scan, literals
@@ -29,16 +29,15 @@
 
 namespace zc {
 
-// per-position match record: NONE; SAT | r (a candidate reached cmp_cap, or the position lies inside a
-// longer match that starts before it; r is the position's index in the hash-sorted order, where its chain
-// starts: finished on demand by the parse, which computes the chain's exact best); BELOW | r (the parse
-// found that the position's match cannot win the lazy test of the position before it, and left it
-// unfinished: finished like SAT if a walk needs it exactly); or the exact (length - 4) << 20 |
-// (distance - 1).  Lengths are <= 4096, so an exact record has at most 0xFFC in its top 12 bits, and
-// r < 2^20 - 3, so SAT | r is never NONE.
+// per-position match record: NONE; SAT | r (the position's chain holds a candidate; r is the position's
+// index in the hash-sorted order, where its chain starts: the exact best is computed when a walk of the
+// parse needs it); BELOW | r (the parse found that the position's match cannot win the lazy test of the
+// position before it, and left it unfinished: finished like SAT if a walk needs it exactly); or the exact
+// (length - 4) << 20 | (distance - 1).  Lengths are <= 4096, so an exact record has at most 0xFFC in its
+// top 12 bits, and r < 2^20 - 3, so SAT | r is never NONE.
 constexpr uint32_t M_NONE = 0xFFFFFFFFu;
 constexpr uint32_t M_SAT = 0xFFF00000u;
-constexpr uint32_t M_BELOW = 0xFFE00000u;  // capped, and known to lose the lazy test of the position before
+constexpr uint32_t M_BELOW = 0xFFE00000u;  // unfinished, and known to lose the lazy test of the position before
 __device__ __forceinline__ bool m_is_sat(uint32_t v) { return (v >> 20) >= 0xFFEu && v != M_NONE; }
 __device__ __forceinline__ bool m_is_below(uint32_t v) { return (v >> 20) == 0xFFEu; }
 __device__ __forceinline__ uint32_t m_pack(uint32_t m, uint32_t d) { return ((m - 4u) << 20) | (d - 1u); }
@@ -50,23 +49,35 @@ __device__ __forceinline__ uint32_t load4(const uint8_t* base, uint64_t x) {
   const uint32_t* w = reinterpret_cast<const uint32_t*>(base) + (x >> 2);
   return __funnelshift_r(__ldg(w), __ldg(w + 1), (uint32_t)(x & 3u) * 8u);
 }
-// the CPU parse's hash: 4 bytes times 2654435761, top 16 bits (src/codec2.h:47)
-__device__ __forceinline__ uint32_t hash16(const uint8_t* base, uint64_t x) { return (load4(base, x) * 2654435761u) >> 16; }
+// The CPU parse's hash is the top 16 bits of the 4 bytes' product with 2654435761 (src/codec2.h:47).  The
+// product is a bijection of the 4 bytes, so its next 12 bits (the tag) tell 4 equal bytes from a mere hash
+// collision, up to its last 4 bits.
+__device__ __forceinline__ uint32_t product(uint32_t x) { return x * 2654435761u; }
+// a sorted entry: its position (20 bits) and its tag
+__device__ __forceinline__ uint32_t entry(uint32_t p, uint32_t prod) { return p | (prod << 16 & 0xFFF00000u); }
+__device__ __forceinline__ uint32_t e_pos(uint32_t e) { return e & 0xFFFFFu; }
+__device__ __forceinline__ uint32_t e_tag(uint32_t e) { return e >> 20; }
 
-// common prefix of the bytes at a and b, at most cap
-__device__ __forceinline__ uint32_t lcp(const uint8_t* base, uint64_t a, uint64_t b, uint32_t cap) {
-  uint32_t l = 0;
-  while (l + 4 <= cap) {
-    const uint32_t x = load4(base, a + l) ^ load4(base, b + l);
-    if (x) return l + ((uint32_t)__ffs(x) - 1u) / 8u;
-    l += 4;
-  }
-  if (l < cap) {
-    const uint32_t x = load4(base, a + l) ^ load4(base, b + l);
-    const uint32_t k = x ? ((uint32_t)__ffs(x) - 1u) / 8u : 4u;
-    return l + min(k, cap - l);
-  }
-  return l;
+// 16 bytes at byte offset x of a 16-aligned buffer, from the two aligned vectors around them (two L1
+// requests a lane where five word loads would make five; the scattered candidates' loads are what the
+// parse waits for)
+__device__ __forceinline__ uint4 load16(const uint8_t* base, uint64_t x) {
+  const uint4* c = reinterpret_cast<const uint4*>(base + (x & ~(uint64_t)15));
+  const uint4 a = __ldg(c), b = __ldg(c + 1);
+  const bool w2 = x & 8u, w1 = x & 4u;
+  const uint32_t sh = (uint32_t)(x & 3u) * 8u;
+  const uint32_t t0 = w2 ? a.z : a.x, t1 = w2 ? a.w : a.y, t2 = w2 ? b.x : a.z, t3 = w2 ? b.y : a.w, t4 = w2 ? b.z : b.x,
+                 t5 = w2 ? b.w : b.y;
+  const uint32_t u0 = w1 ? t1 : t0, u1 = w1 ? t2 : t1, u2 = w1 ? t3 : t2, u3 = w1 ? t4 : t3, u4 = w1 ? t5 : t4;
+  return make_uint4(__funnelshift_r(u0, u1, sh), __funnelshift_r(u1, u2, sh), __funnelshift_r(u2, u3, sh),
+                    __funnelshift_r(u3, u4, sh));
+}
+// the first differing byte of two 16-byte windows (16 when equal)
+__device__ __forceinline__ uint32_t lcp16(const uint4& a, const uint4& b) {
+  const uint32_t x0 = a.x ^ b.x, x1 = a.y ^ b.y, x2 = a.z ^ b.z, x3 = a.w ^ b.w;
+  const uint32_t x = x0 ? x0 : x1 ? x1 : x2 ? x2 : x3;
+  const uint32_t o = x0 ? 0u : x1 ? 4u : x2 ? 8u : 12u;
+  return x ? o + (((uint32_t)__ffs(x) - 1u) >> 3) : 16u;
 }
 
 // ---------------------------------------------------------------- 1. stable sort by hash
@@ -74,21 +85,25 @@ __device__ __forceinline__ uint32_t lcp(const uint8_t* base, uint64_t a, uint64_
 // tiles of 4096 positions, every tile its own CTA: k_sort_count (the tile's digit counts), k_sort_scan
 // (per block: each tile's start for each digit, digit-major), k_sort_scatter (ranks the tile's entries
 // per digit in order with warp match_any, reorders the tile by digit in shared memory, and writes each
-// digit's run to its place).  Pass 0 reads positions in order and hashes them; pass 1 reads pass 0's
-// output.  The counts array holds tiles_per_block(B) * 256 words per block.
+// digit's run to its place).  Pass 0 reads positions in order and hashes them; it writes each entry's word
+// and, in a byte array, its digit of pass 1, which reads both and writes words alone: 16 bytes moved a
+// position in all (22 with the hash beside the position in both passes).  The counts array holds
+// tiles_per_block(B) * 256 words per block.
 constexpr uint32_t kSortTile = 4096, kSortThreads = 512, kSortPer = kSortTile / kSortThreads;
 
 __device__ __forceinline__ uint32_t sort_tiles(uint32_t B) { return (B + kSortTile - 1) / kSortTile; }
 
+// the entry's word and its 16-bit hash (pass 1: its high byte alone, in the high byte's place)
 template <int PASS>
-__device__ __forceinline__ void sort_load(const EncArgs& A, uint32_t b, uint32_t i, uint32_t& p, uint32_t& h) {
+__device__ __forceinline__ void sort_load(const EncArgs& A, uint32_t b, uint32_t i, uint32_t& e, uint32_t& h) {
   if (PASS == 0) {
-    p = i;
-    h = hash16(A.in, A.in_off[b] + i);
+    const uint32_t x = product(load4(A.in, A.in_off[b] + i));
+    e = entry(i, x);
+    h = x >> 16;
   } else {
     const size_t so = (size_t)b * A.B;
-    p = A.tmp_pos[so + i];
-    h = A.tmp_h[so + i];
+    e = A.tmp_e[so + i];
+    h = (uint32_t)A.tmp_d[so + i] << 8;
   }
 }
 template <int PASS>
@@ -96,7 +111,7 @@ __device__ __forceinline__ uint32_t sort_digit(uint32_t h) { return PASS == 0 ? 
 
 // each thread counts 16 consecutive entries of the tile: pass 0 hashes them from three aligned 16-byte
 // loads of the input (the 19 bytes it needs, inside the input's readable slack), pass 1 reads their
-// 16 hashes as two 16-byte loads; per-warp histograms in shared memory, summed at the end
+// 16 digits as one 16-byte load; per-warp histograms in shared memory, summed at the end
 template <int PASS>
 __global__ void __launch_bounds__(256) k_sort_count(EncArgs A) {
   const uint32_t b = blockIdx.y, t = blockIdx.x, tid = threadIdx.x, w = tid >> 5;
@@ -122,13 +137,12 @@ __global__ void __launch_bounds__(256) k_sort_count(EncArgs A) {
 #pragma unroll
       for (int k = 0; k < 5; ++k) x[k] = __funnelshift_r(u[k], u[k + 1], sh);
 #pragma unroll
-      for (int j = 0; j < 16; ++j) h[j] = (__funnelshift_r(x[j >> 2], x[(j >> 2) + 1], 8 * (j & 3)) * 2654435761u) >> 16;
+      for (int j = 0; j < 16; ++j) h[j] = product(__funnelshift_r(x[j >> 2], x[(j >> 2) + 1], 8 * (j & 3))) >> 16;
     } else {
-      const uint4* q = reinterpret_cast<const uint4*>(A.tmp_h + (size_t)b * A.B + i);
-      const uint4 v0 = q[0], v1 = q[1];
-      const uint32_t vw[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+      const uint4 v = *reinterpret_cast<const uint4*>(A.tmp_d + (size_t)b * A.B + i);
+      const uint32_t vw[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-      for (int j = 0; j < 16; ++j) h[j] = (vw[j >> 1] >> (16 * (j & 1))) & 0xFFFFu;
+      for (int j = 0; j < 16; ++j) h[j] = (vw[j >> 2] >> (8 * (j & 3)) & 0xFFu) << 8;
     }
 #pragma unroll
     for (int j = 0; j < 16; ++j)
@@ -165,7 +179,7 @@ template <int PASS>
 __global__ void __launch_bounds__(kSortThreads, 4) k_sort_scatter(EncArgs A) {
   constexpr uint32_t NW = kSortThreads / 32;
   __shared__ uint32_t cw[NW][256];  // per-warp digit counts, then the warp's start within the digit
-  __shared__ uint32_t st_pos[kSortTile];
+  __shared__ uint32_t st_e[kSortTile];
   __shared__ uint16_t st_h[kSortTile];
   __shared__ uint32_t tds[256], dst[256], ws[8];
   const uint32_t b = blockIdx.y, t = blockIdx.x, tid = threadIdx.x, lane = lane_id(), w = tid >> 5;
@@ -180,19 +194,18 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_sort_scatter(EncArgs A) {
   // ranks: warp w holds the tile's entries [kSortPer * 32 w, kSortPer * 32 (w + 1)), 32 per round, in order
   // (all of a thread's entries are loaded first: the ranking's warp syncs would otherwise keep each load
   // behind the previous entry's ranking)
-  uint32_t kp[kSortPer], kh[kSortPer], kr[kSortPer];
+  uint32_t ke[kSortPer], kh[kSortPer], kr[kSortPer];
 #pragma unroll
   for (uint32_t j = 0; j < kSortPer; ++j) {
     const uint32_t li = w * (32 * kSortPer) + j * 32 + lane;
-    kp[j] = 0; kh[j] = 0;
-    if (li < tn) sort_load<PASS>(A, b, i0 + li, kp[j], kh[j]);
+    ke[j] = 0; kh[j] = 0;
+    if (li < tn) sort_load<PASS>(A, b, i0 + li, ke[j], kh[j]);
   }
 #pragma unroll
   for (uint32_t j = 0; j < kSortPer; ++j) {
     const uint32_t li = w * (32 * kSortPer) + j * 32 + lane;
     const bool on = li < tn;
-    const uint32_t p = kp[j], h = kh[j];
-    const uint32_t d = sort_digit<PASS>(h);
+    const uint32_t d = sort_digit<PASS>(kh[j]);
     const unsigned act = __ballot_sync(kFull, on);
     uint32_t rk = 0xFFFFFFFFu;
     if (on) {
@@ -203,7 +216,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_sort_scatter(EncArgs A) {
       if ((peers & ((1u << lane) - 1u)) == 0) cw[w][d] = c + __popc(peers);
     }
     __syncwarp();
-    kp[j] = p; kh[j] = h; kr[j] = rk;
+    kr[j] = rk;
   }
   __syncthreads();
   if (tid < 256) {  // per digit: the warps' starts within it, and the tile's count
@@ -226,262 +239,101 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_sort_scatter(EncArgs A) {
     if (kr[j] == 0xFFFFFFFFu) continue;
     const uint32_t d = sort_digit<PASS>(kh[j]);
     const uint32_t at = tds[d] + cw[w][d] + kr[j];
-    st_pos[at] = kp[j];
+    st_e[at] = ke[j];
     st_h[at] = (uint16_t)kh[j];
   }
   __syncthreads();
-  uint32_t* op = PASS == 0 ? A.tmp_pos : A.srt_pos;
-  uint16_t* oh = PASS == 0 ? A.tmp_h : A.srt_h;
+  uint32_t* oe = PASS == 0 ? A.tmp_e : A.srt;
   for (uint32_t i = tid; i < tn; i += kSortThreads) {
     const uint32_t h = st_h[i], d = sort_digit<PASS>(h);
     const size_t dest = so + dst[d] + (i - tds[d]);
-    op[dest] = st_pos[i];
-    oh[dest] = (uint16_t)h;
+    oe[dest] = st_e[i];
+    if (PASS == 0) A.tmp_d[dest] = (uint8_t)(h >> 8);
   }
 }
 
-// ---------------------------------------------------------------- 2. capped matches at every position
-// A position whose nearest candidate matches at least 4 bytes and also the A.match_defer bytes before them
-// (1..4; 0: never) is inside a longer match; the match pass leaves it to the parse.  The mask selects those
-// bytes in the little-endian word of the 4 bytes before the position.
-__device__ __forceinline__ uint32_t defer_mask(uint32_t back) { return back ? 0xFFFFFFFFu << (8u * (4u - back)) : 0u; }
+// ---------------------------------------------------------------- 2. which positions have a candidate
+// A CTA of 256 threads per kChainTile consecutive sorted entries of a block.  A position whose chain (its
+// `depth` predecessors in the order, as far as they have its hash) holds no entry of its own tag has no
+// match: its record is NONE, and exact.  Every other position is marked SAT with its place in the order, and
+// the parse computes its match if a walk comes there.  No input byte is read: a pass that compared every
+// position's candidates took 21.4 ms per GiB on lz_mix at block 18, level 5 (the input's bytes at scattered
+// positions, two 16-byte loads each, then up to 32 compares), for records of which the parse reads 7 %.
+// What bounds this one is the records' scattered stores (one L1 request each).
+//
+// Chains are not told apart by the hash, which an entry does not hold, but by the positions: they rise within
+// a chain, so an entry whose predecessor's position is higher starts a chain (bnd: a bit an entry).  A
+// start that this misses only leaves entries of another hash among the candidates, which have another tag or,
+// once in thousands, fewer than 4 bytes in common: the parse finds no match there.
+// Most marked positions have the tag of their predecessor; the others, unless they start a chain, go to a list
+// that the CTA's lanes scan, two tags a word.
+constexpr uint32_t kChainTile = 2048, kChainLook = 256;  // (depth is at most kChainLook)
 
-// the first differing byte of two 16-byte windows (16 when equal)
-__device__ __forceinline__ uint32_t lcp16(const uint4& a0, const uint4& b0) {
-  uint32_t x;
-  if ((x = a0.x ^ b0.x)) return ((uint32_t)__ffs(x) - 1u) >> 3;
-  if ((x = a0.y ^ b0.y)) return 4 + (((uint32_t)__ffs(x) - 1u) >> 3);
-  if ((x = a0.z ^ b0.z)) return 8 + (((uint32_t)__ffs(x) - 1u) >> 3);
-  if ((x = a0.w ^ b0.w)) return 12 + (((uint32_t)__ffs(x) - 1u) >> 3);
-  return 16;
-}
-// the first differing byte of two 32-byte windows (32 when equal)
-__device__ __forceinline__ uint32_t lcp32(const uint4& a0, const uint4& a1, const uint4& b0, const uint4& b1) {
-  uint32_t x;
-  if ((x = a0.x ^ b0.x)) return ((uint32_t)__ffs(x) - 1u) >> 3;
-  if ((x = a0.y ^ b0.y)) return 4 + (((uint32_t)__ffs(x) - 1u) >> 3);
-  if ((x = a0.z ^ b0.z)) return 8 + (((uint32_t)__ffs(x) - 1u) >> 3);
-  if ((x = a0.w ^ b0.w)) return 12 + (((uint32_t)__ffs(x) - 1u) >> 3);
-  if ((x = a1.x ^ b1.x)) return 16 + (((uint32_t)__ffs(x) - 1u) >> 3);
-  if ((x = a1.y ^ b1.y)) return 20 + (((uint32_t)__ffs(x) - 1u) >> 3);
-  if ((x = a1.z ^ b1.z)) return 24 + (((uint32_t)__ffs(x) - 1u) >> 3);
-  if ((x = a1.w ^ b1.w)) return 28 + (((uint32_t)__ffs(x) - 1u) >> 3);
-  return 32;
-}
-
-#ifndef ZC_MATCH_GROUP
-#define ZC_MATCH_GROUP 16
-#endif
-constexpr uint32_t kMatchGroup = ZC_MATCH_GROUP;  // lanes per work-list entry in the match pass: 8, 16 or 32
-static_assert(kMatchGroup == 8 || kMatchGroup == 16 || kMatchGroup == 32, "lanes per work-list entry");
-
-// One CTA of 256 threads per `tile` consecutive sorted positions of a block (tile = A.match_tile, a
-// multiple of 256).  The entries it needs (its own and the `depth` before them) are staged once in
-// shared memory with the first WB bytes at each position (WB = 16 or 32, at least the compare cap), so
-// a candidate costs a few shared loads and XORs instead of random global reads.  Pass 1 gives each
-// position its nearest candidate, which decides most of them; the rest go to a work list, scanned a lane
-// per entry when it fills the CTA's lanes (or chains are short), else by groups of lanes, one candidate
-// a lane (one lane per entry would leave most lanes idle while a warp's longest chain finishes).
-// Dynamic shared memory: (tile + depth) * (WB + 4 + 2) + 8 * tile bytes (+4).
-template <uint32_t WB>
-__global__ void __launch_bounds__(256) k_enc_match(EncArgs A) {
-  constexpr uint32_t NV = WB / 16;  // uint4s per window
-  extern __shared__ uint4 sm[];
-  __shared__ uint32_t next, nwork;
+__global__ void __launch_bounds__(256) k_enc_chain(EncArgs A) {
+  __shared__ __align__(16) uint16_t tag[kChainTile + kChainLook];
+  __shared__ uint32_t bnd[(kChainTile + kChainLook) / 32];
+  __shared__ uint16_t list[kChainTile];
+  __shared__ uint32_t nlist;
   const uint32_t b = blockIdx.y, t = threadIdx.x, lane = lane_id();
-  const uint32_t tile = A.match_tile;
-  const uint32_t r0 = blockIdx.x * tile;
+  const uint32_t r0 = blockIdx.x * kChainTile;
   const uint32_t n = A.in_len[b];
   if (r0 >= n) return;
   const uint32_t count = n >= 4 ? n - 3 : 0;
   const size_t so = (size_t)b * A.B;
+  const uint32_t* E = A.srt + so;
   const uint32_t D = (uint32_t)A.depth;
-  const uint32_t cap_e = tile + D;
-  const uint32_t dmask = defer_mask(A.match_defer);
-  uint4* win = sm;  // entry i: bytes 16 v .. 16 v + 15 at win[NV i + v]
-  uint32_t* spos = reinterpret_cast<uint32_t*>(win + NV * cap_e);
-  uint16_t* sh = reinterpret_cast<uint16_t*>(spos + cap_e);
-  uint32_t* wl = reinterpret_cast<uint32_t*>(sh + ((cap_e + 1) & ~1u));  // work list: entry | best << 16, distance
-  const uint32_t e0 = r0 > D ? r0 - D : 0, e1 = min(r0 + tile, count);
-  const uint64_t base = A.in_off[b];
-  // (a window may reach up to WB + 15 bytes past its position, inside the input's readable slack; bytes past
-  // the block never decide a match: every compare is capped at the block's end)
-  if (t == 0) { next = 0; nwork = 0; }
-  for (uint32_t i = t; e0 + i < e1; i += 256) {
+  const uint32_t look = (D + 31u) & ~31u;  // (whole words of bnd)
+  const uint32_t e0 = r0 > look ? r0 - look : 0, e1 = min(r0 + kChainTile, count), own = r0 - e0;
+  if (t == 0) nlist = 0;
+  for (uint32_t i = t; e0 + (i & ~31u) < e1; i += 256) {
     const uint32_t r = e0 + i;
-    const uint32_t p = A.srt_pos[so + r];
-    spos[i] = p;
-    sh[i] = A.srt_h[so + r];
-    // the window from WB / 16 + 1 aligned 16-byte loads (a few L1 requests an entry instead of one a word:
-    // the entries' positions are scattered), its words picked by selects on the word offset
-    const uint64_t a = base + p;
-    const uint4* c = reinterpret_cast<const uint4*>(A.in + (a & ~(uint64_t)15));
-    constexpr uint32_t NC = WB / 16 + 1;
-    uint32_t cw[4 * NC];
-#pragma unroll
-    for (uint32_t k = 0; k < NC; ++k) {
-      const uint4 x = __ldg(c + k);
-      cw[4 * k] = x.x; cw[4 * k + 1] = x.y; cw[4 * k + 2] = x.z; cw[4 * k + 3] = x.w;
-    }
-    const uint32_t o = (uint32_t)(a >> 2) & 3u, shf = (uint32_t)(a & 3u) * 8u;
-    uint32_t w[WB / 4 + 1];
-#pragma unroll
-    for (uint32_t q = 0; q <= WB / 4; ++q) w[q] = o == 0 ? cw[q] : o == 1 ? cw[q + 1] : o == 2 ? cw[q + 2] : cw[q + 3];
-    uint32_t v[WB / 4];
-#pragma unroll
-    for (uint32_t q = 0; q < WB / 4; ++q) v[q] = __funnelshift_r(w[q], w[q + 1], shf);
-#pragma unroll
-    for (uint32_t q = 0; q < NV; ++q) win[NV * i + q] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+    const uint32_t e = r < e1 ? E[r] : 0u;
+    uint32_t before = __shfl_up_sync(kFull, e, 1);
+    if (lane == 0) before = r > 0 ? E[r - 1] : 0xFFFFFFFFu;
+    const unsigned m = __ballot_sync(kFull, e_pos(before) >= e_pos(e));
+    if (lane == 0) bnd[i >> 5] = m;
+    tag[i] = (uint16_t)e_tag(e);
   }
   // positions past the last hashed one (the block's final 3 bytes) have no match
-  for (uint32_t r = max(r0, count) + t; r < min(r0 + tile, n); r += 256) A.minfo[so + r] = M_NONE;
+  for (uint32_t r = max(r0, count) + t; r < min(r0 + kChainTile, n); r += 256) A.minfo[so + r] = M_NONE;
   __syncthreads();
-  const uint32_t tn = e1 > r0 ? e1 - r0 : 0;  // positions of this tile
-  // pass 1, a thread per position: the nearest candidate decides most positions (no candidate, a chain
-  // of one, or a match that reaches the cap); the others go to the work list with what it found
-  for (uint32_t my = t; my < tn; my += 256) {
-    const uint32_t r = r0 + my, li = r - e0;
-    const uint32_t p = spos[li], h = sh[li];
-    const uint32_t lim = min(kMaxMatch, n - p), cap = min(min(A.cmp_cap, WB), lim);
-    uint32_t v = M_NONE;
-    if (r > 0 && sh[li - 1] == h) {
-      const uint32_t e = li - 1;
-      const uint32_t l = min(NV == 2 ? lcp32(win[2 * e], win[2 * e + 1], win[2 * li], win[2 * li + 1])
-                                     : lcp16(win[e], win[li]), cap);
-      const uint32_t d = p - spos[e];
-      if (l == cap) {
-        v = cap < lim ? M_SAT | r : m_pack(l, d);
-      } else if (r < 2 || D < 2 || sh[li - 2] != h) {
-        v = l < 4 ? M_NONE : m_pack(l, d);
-      } else if (dmask && l >= 4 && p >= 4 && p - d >= 4 &&
-                 ((load4(A.in, base + p - 4) ^ load4(A.in, base + p - d - 4)) & dmask) == 0) {
-        // the nearest candidate's match also runs match_defer bytes back, so p lies inside a longer match
-        // that starts earlier: the parse rarely visits it (it lands on match starts and the position after
-        // them).  It is left capped, to be finished exactly, like any capped record, if the parse comes.
-        v = M_SAT | r;
-      } else {
-        const uint32_t w = atomicAdd(&nwork, 1u);
-        wl[2 * w] = li | (l << 16);
-        wl[2 * w + 1] = d;
-        continue;
-      }
+  for (uint32_t i = own + t; e0 + (i & ~31u) < e1; i += 256) {
+    const bool on = e0 + i < e1;
+    const bool starts = bnd[i >> 5] >> lane & 1u;  // (i & 31 == lane: own is a multiple of 32)
+    const bool same = on && !starts && tag[i] == tag[i - 1];
+    const bool ask = on && !starts && !same && D > 1;
+    const unsigned am = __ballot_sync(kFull, ask);
+    if (am) {
+      uint32_t at = 0;
+      if (lane == 0) at = atomicAdd(&nlist, (uint32_t)__popc(am));
+      at = __shfl_sync(kFull, at, 0);
+      if (ask) list[at + __popc(am & ((1u << lane) - 1u))] = (uint16_t)i;
     }
-    A.minfo[so + p] = v;
+    if (on && !ask) A.minfo[so + e_pos(E[e0 + i])] = same ? M_SAT | (e0 + i) : M_NONE;
   }
   __syncthreads();
-  const uint32_t tw = nwork;
-  if (tw >= A.match_dense || D <= 8) {
-    // pass 2, a lane per work-list entry (a work list that fills the CTA, or chains of at most 8): lanes take
-    // entries from a CTA counter, a warp claiming entries for all its idle lanes at once.  Per-lane state: the
-    // position's entry li, its chain of kend earlier entries with the same hash (a binary search: the entries
-    // are sorted by hash), the candidate k reached so far, the best length, its distance, and the position's
-    // own byte at offset `best`: a candidate whose byte there differs cannot be longer and is skipped after
-    // one shared byte load (the CPU parse's probe, src/codec2.h:62)
-    const uint8_t* wb = reinterpret_cast<const uint8_t*>(win);
-    uint32_t li = 0xFFFFFFFFu, p = 0, lim = 0, cap = 0, best = 0, bd = 0, k = 0, kend = 0, pb = 0;
-    uint4 p0 = make_uint4(0, 0, 0, 0), p1 = p0;
-    bool dry = false;  // the tile has no unclaimed entries left (warp-uniform)
-    for (;;) {
-      const bool idle = li == 0xFFFFFFFFu;
-      const unsigned want = __ballot_sync(kFull, idle);
-      if (want && !dry) {
-        const uint32_t leader = (uint32_t)__ffs(want) - 1u;
-        uint32_t got = 0;
-        if (lane == leader) got = atomicAdd(&next, (uint32_t)__popc(want));
-        got = __shfl_sync(kFull, got, leader);
-        if (got + (uint32_t)__popc(want) >= tw) dry = true;
-        if (idle) {
-          const uint32_t my = got + (uint32_t)__popc(want & ((1u << lane) - 1u));
-          if (my < tw) {
-            const uint32_t wa = wl[2 * my];
-            li = wa & 0xFFFFu;
-            best = wa >> 16;
-            bd = wl[2 * my + 1];
-            const uint32_t r = li + e0;
-            p = spos[li];
-            const uint32_t h = sh[li];
-            lim = min(kMaxMatch, n - p);
-            cap = min(min(A.cmp_cap, WB), lim);
-            p0 = win[NV * li];
-            p1 = win[NV * li + NV - 1];
-            k = 1;
-            pb = wb[WB * li + best];
-            uint32_t lo = li - min(D, r), hi = li;  // the first entry of [lo, li] with hash h
-            while (lo < hi) {
-              const uint32_t mid = (lo + hi) >> 1;
-              if (sh[mid] < h) lo = mid + 1; else hi = mid;
-            }
-            kend = li - lo;
-          }
-        }
-      }
-      if (!__any_sync(kFull, li != 0xFFFFFFFFu)) break;
-      if (li == 0xFFFFFFFFu) continue;
-      // four candidates of this lane's chain: probes first, full compares for those that pass, in order
-      bool fin = false;
-      uint32_t pass = 0;
-#pragma unroll
-      for (uint32_t u = 0; u < 4; ++u) {
-        const uint32_t kk = k + 1 + u;
-        if (kk <= kend && (best == 0 || wb[WB * (li - kk) + best] == pb)) pass |= 1u << u;
-      }
-      while (pass) {
-        const uint32_t u = (uint32_t)__ffs(pass) - 1u;
-        pass &= pass - 1u;
-        const uint32_t kk = k + 1 + u, e = li - kk;
-        const uint32_t l = min(NV == 2 ? lcp32(win[2 * e], win[2 * e + 1], p0, p1) : lcp16(win[e], p0), cap);
-        if (l > best) {
-          best = l;
-          bd = p - spos[e];
-          if (best == cap) { fin = true; break; }
-          pb = wb[WB * li + best];
-        }
-      }
-      k += 4;
-      if (fin || k >= kend) {
-        A.minfo[so + p] = best < 4 ? M_NONE : best == cap && cap < lim ? M_SAT | (li + e0) : m_pack(best, bd);
-        li = 0xFFFFFFFFu;
-      }
+  const uint32_t* tw = reinterpret_cast<const uint32_t*>(tag);
+  for (uint32_t k = t; k < nlist; k += 256) {
+    const uint32_t i = list[k], tt = tag[i] * 0x00010001u;
+    uint32_t lo = i > D ? i - D : 0;  // the chain's first entry within the depth: the last start at or before i
+    for (int w = (int)(i >> 5); w >= (int)(lo >> 5); --w) {
+      uint32_t m = bnd[w];
+      if (w == (int)(i >> 5)) m &= 0xFFFFFFFFu >> (31u - (i & 31u));
+      if (m) { lo = max(lo, 32u * w + 31u - __clz(m)); break; }
     }
-    return;
-  }
-  // pass 2, kMatchGroup lanes per work-list entry (a short work list: a lane each would leave most lanes
-  // idle while the longest chain finishes): lane g of the group compares the chain's candidate k = kb + g
-  // (kb = 2, then kMatchGroup further each round; candidate 1 was pass 1's), all from shared memory; the
-  // group's longest, the nearest on a tie, replaces the best only when longer, so nearer rounds win ties
-  // too, as in the CPU parse's nearest-first scan.  The chain is the run of entries before the position with
-  // its hash (the entries are sorted by hash), so it ends at the first lane whose entry differs; a round
-  // ends the scan when the chain ends in it or the best reaches the cap.
-  constexpr uint32_t G = kMatchGroup, NG = 32 / G;
-  const uint32_t gl = lane % G;
-  const unsigned gmask = G == 32 ? kFull : ((1u << G) - 1u) << (lane - gl);
-  for (uint32_t wi = (t >> 5) * NG + lane / G; wi < tw; wi += 8 * NG) {
-    const uint32_t wa = wl[2 * wi];
-    const uint32_t li = wa & 0xFFFFu, r = li + e0;
-    uint32_t best = wa >> 16, bd = wl[2 * wi + 1];
-    const uint32_t p = spos[li], h = sh[li];
-    const uint32_t lim = min(kMaxMatch, n - p), cap = min(min(A.cmp_cap, WB), lim);
-    const uint4 p0 = win[NV * li], p1 = win[NV * li + NV - 1];
-    const uint32_t kmax = min(D, r);  // (li >= kmax: the tile's entries are staged from depth before it)
-    for (uint32_t kb = 2; kb <= kmax; kb += G) {
-      const uint32_t k = kb + gl;
-      const bool on = k <= kmax && sh[li - k] == h;
-      uint32_t key = 0;
-      if (on) {
-        const uint32_t e = li - k;
-        const uint32_t l = min(NV == 2 ? lcp32(win[2 * e], win[2 * e + 1], p0, p1) : lcp16(win[e], p0), cap);
-        key = (l << 8) | (G - 1u - gl);  // (l <= 32)
-      }
-      const uint32_t mk = __reduce_max_sync(gmask, key);
-      if ((mk >> 8) > best) {
-        best = mk >> 8;
-        bd = p - spos[li - (kb + G - 1u - (mk & 0xFFu))];
-      }
-      if (best == cap || __ballot_sync(gmask, on) != gmask) break;
+    bool found = false;
+    const int w0 = (int)(lo >> 1);
+    for (int w = (int)((i - 1) >> 1); w >= w0; --w) {  // two tags a word, the nearest first
+      const uint32_t x = tw[w] ^ tt;
+      uint32_t z = (x - 0x00010001u) & ~x & 0x80008000u;  // a half of x that is zero (a borrow can only add one)
+      if (w == (int)(i >> 1)) z &= 0x8000u;               // (i odd: the upper half is the entry itself)
+      if (w == w0 && (lo & 1u)) z &= 0x80000000u;
+      if (z) { found = true; break; }
     }
-    if (gl == 0) A.minfo[so + p] = best < 4 ? M_NONE : best == cap && cap < lim ? M_SAT | r : m_pack(best, bd);
+    A.minfo[so + e_pos(E[e0 + i])] = found ? M_SAT | (e0 + i) : M_NONE;
   }
 }
+
 
 // ---------------------------------------------------------------- 3. the parse
 struct ParseBlock {
@@ -489,155 +341,302 @@ struct ParseBlock {
   uint64_t base;
   uint32_t n, depth;
   uint32_t* minfo;
-  const uint32_t* spos;
-  const uint16_t* sh;
+  const uint32_t* srt;
 };
 
-// The exact match at x, all 32 lanes together (x the same in every lane).  A capped record names x's
-// index r in the hash-sorted order; its chain is the entries before r with the same hash, nearest first
-// (the order src/codec2.h:58-67 walks them).  Up to 32 candidates at a time: each
-// lane compares its candidate's first 32 bytes; those equal for 32 bytes (when the match may be longer)
-// are extended in chain order by the whole warp, 128 bytes a step.  The longest wins, the nearest on a
-// tie, and a match of the whole remaining length ends the walk, as in the CPU parse.  The exact record
-// replaces the capped one in minfo.
-// With need > 0 the caller only needs the exact match if it is at least `need` bytes long: a candidate whose
-// byte at need - 1 differs from x's is shorter and dropped after that one load, and when no candidate
-// reaches need the result is NONE and minfo keeps the capped record.
-__device__ uint32_t coop_exact(const ParseBlock& P, uint32_t x, uint32_t need = 0) {
-  const uint32_t lane = lane_id();
-  const uint32_t v = P.minfo[x];
-  if (!m_is_sat(v)) return v;
-  const uint32_t r = v & 0xFFFFFu, h = P.sh[r];
-  const uint32_t lim = min(kMaxMatch, P.n - x);
-  if (need > lim) return M_NONE;
-  const uint32_t l32 = min(32u, lim);
-  const uint32_t kmax = min(P.depth, r);
-  const uint64_t ax = P.base + x;
-  uint32_t best = 0, bd = 0;
-  bool stop = false;
-  for (uint32_t kb = 1; kb <= kmax && !stop; kb += 32) {
-    const uint32_t k = kb + lane;
-    const bool in_chain = k <= kmax && P.sh[r - k] == h;
-    const unsigned chain = __ballot_sync(kFull, in_chain);
-    const unsigned live = ~chain ? chain & ((1u << __ffs(~chain) - 1) - 1u) : chain;  // up to the first break
-    if (live != chain || chain != kFull) stop = true;  // the chain ends in this chunk
-    bool on = (live >> lane) & 1u;
-    const uint32_t j = on ? P.spos[r - k] : 0u;
-    if (need && on) on = __ldg(P.in + P.base + j + need - 1) == __ldg(P.in + ax + need - 1);
-    uint32_t l = 0;
-    if (on) {  // 16 bytes a round from independent word loads (at most two rounds)
-      const uint64_t aj = P.base + j;
-      for (uint32_t o = 0; o < l32; o += 16) {
-        uint32_t x[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) x[q] = load4(P.in, aj + o + 4 * q) ^ load4(P.in, ax + o + 4 * q);
-        uint32_t k = 16;
-#pragma unroll
-        for (int q = 3; q >= 0; --q) if (x[q]) k = 4 * q + (((uint32_t)__ffs(x[q]) - 1u) >> 3);
-        l = min(o + k, l32);
-        if (k < 16) break;
+// A warp's requests for exact matches, one a lane (slot = lane), and the candidates still to be compared, in shared
+// memory.  A candidate is slot << 20 | its position.
+constexpr uint32_t kTasks = 4;                        // chain loads in flight together
+constexpr uint32_t kItems = 32 + 32 * kTasks;         // the most candidates that wait at a time
+constexpr uint32_t kBatch = 8;
+struct Finish {
+  uint4 xw[32];                                       // the first 16 bytes at the request's position
+  uint32_t x[32], rt[32], key[32];                    // its position; its entry's place | tag << 20; best so far
+  uint32_t po[32], pw[32];                            // a candidate that matters has these 4 bytes at this offset
+  uint32_t ord[32];                                   // the requests' slots, one after the other
+  uint32_t it[kItems], deep[kItems + 32], far[kItems + 32];  // not compared; equal for 16 bytes; for 32
+  uint32_t batch[kBatch];
+};
+
+// key: (length - 1) << 20 | the candidate's position: the longest match, the nearest on a tie, is the largest
+__device__ __forceinline__ uint32_t k_len(uint32_t key) { return (key >> 20) + 1u; }
+
+// Works the lists off: cnt candidates not compared (W.it), n2 equal for 16 bytes (W.deep), into the slots' keys.
+__device__ __forceinline__ void finish_lists(const ParseBlock& P, Finish& W, uint32_t cnt, uint32_t n2) {
+  const uint32_t lane = lane_id(), below = (1u << lane) - 1u;
+  const uint64_t base = P.base;
+  __syncwarp();
+  // the first 16 bytes, a lane a candidate
+  for (uint32_t k = 0; k < cnt; k += 32) {
+    const bool on = k + lane < cnt;
+    const uint32_t c = on ? W.it[k + lane] : 0u, i = c >> 20, j = c & 0xFFFFFu;
+    bool more = false;
+    if (on) {
+      const uint32_t lim = min(kMaxMatch, P.n - W.x[i]);
+      const uint32_t l = lcp16(load16(P.in, base + j), W.xw[i]);
+      if (l >= 4u) atomicMax(&W.key[i], (min(l, lim) - 1u) << 20 | j);  // (lim >= 4)
+      more = l == 16u && lim > 16u;
+    }
+    const unsigned mm = __ballot_sync(kFull, more);
+    if (more) W.deep[n2 + __popc(mm & below)] = c;
+    n2 += (uint32_t)__popc(mm);
+  }
+  if (!n2) { __syncwarp(); return; }
+  __syncwarp();
+  // the next 16, a lane a candidate
+  uint32_t n3 = 0;
+  for (uint32_t k = 0; k < n2; k += 32) {
+    const bool on = k + lane < n2;
+    const uint32_t c = on ? W.deep[k + lane] : 0u, i = c >> 20, j = c & 0xFFFFFu;
+    const uint32_t x = W.x[i], key = W.key[i], lim = min(kMaxMatch, P.n - x);
+    bool more = false;
+    if (on && !(k_len(key) == lim && j < (key & 0xFFFFFu))) {  // (a nearer match of the whole length cannot be beaten)
+      const uint32_t l = lcp16(load16(P.in, base + j + 16), load16(P.in, base + x + 16));
+      const uint32_t len = min(16u + l, lim);
+      if (len > 16u) atomicMax(&W.key[i], (len - 1u) << 20 | j);
+      more = l == 16u && lim > 32u;
+    }
+    const unsigned mm = __ballot_sync(kFull, more);
+    if (more) W.far[n3 + __popc(mm & below)] = c;
+    n3 += (uint32_t)__popc(mm);
+  }
+  __syncwarp();
+  // The rest: those that can still win are extended, the first one of up to eight requests at a time, four lanes
+  // each, 64 bytes a step, until none is left.  One that is nearer than its request's best wins with the best's
+  // length, a farther one only with more: it is dropped when its byte there differs.
+  const uint32_t g = lane >> 2, gl = lane & 3u;
+  while (n3) {
+    uint32_t m = 0, nb = 0, carry = 32;  // kept ones, this round's, the last kept one's slot
+    for (uint32_t k = 0; k < n3; k += 32) {
+      const bool on = k + lane < n3;
+      const uint32_t c = on ? W.far[k + lane] : 0u, i = c >> 20, j = c & 0xFFFFFu;
+      const uint32_t x = W.x[i], key = W.key[i], lim = min(kMaxMatch, P.n - x);
+      const bool best = j == (key & 0xFFFFFu);  // (the best is here only until it has been extended)
+      const uint32_t at = k_len(key) - (j > (key & 0xFFFFFu) ? 1u : 0u);
+      bool keep = on && at < lim;
+      if (keep && !best) keep = __ldg(P.in + base + j + at) == __ldg(P.in + base + x + at);
+      const unsigned km = __ballot_sync(kFull, keep);
+      const unsigned pm = km & below;
+      const uint32_t pi = __shfl_sync(kFull, i, pm ? 31u - __clz(pm) : 0u);
+      const bool first = keep && (pm ? pi : carry) != i;
+      const unsigned fm = __ballot_sync(kFull, first);
+      const uint32_t fk = nb + __popc(fm & below);
+      const bool sel = first && fk < kBatch;
+      if (sel) W.batch[fk] = c;
+      const unsigned rm = km & ~__ballot_sync(kFull, sel);
+      if (rm >> lane & 1u) W.far[m + __popc(rm & below)] = c;
+      m += (uint32_t)__popc(rm);
+      nb = min(kBatch, nb + (uint32_t)__popc(fm));
+      if (km) carry = __shfl_sync(kFull, i, 31u - __clz(km));
+      __syncwarp();
+    }
+    n3 = m;
+    if (!nb) break;  // (none was kept)
+    bool act = g < nb;
+    const uint32_t c = act ? W.batch[g] : 0u, i = c >> 20, j = c & 0xFFFFFu;
+    const uint32_t x = W.x[i], lim = min(kMaxMatch, P.n - x);
+    const bool mine = act && gl == 0;
+    uint32_t len = 32;
+    for (uint32_t o = 32; __any_sync(kFull, act); o += 64) {
+      const uint32_t q = o + 16u * gl;
+      uint32_t e = lim;  // the match's end, if it lies in this lane's 16 bytes
+      bool stop = act;
+      if (act && q < lim) {
+        const uint32_t l = lcp16(load16(P.in, base + j + q), load16(P.in, base + x + q));
+        e = min(q + l, lim);
+        stop = l < 16u || q + 16u >= lim;
+      }
+      const unsigned sm = __ballot_sync(kFull, stop) >> (4u * g) & 0xFu;
+      const uint32_t v = __shfl_sync(kFull, e, 4u * g + (sm ? (uint32_t)__ffs(sm) - 1u : 0u));
+      if (act && sm) { len = v; act = false; }
+    }
+    if (mine) atomicMax(&W.key[i], (len - 1u) << 20 | j);
+    __syncwarp();
+  }
+  __syncwarp();
+}
+
+// The exact matches at p, where v is unfinished, and at p + 1, where v2 is, for every lane with `act`, by the
+// whole warp; v and v2 get the records, which replace the unfinished ones in minfo.  A position's chain is the
+// entries before its place in the order, nearest first (the order src/codec2.h:58-67 walks them); the longest
+// of the first `depth` wins, the nearest on a tie.  Three rounds:
+//   0  p's nearest candidate (one of the first three entries with its tag), a lane a request, to its full length
+//   1  p's other candidates: one can only win if it is longer, so it must have the 4 bytes of p that end with the
+//      byte after that length; the few that do are compared
+//   2  p + 1's candidates: its match is only needed if it is long enough to replace p's, which happens only if
+//      8 m2 - bitlen(d2) - 8 > 8 m - bitlen(d), so (bitlen(d2) >= 0) only if 8 m2 > 8 m + 8 - bitlen(d): a
+//      candidate must have the 4 bytes that end that shortest match.  When none reaches the length, v2 is NONE and
+//      minfo keeps p + 1 unfinished, marked BELOW.
+// In rounds 1 and 2 a request's chain is one load of its 32 predecessors (four requests a load at depth 8) and one
+// word load a candidate of its tag, four such loads in flight together; the candidates that pass, of all the
+// warp's requests, form one list and are compared a lane each whatever request they belong to.
+// (One request after the other by the whole warp, its 32 candidates a lane each, waited for three to six
+// dependent loads a request: 5.4 us each with 64 warps an SM.  Comparing every candidate of the tag, 16 bytes and
+// on, took 530 warp instructions a token of lz_mix at block 18, level 5.)
+__device__ __forceinline__ void warp_finish(const ParseBlock& P, Finish& W, bool act, uint32_t p, uint32_t& v,
+                                            uint32_t& v2) {
+  const uint32_t lane = lane_id(), below = (1u << lane) - 1u;
+  const uint32_t G = min(32u, P.depth);  // lanes a request: 32, or 8 at depth 8
+  const uint32_t gl = lane & (G - 1u), NR = 32u / G;
+  const bool on0 = act && m_is_sat(v), on1 = act && m_is_sat(v2);
+  const uint32_t r2 = v2 & 0xFFFFFu;
+  uint32_t n2 = 0;
+  __syncwarp();
+  if (__any_sync(kFull, on0)) {
+    bool more = false;
+    uint32_t c = 0;
+    if (on0) {
+      const uint32_t r = v & 0xFFFFFu;
+      const uint32_t e1 = P.srt[r - min(r, 1u)], e2 = P.srt[r - min(r, 2u)], e3 = P.srt[r - min(r, 3u)];
+      const uint4 w = load16(P.in, P.base + p);
+      const uint32_t rt = r | (product(w.x) << 16 & 0xFFF00000u);
+      const uint32_t tag = rt >> 20;
+      const uint32_t e = e_tag(e1) == tag ? e1 : e_tag(e2) == tag ? e2 : e3;
+      const uint32_t j = e_pos(e), lim = min(kMaxMatch, P.n - p);
+      uint32_t key = 0;
+      if (e_tag(e) == tag && j < p) {  // (with fewer than three predecessors, e may be p's own entry)
+        const uint32_t l = lcp16(load16(P.in, P.base + j), w);
+        if (l >= 4u) key = (min(l, lim) - 1u) << 20 | j;
+        more = l == 16u && lim > 16u;
+      }
+      c = lane << 20 | j;
+      W.xw[lane] = w;
+      W.x[lane] = p;
+      W.rt[lane] = rt;
+      W.key[lane] = key;
+    }
+    const unsigned mm = __ballot_sync(kFull, more);
+    if (more) W.deep[__popc(mm & below)] = c;
+    n2 = (uint32_t)__popc(mm);
+  }
+  uint32_t need = 0;
+#pragma unroll 1
+  for (uint32_t ph = 0; ph < 3; ++ph) {
+    bool ask = false;
+    uint32_t at = 0;  // the length that a candidate must exceed (round 1), or reach less one (round 2)
+    if (ph == 1) {
+      if (on0) {
+        const uint32_t key = W.key[lane];
+        at = key ? k_len(key) : 0u;
+        ask = at < min(kMaxMatch, P.n - p);
+      }
+    } else if (ph == 2) {
+      if (on0) {
+        const uint32_t key = W.key[lane];
+        v = key ? m_pack(k_len(key), p - (key & 0xFFFFFu)) : M_NONE;
+        P.minfo[p] = v;
+      }
+      if (on1 && v != M_NONE) {
+        need = ((8u * m_len(v) + 8u - bitlen(m_dist(v))) >> 3) + 1u;
+        at = need - 1u;
+        ask = need <= min(kMaxMatch, P.n - p - 1u);
       }
     }
-    // candidates shorter than 32 bytes (or the whole remaining length): the longest, nearest on a tie
-    uint32_t key = on ? (l << 8) | (31u - lane) : 0u;  // (l <= 32, lanes in chain order)
-    key = __reduce_max_sync(kFull, key);
-    const uint32_t cl = key >> 8, cw = 31u - (key & 0xFFu);
-    const uint32_t jw = __shfl_sync(kFull, j, cw);
-    if (cl > best) { best = cl; bd = x - jw; }
-    if (best == lim) break;
-    // candidates equal for 32 bytes: extended in chain order
-    unsigned ext = __ballot_sync(kFull, on && l == 32u && lim > 32u);
-    while (ext) {
-      // (best >= 32 < lim here) a candidate whose byte at `best` differs from x's is no longer than best:
-      // all such are dropped at once, before the next one in chain order is extended
-      const bool keep = ((ext >> lane) & 1u) && __ldg(P.in + P.base + j + best) == __ldg(P.in + ax + best);
-      ext = __ballot_sync(kFull, keep);
-      if (!ext) break;
-      const uint32_t c = (uint32_t)__ffs(ext) - 1u;
-      ext &= ext - 1u;
-      const uint32_t jc = __shfl_sync(kFull, j, c);
-      const uint64_t aj = P.base + jc;
-      uint32_t len = lim;
-      for (uint32_t o = 32; o < lim; o += 128) {
-        const uint32_t q = o + 4 * lane;
-        uint32_t diff = 0;
-        if (q < lim) diff = load4(P.in, aj + q) ^ load4(P.in, ax + q);
-        const uint32_t nb = q < lim ? (diff ? ((uint32_t)__ffs(diff) - 1u) >> 3 : 4u) : 0u;
-        const bool miss = q < lim && (nb < 4u || q + 4 > lim);
-        const unsigned mm = __ballot_sync(kFull, miss);
-        if (mm) {
-          const uint32_t f = (uint32_t)__ffs(mm) - 1u;
-          const uint32_t qf = o + 4 * f, nf = __shfl_sync(kFull, nb, f);
-          len = min(qf + nf, lim);
-          break;
+    const unsigned am = __ballot_sync(kFull, ask);
+    if (ask) {
+      const uint32_t x = p + ph - 1u, po = max(at, 3u) - 3u;
+      if (ph == 2) {
+        const uint4 w = load16(P.in, P.base + x);
+        W.xw[lane] = w;
+        W.x[lane] = x;
+        W.rt[lane] = r2 | (product(w.x) << 16 & 0xFFF00000u);
+        W.key[lane] = 0;
+      }
+      W.po[lane] = po;
+      W.pw[lane] = load4(P.in, P.base + x + po);
+      W.ord[__popc(am & below)] = lane;
+    }
+    __syncwarp();
+    const uint32_t nreq = (uint32_t)__popc(am);
+    const bool chunks = P.depth > 32;  // (then 8 chunks of 32 entries a request, four of them at a time)
+    const uint32_t nt = chunks ? nreq * (P.depth / 32) : (nreq + NR - 1) / NR;
+    uint32_t t = 0;
+    do {
+      uint32_t cnt = 0;
+      while (t < nt && cnt <= 32) {
+        uint32_t e[kTasks], s[kTasks], w[kTasks];
+        bool hit[kTasks];
+#pragma unroll
+        for (uint32_t u = 0; u < kTasks; ++u) {
+          const uint32_t k = chunks ? (t + u) / (P.depth / 32) : (t + u) * NR + lane / G;
+          const uint32_t q = chunks ? (t + u) % (P.depth / 32) * 32 + lane : gl;
+          s[u] = k < nreq ? W.ord[k] : 0u;
+          const uint32_t rt = k < nreq ? W.rt[s[u]] : 0u, r = rt & 0xFFFFFu;
+          e[u] = q < min(P.depth, r) ? P.srt[r - 1u - q] : ~rt;  // (else: another tag)
+          hit[u] = e[u] - (rt & 0xFFF00000u) < W.x[s[u]];         // the same tag and an earlier position
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < kTasks; ++u)
+          w[u] = hit[u] ? load4(P.in, P.base + e_pos(e[u]) + W.po[s[u]]) : 0u;
+#pragma unroll
+        for (uint32_t u = 0; u < kTasks; ++u) {
+          const bool pass = hit[u] && w[u] == W.pw[s[u]];
+          const unsigned hm = __ballot_sync(kFull, pass);
+          if (pass) W.it[cnt + __popc(hm & below)] = s[u] << 20 | e_pos(e[u]);
+          cnt += (uint32_t)__popc(hm);
+        }
+        t += kTasks;
+        // a deep chain's second half is skipped when it ended in the first: at the order's start, or where the
+        // positions do not fall (entries of other hashes are harmless: their bytes differ)
+        if (chunks && t % (P.depth / 32)) {
+          bool end = false;
+#pragma unroll
+          for (uint32_t u = 0; u < kTasks; ++u) {
+            const uint32_t up = __shfl_up_sync(kFull, e_pos(e[u]), 1);  // (every lane takes part)
+            if (lane > 0 && e_pos(e[u]) >= up) end = true;
+          }
+          const uint32_t r = W.rt[s[0]] & 0xFFFFFu;
+          if (__any_sync(kFull, end) || r <= 32 * kTasks) t += kTasks;
         }
       }
-      if (len > best) {
-        best = len;
-        bd = x - jc;
-        if (best == lim) { stop = true; break; }
-      }
+      finish_lists(P, W, cnt, n2);
+      n2 = 0;
+    } while (t < nt);
+  }
+  if (on1) {
+    v2 = M_NONE;
+    if (need) {
+      const uint32_t key = need <= min(kMaxMatch, P.n - p - 1u) ? W.key[lane] : 0u;
+      uint32_t rec = M_BELOW | r2;  // marked, so a later walk's lazy test skips it
+      if (key && k_len(key) >= need) rec = v2 = m_pack(k_len(key), p + 1 - (key & 0xFFFFFu));
+      P.minfo[p + 1] = rec;
     }
   }
-  if (best < need) {  // (warp-uniform) marked, so a later walk's lazy test skips it
-    __syncwarp();
-    if (lane == 0) P.minfo[x] = M_BELOW | r;
-    __syncwarp();
-    return M_NONE;
-  }
-  const uint32_t e = best < 4 ? M_NONE : m_pack(best, bd);  // (capped records match >= 4 bytes: never NONE)
-  __syncwarp();
-  if (lane == 0) P.minfo[x] = e;
-  __syncwarp();
-  return e;
 }
 
 // One step of the CPU parse (src/codec2.h:69-80) for every lane with `act` (all 32 lanes call it):
 // returns the next position (p itself when !act); the token, when the step emits one, in (ti, tm, td).
-// Capped records at p or p + 1 are finished first, one at a time, by the whole warp.  A position with
-// no match is a literal step to the next position, so a run of them is taken at once, up to `lim` (the
-// walk's end): the walk lands where the CPU parse's single steps would first leave the run or reach lim.
-__device__ __forceinline__ uint32_t warp_step(const ParseBlock& P, uint32_t p, uint32_t lim, bool act, bool& tok,
-                                              uint32_t& ti, uint32_t& tm, uint32_t& td) {
-  uint32_t v = act ? P.minfo[p] : M_NONE;
-  const bool lz = act && v != M_NONE && p + 1 < P.n;
-  uint32_t v2 = lz ? P.minfo[p + 1] : M_NONE;
-  unsigned s1 = __ballot_sync(kFull, act && m_is_sat(v));
-  while (s1) {
-    const uint32_t L = (uint32_t)__ffs(s1) - 1u;
-    s1 &= s1 - 1u;
-    const uint32_t e = coop_exact(P, __shfl_sync(kFull, p, L));
-    if (lane_id() == L) v = e;
+// Positions without a match are literal steps to the next one: a run of them is taken together with the token
+// after it, up to `lim` (the walk's end), where the walk lands if the run reaches it.  A position whose
+// finished record turns out to be NONE is a literal step by itself.
+__device__ __forceinline__ uint32_t warp_step(const ParseBlock& P, Finish& W, uint32_t p, uint32_t lim, bool act,
+                                              bool& tok, uint32_t& ti, uint32_t& tm, uint32_t& td) {
+  uint32_t v = M_NONE, v2 = M_NONE;
+  if (act) {
+    const uint32_t* m = P.minfo;
+    v = m[p];
+    if (v == M_NONE) {
+      ++p;
+      while (p + 4 <= lim) {
+        const uint32_t q0 = m[p], q1 = m[p + 1], q2 = m[p + 2], q3 = m[p + 3];
+        if (q0 != M_NONE) break;
+        if (q1 != M_NONE) { p += 1; break; }
+        if (q2 != M_NONE) { p += 2; break; }
+        if (q3 != M_NONE) { p += 3; break; }
+        p += 4;
+      }
+      while (p < lim && m[p] == M_NONE) ++p;
+      if (p < lim) v = m[p];
+    }
+    if (v != M_NONE && p + 1 < P.n) v2 = m[p + 1];
+    if (m_is_below(v2)) v2 = M_NONE;  // (of no use to p's lazy test)
   }
-  // the match at p + 1 replaces p's only if 8 m2 - bitlen(d2) - 8 > 8 m - bitlen(d), so (bitlen(d2) >= 0)
-  // only if 8 m2 > 8 m + 8 - bitlen(d), m2 >= need; a shorter one is never needed exactly
-  const uint32_t need = lz ? ((8u * m_len(v) + 8u - bitlen(m_dist(v))) >> 3) + 1u : 0u;
-  if (m_is_below(v2)) v2 = M_NONE;
-  unsigned s2 = __ballot_sync(kFull, lz && m_is_sat(v2));
-  while (s2) {
-    const uint32_t L = (uint32_t)__ffs(s2) - 1u;
-    s2 &= s2 - 1u;
-    const uint32_t e = coop_exact(P, __shfl_sync(kFull, p, L) + 1u, __shfl_sync(kFull, need, L));
-    if (lane_id() == L) v2 = e;
-  }
+  if (__any_sync(kFull, m_is_sat(v) || m_is_sat(v2))) warp_finish(P, W, act, p, v, v2);
   tok = false;
   if (!act) return p;
-  if (v == M_NONE) {
-    const uint32_t* m = P.minfo;
-    uint32_t q = p + 1;
-    while (q + 4 <= lim) {
-      const uint32_t a0 = m[q], a1 = m[q + 1], a2 = m[q + 2], a3 = m[q + 3];
-      if (a0 != M_NONE) break;
-      if (a1 != M_NONE) { q += 1; break; }
-      if (a2 != M_NONE) { q += 2; break; }
-      if (a3 != M_NONE) { q += 3; break; }
-      q += 4;
-    }
-    while (q < lim && m[q] == M_NONE) ++q;
-    return q;
-  }
+  if (v == M_NONE) return p < lim ? p + 1 : p;
   uint32_t m = m_len(v), d = m_dist(v), at = p;
-  if (lz && v2 != M_NONE) {
+  if (v2 != M_NONE) {
     const uint32_t m2 = m_len(v2), d2 = m_dist(v2);
     if ((int)(8 * m2) - (int)bitlen(d2) - 8 > (int)(8 * m) - (int)bitlen(d)) { at = p + 1; m = m2; d = d2; }
   }
@@ -645,29 +644,68 @@ __device__ __forceinline__ uint32_t warp_step(const ParseBlock& P, uint32_t p, u
   return at + m;
 }
 
-// One CTA per block, 256 segments of the block, a lane each.  The parse is a chain 0 -> next(0) -> ...;
-// round 0 walks every segment from its own start; each later round re-walks a segment from where the
-// chain before it leaves, until that walk meets the previous one (a two-pointer merge), and rounds end
-// when no segment's exit moves.  Then every segment counts and writes its tokens.  Each warp's 32 walks
-// step together (warp_step), so capped matches are finished by whole warps.
-__global__ void __launch_bounds__(256, 8) k_enc_parse(EncArgs A) {  // (8 CTAs an SM: latency-bound walks)
+// The parse is a chain 0 -> next(0) -> ... cut into A.nseg segments of each block.  Every segment's walk from its
+// own start, a lane a walk: it leaves the exact records of the positions that it visits in minfo, and where it
+// leaves the segment in seg_exit.  A warp, a CTA of its own, takes A.walk_segs consecutive segments of a block and
+// hands the next one to each lane that is done, so its lanes stay busy; no warp waits for another, so a launch of
+// few blocks spreads over the whole GPU.
+__global__ void __launch_bounds__(32, 32) k_enc_walk(EncArgs A) {
+  __shared__ Finish W;
+  const uint32_t lane = lane_id();
+  const uint32_t per = A.nseg / A.walk_segs, b = blockIdx.x / per;
+  const uint32_t n = A.in_len[b];
+  const size_t so = (size_t)b * A.B;
+  ParseBlock P;
+  P.in = A.in; P.base = A.in_off[b]; P.n = n; P.depth = (uint32_t)A.depth;
+  P.minfo = A.minfo + so; P.srt = A.srt + so;
+  uint32_t* out = A.seg_exit + (size_t)b * A.nseg;
+  const uint32_t S = seg_bytes(n, A.nseg);
+  uint32_t next = (blockIdx.x % per) * A.walk_segs;  // the next segment to hand out (warp-uniform)
+  const uint32_t last = next + A.walk_segs;
+  uint32_t q = next + lane;
+  next += 32;
+  uint32_t p = min(q * S, n), e = min(p + S, n);
+  bool t; uint32_t ta, tc, td;
+  for (;;) {
+    bool on = p < e;
+    // done: the exit is written, and the next segment taken (one past the block's end is empty)
+    for (;;) {
+      const unsigned done = __ballot_sync(kFull, !on && q < last);
+      if (!done) break;
+      if (!on && q < last) {
+        out[q] = p;
+        q = next + __popc(done & ((1u << lane) - 1u));
+        p = min(q * S, n);
+        e = min(p + S, n);
+        if (q >= last) e = p;
+        on = p < e;
+      }
+      next += (uint32_t)__popc(done);
+    }
+    if (!__any_sync(kFull, on)) break;
+    p = warp_step(P, W, p, e, on, t, ta, tc, td);
+  }
+}
+
+// One CTA per block, a lane a segment.  Rounds re-walk each segment from where the chain before it leaves, until
+// that walk meets the previous one (a two-pointer merge), and end when no segment's exit moves.  Then every
+// segment counts and writes its tokens.  Most records that these walks read were finished by k_enc_walk.
+template <uint32_t T>
+__global__ void __launch_bounds__(T, 1024 / T) k_enc_parse(EncArgs A) {
   const uint32_t b = blockIdx.x, q = threadIdx.x;
   const uint32_t n = A.in_len[b];
   const size_t so = (size_t)b * A.B;
-  __shared__ uint32_t ent[256], ex[256], wsum[8];
+  __shared__ uint32_t ent[T], ex[T], wsum[T / 32];
+  extern __shared__ uint4 parse_sm[];
+  Finish& W = reinterpret_cast<Finish*>(parse_sm)[q >> 5];
   ParseBlock P;
   P.in = A.in; P.base = A.in_off[b]; P.n = n; P.depth = (uint32_t)A.depth;
-  P.minfo = A.minfo + so; P.spos = A.srt_pos + so; P.sh = A.srt_h + so;
-  const uint32_t S = max(1u, (n + 255) / 256);
+  P.minfo = A.minfo + so; P.srt = A.srt + so;
+  const uint32_t S = seg_bytes(n, T);
   const uint32_t s = min(q * S, n), e = min(s + S, n);
   bool t; uint32_t ta, tc, td;
-  // round 0: every segment walked from its own start
-  {
-    uint32_t p = s;
-    while (__any_sync(kFull, p < e)) p = warp_step(P, p, e, p < e, t, ta, tc, td);
-    ent[q] = s;
-    ex[q] = s < e ? p : s;
-  }
+  ent[q] = s;
+  ex[q] = A.seg_exit[(size_t)b * T + q];
   // rounds: each segment re-walked from where the chain before it leaves, until it meets its old walk
   for (;;) {
     __syncthreads();
@@ -685,7 +723,7 @@ __global__ void __launch_bounds__(256, 8) k_enc_parse(EncArgs A) {  // (8 CTAs a
     }
     while (__any_sync(kFull, mode != 0)) {
       const bool adv_a = mode == 1 || (mode == 2 && a < c);
-      const uint32_t y = warp_step(P, adv_a ? a : c, e, mode != 0, t, ta, tc, td);
+      const uint32_t y = warp_step(P, W, adv_a ? a : c, e, mode != 0, t, ta, tc, td);
       if (mode == 1) {
         a = y;
         if (a >= e) { nx = a; mode = 0; }
@@ -710,7 +748,7 @@ __global__ void __launch_bounds__(256, 8) k_enc_parse(EncArgs A) {  // (8 CTAs a
   uint32_t* gd = gm + seg_tok_cap(A.B);
   uint32_t cnt = 0;
   for (uint32_t p = from; __any_sync(kFull, p < e);) {
-    p = warp_step(P, p, e, p < e, t, ta, tc, td);
+    p = warp_step(P, W, p, e, p < e, t, ta, tc, td);
     if (t) { gi[cnt] = ta; gm[cnt] = tc; gd[cnt] = td; ++cnt; }
   }
   const uint32_t incl = warp_incl_scan(cnt);
@@ -720,7 +758,7 @@ __global__ void __launch_bounds__(256, 8) k_enc_parse(EncArgs A) {  // (8 CTAs a
   for (uint32_t k = 0; k < (q >> 5); ++k) off += wsum[k];
   const size_t to = (size_t)b * tok_cap(A.B) + off;
   for (uint32_t k = 0; k < cnt; ++k) { A.tk_i[to + k] = gi[k]; A.tk_m[to + k] = gm[k]; A.tk_d[to + k] = gd[k]; }
-  if (q == 255) A.bcnt[b * 8 + 0] = off + cnt;
+  if (q == T - 1) A.bcnt[b * 8 + 0] = off + cnt;
 }
 
 // ---------------------------------------------------------------- 4. tokens -> streams
@@ -1239,16 +1277,10 @@ __global__ void __launch_bounds__(256) k_enc_emit(EncArgs A) {
   for (uint32_t k = i + threadIdx.x; k < len; k += blockDim.x) d[k] = s[k];
 }
 
-size_t match_smem_bytes(uint32_t tile, uint32_t depth, uint32_t wb) {
-  return (size_t)(tile + depth) * (wb + 4 + 2) + 4 + (size_t)tile * 8;  // (+ the work list)
-}
-
 cudaError_t prepare_kernels() {  // with the device current, once per context
-  cudaError_t e = cudaFuncSetAttribute(k_enc_match<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)match_smem_bytes(kMaxMatchTile, 256, 32));
+  cudaError_t e = cudaFuncSetAttribute(k_enc_parse<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, 512 / 32 * sizeof(Finish));
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_enc_match<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)match_smem_bytes(kMaxMatchTile, 256, 16));
+    e = cudaFuncSetAttribute(k_enc_parse<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, 1024 / 32 * sizeof(Finish));
   return e == cudaSuccess ? prepare_fill() : e;
 }
 
@@ -1274,13 +1306,17 @@ void launch_encode(const EncArgs& A, const CrcArgs& crc_in, cudaStream_t st, Sta
   S.begin("k_sort_scatter", st);
   k_sort_scatter<1><<<sg, kSortThreads, 0, st>>>(A);
   S.end(st);
-  S.begin("k_enc_match", st);
-  const dim3 mg((A.B + A.match_tile - 1) / A.match_tile, A.nb);
-  if (A.cmp_cap <= 16) k_enc_match<16><<<mg, 256, match_smem_bytes(A.match_tile, (uint32_t)A.depth, 16), st>>>(A);
-  else k_enc_match<32><<<mg, 256, match_smem_bytes(A.match_tile, (uint32_t)A.depth, 32), st>>>(A);
+  S.begin("k_enc_chain", st);
+  k_enc_chain<<<dim3((A.B + kChainTile - 1) / kChainTile, A.nb), 256, 0, st>>>(A);
+  S.end(st);
+  S.begin("k_enc_walk", st);
+  k_enc_walk<<<A.nb * (A.nseg / A.walk_segs), 32, 0, st>>>(A);
   S.end(st);
   S.begin("k_enc_parse", st);
-  k_enc_parse<<<A.nb, 256, 0, st>>>(A);
+  const size_t fin = A.nseg / 32 * sizeof(Finish);
+  if (A.nseg == 256) k_enc_parse<256><<<A.nb, 256, fin, st>>>(A);
+  else if (A.nseg == 512) k_enc_parse<512><<<A.nb, 512, fin, st>>>(A);
+  else k_enc_parse<1024><<<A.nb, 1024, fin, st>>>(A);
   S.end(st);
   S.begin("k_enc_streams", st);
   k_enc_streams<<<(A.nb + 3) / 4, 128, 0, st>>>(A);

@@ -67,8 +67,8 @@ struct GraphEntry {
   uint64_t launches;  // kernels in the graph
 };
 
-// per (block size, level class) launch shapes: the fill's ring, warps per CTA and words a lane a round,
-// the match pass's compare cap and tile (none of them changes a result byte)
+// per (block size, level class) launch shapes: the fill's ring, warps per CTA and words a lane a round; the
+// match fields are kept for callers that set them (none of them changes a result byte)
 struct Shape {
   uint32_t ring_log = 12, fill_warps = 4, cmp_cap = 16, match_tile = 1024, fill_words = 1, match_dense = 256,
            match_defer = 3;
@@ -89,7 +89,7 @@ struct zc_ctx {
   zch::StageRecords records;
   zc::CrcTables* d_crct = nullptr;
   // encoder scratch (sized by capacity: any block size whose blocks fit)
-  zch::DevBuf e_tmp_pos, e_srt_pos, e_minfo, e_scnt, e_tk_seg, e_tmp_h, e_srt_h, e_tk_i, e_tk_m, e_tk_d, e_bcnt, e_lit, e_tok,
+  zch::DevBuf e_tmp, e_tmp_d, e_srt, e_minfo, e_scnt, e_tk_seg, e_seg, e_tk_i, e_tk_m, e_tk_d, e_bcnt, e_lit, e_tok,
       e_ext, e_sym, e_grp, e_bits, e_lanes, e_freq, e_lanelen, e_sinfo, e_slab;
   // decoder scratch (likewise)
   zch::DevBuf d_lit, d_tok, d_sym, d_grp, d_ext, d_meta, d_tks, d_tkm, d_tkd, d_tkl;

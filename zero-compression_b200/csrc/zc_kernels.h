@@ -74,16 +74,15 @@ struct EncArgs {
   const uint32_t* in_len;
   uint32_t nb, B, block_log;
   int depth;                  // hash chain steps (8 / 32 / 256)
-  uint32_t cmp_cap;           // bytes the all-position match pass compares before deferring to the parse
-  uint32_t match_tile;        // sorted positions per match CTA: 256, 512 or 1024
-  uint32_t match_dense;       // unfinished positions from which a match tile scans a lane per position
-  uint32_t match_defer;       // backward bytes that mark a position as inside a longer match (0: none)
   // scratch, per block slot (capacity B positions)
-  uint32_t *tmp_pos, *srt_pos, *minfo;
+  uint32_t *tmp_e, *srt, *minfo;  // sort entries after pass 0 and in order; match records
+  uint8_t* tmp_d;                 // the entries' digits of pass 1, beside tmp_e
   uint32_t* scnt;                 // sort: per block ceil(B / 4096) * 256 tile digit counts / starts
-  uint16_t *tmp_h, *srt_h;
   uint32_t *tk_i, *tk_m, *tk_d;   // tokens, tok_cap(B) per block
   uint32_t* tk_seg;               // the parse's per-segment token slots: 3 * seg_tok_cap(B) per block
+  uint32_t nseg;                  // segments a block is parsed in: 256, 512 or 1024
+  uint32_t walk_segs;             // of those, how many a warp of k_enc_walk takes: 32 or 64
+  uint32_t* seg_exit;             // where each segment's first walk leaves it: nseg per block
   uint32_t* bcnt;                 // per block [8]: nt, nl, ne, nob, ng, payload size, method
   uint8_t *s_lit, *s_tok, *s_ext, *s_sym, *s_grp, *s_bits;
   uint8_t* lanes;                 // rANS lane scratch, lanes_per_block(B) per block
@@ -122,12 +121,16 @@ __host__ __device__ inline uint64_t lane_base(uint32_t B, uint32_t s) {
 }
 __host__ __device__ inline uint64_t lanes_per_block(uint32_t B) { return lane_base(B, 5); }
 __host__ __device__ inline uint32_t bits_cap(uint32_t B) { return 5 * B / 8 + 64; }
-// the parse's token slots per block: 256 segments of ceil(B / 256) bytes, ceil(B / 256) / 4 + 2 each
-__host__ __device__ inline uint32_t seg_tok_cap(uint32_t B) { return 256 * (((B + 255) / 256) / 4 + 2); }
+// the parse's segments: ceil(n / nseg) bytes each, at least kMinSeg; their token slots per block: a token takes at
+// least 4 bytes, so a segment of S bytes has at most S / 4 + 1, S / 4 + 2 slots are kept for it, and nseg <= 1024
+constexpr uint32_t kMaxSegs = 1024, kMinSeg = 64;
+__host__ __device__ inline uint32_t seg_bytes(uint32_t n, uint32_t nseg) {
+  const uint32_t s = (n + nseg - 1) / nseg;
+  return s > kMinSeg ? s : kMinSeg;
+}
+__host__ __device__ inline uint32_t seg_tok_cap(uint32_t B) { return B / 4 + 2 * kMaxSegs; }
 
 void launch_encode(const EncArgs& A, const CrcArgs& crc_in, cudaStream_t st, Stages& S);
-constexpr uint32_t kMaxMatchTile = 1024;
-size_t match_smem_bytes(uint32_t tile, uint32_t depth, uint32_t window_bytes);
 cudaError_t prepare_kernels();
 cudaError_t prepare_fill();  // per-kernel attributes (the sort's shared memory), the device current
 
