@@ -138,8 +138,8 @@ int ensure_dec(zc_ctx* c, uint32_t nb, uint32_t block_log) {
   Need need[] = {
       {&c->d_lit, (size_t)nb * B}, {&c->d_tok, (size_t)nb * TC}, {&c->d_sym, (size_t)nb * TC},
       {&c->d_grp, (size_t)nb * TC}, {&c->d_ext, (size_t)nb * EC}, {&c->d_meta, (size_t)nb * sizeof(zc::DecMeta)},
-      {&c->d_tks, (size_t)nb * TC * 4}, {&c->d_tkm, (size_t)nb * TC * 4}, {&c->d_tkd, (size_t)nb * TC * 4},
-      {&c->d_tkl, (size_t)nb * TC * 4}};
+      {&c->d_tkp, (size_t)nb * TC * 8}, {&c->d_tkd, (size_t)nb * TC * 4},
+      {&c->d_line, (size_t)nb * zc::line_cap((uint32_t)B) * 8}};
   return ensure(c, need);
 }
 
@@ -229,8 +229,7 @@ int decode_device(zc_ctx* c, const uint8_t* d_comp, const uint64_t* d_comp_offs,
   A.nb = nb; A.B = 1u << block_log; A.out = d_out; A.out_off = d_out_offs; A.err = d_err;
   A.s_lit = c->d_lit.as<uint8_t>(); A.s_tok = c->d_tok.as<uint8_t>(); A.s_sym = c->d_sym.as<uint8_t>();
   A.s_grp = c->d_grp.as<uint8_t>(); A.s_ext = c->d_ext.as<uint8_t>(); A.meta = c->d_meta.as<zc::DecMeta>();
-  A.tk_start = c->d_tks.as<uint32_t>(); A.tk_ms = c->d_tkm.as<uint32_t>(); A.tk_d = c->d_tkd.as<uint32_t>();
-  A.tk_lik = c->d_tkl.as<uint32_t>();
+  A.tk_pos = c->d_tkp.as<uint2>(); A.tk_d = c->d_tkd.as<uint32_t>(); A.line = c->d_line.as<uint2>();
   const Shape& sh = c->shape[block_log - zc::kMinBlockLog][level_class(c->level)];
   A.ring_log = sh.ring_log; A.fill_warps = sh.fill_warps; A.fill_words = sh.fill_words;
   A.work = c->work.as<uint32_t>() + 1;
@@ -448,7 +447,7 @@ void zc_close(zc_ctx* c) {
   for (DevBuf* b : {&c->e_tmp, &c->e_tmp_d, &c->e_srt, &c->e_minfo, &c->e_scnt, &c->e_tk_seg, &c->e_seg, &c->e_tk_i,
                     &c->e_tk_m, &c->e_tk_d, &c->e_bcnt, &c->e_lit, &c->e_tok, &c->e_ext, &c->e_sym, &c->e_grp,
                     &c->e_bits, &c->e_lanes, &c->e_freq, &c->e_lanelen, &c->e_sinfo, &c->e_slab, &c->d_lit, &c->d_tok,
-                    &c->d_sym, &c->d_grp, &c->d_ext, &c->d_meta, &c->d_tks, &c->d_tkm, &c->d_tkd, &c->d_tkl, &c->s_in, &c->s_blk, &c->s_out, &c->s_meta, &c->work,
+                    &c->d_sym, &c->d_grp, &c->d_ext, &c->d_meta, &c->d_tkp, &c->d_tkd, &c->d_line, &c->s_in, &c->s_blk, &c->s_out, &c->s_meta, &c->work,
                     &c->a_desc, &c->a_work})
     release(*b);
   if (c->h_meta.p) cudaFreeHost(c->h_meta.p);

@@ -2,15 +2,17 @@
 //
 //   k_dec_tokens  one CTA of 1024 threads per block: every token's literal run and match length (ext
 //                 bytes), offset (offset bits), output start and literal start, from block-wide scans, in
-//                 parallel over the tokens; then the groups (a scan of their counts) and the recent-offset
-//                 symbols (each names an earlier token's offset, src/codec2.h:180-192), resolved by pointer
-//                 jumping over all tokens at once.  Every check of the reference decoder is made here; a
-//                 failing one records a status and the block is not replayed.
+//                 parallel over the tokens; which token holds each 128-byte line's first byte; then the groups
+//                 (a scan of their counts) and the recent-offset symbols (each names an earlier token's offset,
+//                 src/codec2.h:180-192), resolved by pointer jumping over all tokens at once.  Every check of the
+//                 reference decoder is made here; a failing one records a status and the block is not replayed.
 //   k_dec_fill    one warp per block: fills the block in rounds of 128 output bytes (a 4-byte word a lane)
 //                 straight through, group boundaries or not: a byte whose source lies earlier in the same
 //                 round is passed along by shuffles once known; the token table is a 64-row ring in shared
 //                 memory, refilled 32 tokens at a time from registers loaded one window ahead.
-// Stored blocks are copied by k_dec_fill.  The rANS streams come from k_dec_streams (zc_decode.cu).
+//   k_dec_fill_multi  the same with several warps a block, a line each, for launches of few blocks: words wait for
+//                 their source words, which are published in shared memory.
+// Stored blocks are copied by the fill.  The rANS streams come from k_dec_streams (zc_decode.cu).
 #include <algorithm>
 
 #include "zc_internal.cuh"
@@ -43,6 +45,15 @@ __device__ __forceinline__ uint32_t cta_scan(uint32_t v, uint32_t* ws, uint32_t&
 
 constexpr uint32_t kRepMark = 0x80000000u;  // a recent-offset symbol not resolved yet: kRepMark | index
 constexpr uint32_t kGrpStart = 0x40000000u; // (while groups are scanned) the first token of a group
+
+// A token's row: its output start and its literals' start before it (21 bits each: start - literal start is never
+// negative), and its literal count (21 bits, split over the two words' upper bits).
+__device__ __forceinline__ uint2 tok_row(uint32_t start, uint32_t lits, uint32_t lit0) {
+  return make_uint2((start & 0x1FFFFFu) | lits << 21, ((start - lit0) & 0x1FFFFFu) | lits >> 11 << 21);
+}
+__device__ __forceinline__ uint32_t row_start(const uint2& r) { return r.x & 0x1FFFFFu; }
+__device__ __forceinline__ uint32_t row_back(const uint2& r) { return r.y & 0x1FFFFFu; }  // start - literal start
+__device__ __forceinline__ uint32_t row_lits(const uint2& r) { return r.x >> 21 | r.y >> 21 << 11; }
 
 // inclusive max over the CTA in thread order (blockDim.x == 1024); `total` gets the CTA's max.  ws: 33 words
 __device__ __forceinline__ uint32_t cta_max_incl(uint32_t v, uint32_t* ws, uint32_t& total) {
@@ -87,10 +98,12 @@ __global__ void __launch_bounds__(1024, 2) k_dec_tokens(DecArgs A) {
   const uint8_t* ext = A.s_ext + (size_t)b * EC;
   const uint8_t* bits = A.comp + A.comp_off[b] + m.bits_off;
   const uint64_t nbits = 8ull * m.nob;
-  uint32_t* Ts = A.tk_start + (size_t)b * TC;
-  uint32_t* Tm = A.tk_ms + (size_t)b * TC;
+  uint2* Tp = A.tk_pos + (size_t)b * TC;
   uint32_t* Td = A.tk_d + (size_t)b * TC;
-  uint32_t* Tl = A.tk_lik + (size_t)b * TC;
+  uint2* line = A.line ? A.line + (size_t)b * line_cap(B) : nullptr;  // (none for one warp a block)
+  const uint32_t al = (uint32_t)(uintptr_t)(A.out + A.out_off[b]) & 127u;  // output byte q lies in line (q + al) / 128
+  if (line)
+    for (uint32_t k = tid; k < (raw + al + 127u) >> 7; k += 1024) line[k] = make_uint2(0, 0);
   if (tid == 0) any_bad = 0;
   __syncthreads();
   // ---- lengths, offsets and positions, 1024 tokens a tile
@@ -134,12 +147,21 @@ __global__ void __launch_bounds__(1024, 2) k_dec_tokens(DecArgs A) {
     const uint32_t opre = cta_scan(L + M, ws, osum);
     const uint32_t opk = op + opre, lik = li + lpre;
     if (on && ((uint64_t)lik + L > m.nl || (uint64_t)opk + L + M > raw)) bad = true;
-    if (on) { Ts[t] = opk; Tm[t] = opk + L; Tl[t] = lik; Td[t] = D; }
+    if (on) { Tp[t] = tok_row(opk, L, lik); Td[t] = D; }
+    if (line && on && !bad) {  // the lines whose first byte the token holds, and its own start inside a line
+      for (uint32_t k = (opk + al + 127u) >> 7; k < (opk + L + M + al + 127u) >> 7; ++k) line[k].x = t;
+      if (t && ((opk + al) & 127u)) atomicOr(&line[(opk + al) >> 7].y, 1u << ((opk + al) >> 2 & 31u));
+    }
     op += osum;
     li += lsum;
   }
   if (bad) any_bad = 1;
   __syncthreads();
+  if (tid == 0) { Tp[m.nt] = tok_row(op, raw - op, li); Td[m.nt] = 1; }  // token nt: the literal tail
+  if (line && !any_bad && op < raw) {  // the literal tail's lines and start (a line 0 that starts before the output: token 0)
+    for (uint32_t k = ((op + al + 127u) >> 7) + tid; k < (raw + al + 127u) >> 7; k += 1024) line[k].x = m.nt;
+    if (tid == 0 && op && ((op + al) & 127u)) atomicOr(&line[(op + al) >> 7].y, 1u << ((op + al) >> 2 & 31u));
+  }
   // ---- groups and recent offsets (src/codec2.h:179-199).  A recent-offset symbol r of a group whose first
   //      token is gs names the offset of token gs - 1 - r (the last three offsets before the group,
   //      nearest first), or the initial 1, 4, 8 when r >= gs.  So: group starts (a scan of the group
@@ -196,7 +218,8 @@ __global__ void __launch_bounds__(1024, 2) k_dec_tokens(DecArgs A) {
     }
     for (uint32_t t = tid; t < m.nt; t += 1024) {
       const uint32_t D = Td[t];
-      if ((D & kRepMark) || D == 0 || D > Tm[t]) bad = true;
+      const uint2 r = Tp[t];
+      if ((D & kRepMark) || D == 0 || D > row_start(r) + row_lits(r)) bad = true;
     }
     if (bad) any_bad = 1;
   }
@@ -227,18 +250,18 @@ __host__ __device__ constexpr uint32_t fill_flag_bytes(uint32_t wpl) { return 12
 
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
-__device__ inline void copy_bytes(uint8_t* d, const uint8_t* s, uint32_t n) {  // all lanes; no overlap
-  const uint32_t l = lane_id();
+// thread l of nth copies its share; no overlap
+__device__ inline void copy_bytes(uint8_t* d, const uint8_t* s, uint32_t n, uint32_t l, uint32_t nth) {
   uint32_t i = 0;
   if ((((uintptr_t)d ^ (uintptr_t)s) & 15u) == 0) {
     const uint32_t head = (uint32_t)((16u - ((uintptr_t)d & 15u)) & 15u);
     if (l < head && l < n) d[l] = s[l];
     i = head < n ? head : n;
-    for (uint32_t j = i + 16 * l; j + 16 <= n; j += 16 * 32)
+    for (uint32_t j = i + 16 * l; j + 16 <= n; j += 16 * nth)
       *reinterpret_cast<uint4*>(d + j) = *reinterpret_cast<const uint4*>(s + j);
     i += (n - i) & ~15u;
   }
-  for (uint32_t j = i + l; j < n; j += 32) d[j] = s[j];
+  for (uint32_t j = i + l; j < n; j += nth) d[j] = s[j];
 }
 
 }  // namespace
@@ -267,7 +290,7 @@ __device__ __forceinline__ void fill_block(const DecArgs& A, uint32_t b, FillTab
   if (raw > B) { if (lane == 0) flag(A.err, b, E_RAWLEN); return; }
   if (method == 0) {
     if (clen != raw) { if (lane == 0) flag(A.err, b, E_STORED); return; }
-    copy_bytes(o, p, raw);
+    copy_bytes(o, p, raw, lane, 32);
     return;
   }
   if (method != 1) { if (lane == 0) flag(A.err, b, E_METHOD); return; }
@@ -276,10 +299,8 @@ __device__ __forceinline__ void fill_block(const DecArgs& A, uint32_t b, FillTab
   const uint32_t nt = m.nt, op_total = m.op_total, li_total = m.li_total;
   const size_t TC = tok_cap(B);
   const uint8_t* lit = A.s_lit + (size_t)b * B;
-  const uint32_t* Ts = A.tk_start + (size_t)b * TC;
-  const uint32_t* Tm = A.tk_ms + (size_t)b * TC;
+  const uint2* Tp = A.tk_pos + (size_t)b * TC;
   const uint32_t* Td = A.tk_d + (size_t)b * TC;
-  const uint32_t* Tl = A.tk_lik + (size_t)b * TC;
   const uint32_t ob = (uint32_t)(uintptr_t)o;
   // rows for tokens committed so far: [loaded - TR, loaded); row TR - 1 first holds a token "-1" (no byte
   // uses it).  The next 32 tokens wait in registers (lane k: token loaded + k), fetched one window ahead;
@@ -290,10 +311,10 @@ __device__ __forceinline__ void fill_block(const DecArgs& A, uint32_t b, FillTab
     const uint32_t t = base + lane;
     ns = 0xFFFFFFFFu; nm = 0xFFFFFFFFu; nd = 1; nl = 0;
     if (t < nt) {
-      ns = Ts[t]; nm = Tm[t]; nd = Td[t];
-      const uint32_t lk = Tl[t];
-      nl = lk - ns;
-      prefetch_l2(lit + lk);
+      const uint2 r = Tp[t];
+      nd = Td[t];
+      ns = row_start(r); nm = ns + row_lits(r); nl = 0u - row_back(r);
+      prefetch_l2(lit + (ns + nl));
       if (nd >= R) {
         prefetch_l2(o + (nm - nd));
         prefetch_l2(o + (nm - nd) + 128);
@@ -436,6 +457,226 @@ __global__ void __maxnreg__(72) k_dec_fill(DecArgs A) {  // (72 registers: 28 wa
   }
 }
 
+// ---- several warps a block
+// With fewer blocks than the GPU has room for warps, one warp a block leaves it idle and takes a block's 2^block_log
+// / 128 rounds one after the other (about 0.8 us each: 1.6 ms for 256 KiB).  Here the CTA's NW warps share a block:
+// warp w fills the 128-byte lines w, w + NW, ..., each looked up by itself in the token table (DecArgs.line gives
+// the token that holds a line's first byte).  A word's bytes from literals and from lines that are complete are
+// loaded at once; the others wait for their source words.  state[v] is the line that warp v is at, with a bit for
+// each word of it that is done: a source word is there once its line lies below its warp's, or is its warp's
+// line with the word's bit set.  A word's sources lie before it (or earlier in the word itself), so the first
+// word not done never waits for another: all of them end; the polls are bounded all the same.
+//
+// Recent output is read from a ring of kMultiRing lines a warp.  A warp starts a line only within kMultiAhead * NW
+// lines of the lowest incomplete one; a line then overwrites none that a warp may still read (a source at most
+// (kMultiRing - kMultiAhead) * NW lines back is read from the ring, a farther one from the output itself, which
+// its warp stored before it published its next line).
+constexpr uint32_t kMultiWarps = 16, kMultiRing = 16, kMultiAhead = 4;
+constexpr uint32_t kMultiPoll = 1u << 24;  // polls before a warp gives up
+__host__ __device__ constexpr size_t multi_smem(uint32_t nw) { return nw * kMultiRing * 128; }
+
+// a warp's state, read and published in the order of the CTA's memory: what was stored before it was published is
+// there for who has read it
+__device__ __forceinline__ uint64_t load_state(const uint64_t* p) {
+  uint64_t v;
+  asm volatile("ld.acquire.cta.shared.u64 %0, [%1];" : "=l"(v) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+  return v;
+}
+__device__ __forceinline__ void store_state(uint64_t* p, uint64_t v) {
+  asm volatile("st.release.cta.shared.u64 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(p)), "l"(v) : "memory");
+}
+
+__global__ void __launch_bounds__(32 * kMultiWarps, 2) k_dec_fill_multi(DecArgs A) {
+  extern __shared__ __align__(16) uint8_t fsm[];
+  __shared__ uint32_t next;
+  __shared__ uint64_t state[kMultiWarps];
+  const uint32_t NW = blockDim.x >> 5, w = threadIdx.x >> 5, lane = lane_id();
+  const uint32_t RB = kMultiRing * 128 * NW, rmask = RB - 1u;
+  uint8_t* ring = fsm;
+  const uint32_t upto = 0xFFFFFFFFu >> (31u - lane);
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) next = atomicAdd(A.work, 1u);
+    if (threadIdx.x < kMultiWarps) state[threadIdx.x] = (uint64_t)threadIdx.x << 32;
+    __syncthreads();
+    const uint32_t b = next;
+    if (b >= A.nb) break;
+    const uint32_t raw = A.raw_len[b], method = A.method[b], clen = A.comp_len[b], B = A.B;
+    uint8_t* o = A.out + A.out_off[b];
+    if (raw > B || method > 1 || (method == 0 && clen != raw)) {
+      if (threadIdx.x == 0) flag(A.err, b, raw > B ? E_RAWLEN : method > 1 ? E_METHOD : E_STORED);
+      continue;
+    }
+    if (method == 0) {
+      copy_bytes(o, A.comp + A.comp_off[b], raw, threadIdx.x, blockDim.x);
+      continue;
+    }
+    if (A.err[b]) continue;
+    const DecMeta& m = A.meta[b];
+    const size_t TC = tok_cap(B);
+    const uint8_t* lit = A.s_lit + (size_t)b * B;
+    const uint2* Tp = A.tk_pos + (size_t)b * TC;
+    const uint32_t* Td = A.tk_d + (size_t)b * TC;
+    const uint2* line = A.line + (size_t)b * line_cap(B);
+    const uint32_t a = (uint32_t)(uintptr_t)o & 127u;  // output byte q lies in line (q + a) / 128
+    const uint32_t NL = (raw + a + 127u) >> 7;
+    const uint32_t back = (kMultiRing - kMultiAhead) * NW - 1u;  // lines before a line that the ring holds
+    // The lane's word of a line: its last byte's token (row 1) and, where a token starts in the word, the one before
+    // (row 0; the same one otherwise).  Loaded a line ahead.
+    uint2 p1, p0;
+    uint32_t d1, d0;
+    auto fetch = [&](const uint2& l) {
+      const uint32_t t1 = l.x + __popc(l.y & upto), t0 = t1 - (l.y >> lane & 1u);
+      p1 = Tp[t1]; d1 = Td[t1];  // (t1 <= nt)
+      p0 = Tp[t0]; d0 = Td[t0];
+    };
+    const uint2 none = make_uint2(m.nt, 0);
+    uint2 lt = w < NL ? line[w] : none;
+    fetch(lt);
+    lt = w + NW < NL ? line[w + NW] : none;
+    bool dead = false;
+    for (uint32_t ln = w; ln < NL; ln += NW) {
+      const uint32_t st1 = row_start(p1), st0 = row_start(p0);
+      const uint32_t ms1 = st1 + row_lits(p1), ms0 = st0 + row_lits(p0);
+      const uint32_t bk1 = row_back(p1), bk0 = row_back(p0), D1 = d1, D0 = d0;
+      fetch(lt);
+      lt = ln + 2 * NW < NL ? line[ln + 2 * NW] : none;
+      // the lowest incomplete line; this one starts once it lies within the window
+      uint32_t low;
+      for (uint32_t k = 0;; ++k) {
+        low = __reduce_min_sync(kFull, lane < NW ? (uint32_t)(load_state(&state[lane]) >> 32) : 0xFFFFFFFFu);
+        if (ln < low + kMultiAhead * NW) break;
+        if (k > kMultiPoll) { dead = true; break; }
+      }
+      if (dead) break;
+      __syncwarp();
+      const int32_t lb = (int32_t)(ln << 7) - (int32_t)a;
+      const int32_t q0 = lb + 4 * (int32_t)lane;
+      const int32_t rlo = lb - (int32_t)(back << 7);
+      // A byte's source: itself for a literal, D before it for a match byte, its period's start for one that repeats
+      // the match's own bytes (q - D - D * (x / D), x its offset in the match, x >= D: few lines hold one).  Bytes
+      // from a token's own literals are read from the literals.
+      uint32_t v[4], s[4], wait = 0, over = 0;  // bit j of wait: byte j's source may not be there yet
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t q = (uint32_t)(q0 + j);
+        const bool hi = q >= st1;
+        const uint32_t ms = hi ? ms1 : ms0, D = hi ? D1 : D0;
+        const int32_t x = (int32_t)(q - ms);
+        s[j] = x >= 0 ? q - D : q;
+        over |= (uint32_t)(x >= (int32_t)D) << j;
+      }
+      if (__any_sync(kFull, over)) {
+        // x / D for x, D < 2^20 by a float product, at most one too low; then D's multiples for the later bytes
+        const uint32_t x1 = (uint32_t)max(q0 - (int32_t)ms1, 0), x0 = (uint32_t)max(q0 - (int32_t)ms0, 0);
+        const uint32_t k1 = (uint32_t)__fdividef((float)x1, (float)D1) * D1;
+        const uint32_t k0 = (uint32_t)__fdividef((float)x0, (float)D0) * D0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t q = (uint32_t)(q0 + j);
+          const bool hi = q >= st1;
+          const uint32_t ms = hi ? ms1 : ms0, D = hi ? D1 : D0;
+          uint32_t r = q - ms - (hi ? k1 : k0);
+#pragma unroll
+          for (int t = 0; t < 4; ++t) r = r >= D ? r - D : r;
+          if (over >> j & 1u) s[j] = ms - D + r;
+        }
+      }
+      const int32_t lows = (int32_t)(low << 7) - (int32_t)a;  // the first output byte that may not be there
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int32_t qi = q0 + j;
+        const bool valid = qi >= 0 && qi < (int32_t)raw;
+        const bool hi = (uint32_t)qi >= st1;
+        const bool own = s[j] >= (hi ? st1 : st0);
+        const bool later = !own && (int32_t)s[j] >= lows;
+        const bool near = !own && (int32_t)s[j] >= rlo;
+        wait |= (uint32_t)(valid && later) << j;
+        v[j] = 0;
+        const uint8_t* from = own ? lit : o;
+        const uint32_t off = own ? s[j] - (hi ? bk1 : bk0) : s[j];
+        if (valid && !near) v[j] = from[off];
+        if (valid && near && !later) v[j] = ring[(s[j] + a) & rmask];
+      }
+      uint32_t word = v[0] | v[1] << 8 | v[2] << 16 | v[3] << 24;
+      uint32_t* const slot = reinterpret_cast<uint32_t*>(ring + (((ln << 7) + 4 * lane) & rmask));
+      if (!wait) *slot = word;
+      uint32_t done = __ballot_sync(kFull, !wait);
+      // The bytes that wait come from one or two source words (sa, sb, by the output's word number) in most words:
+      // those are taken once both are there; the others byte by byte, as are bytes from earlier in the word itself.
+      const uint32_t here = (ln << 5) + lane;
+      auto there = [&](uint32_t sw) {  // is output word sw done?
+        const uint64_t st = load_state(&state[sw >> 5 & (NW - 1u)]);
+        const uint32_t l = (uint32_t)(st >> 32), sl = sw >> 5;
+        return l > sl || (l == sl && ((uint32_t)st >> (sw & 31u) & 1u));
+      };
+      uint32_t sa = 0, sb = 0;
+      bool mixed = false;
+      if (done != kFull && wait) {
+        const int j0 = __ffs(wait) - 1, j1 = 31 - __clz(wait);
+        sa = (j0 == 0 ? s[0] : j0 == 1 ? s[1] : j0 == 2 ? s[2] : s[3]) + a >> 2;
+        sb = (j1 == 3 ? s[3] : j1 == 2 ? s[2] : j1 == 1 ? s[1] : s[0]) + a >> 2;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t sw = (s[j] + a) >> 2;
+          mixed |= (wait >> j & 1u) && ((sw != sa && sw != sb) || sw == here);
+        }
+      }
+      uint32_t shown = 0;
+      for (uint32_t k = 0; done != kFull; ++k) {
+        __syncwarp();
+        if (lane == 0 && done != shown) store_state(&state[w], (uint64_t)ln << 32 | done);
+        shown = done;
+        if (wait && !mixed && there(sa) && there(sb)) {  // (a line not complete at the start is in the ring)
+          const uint32_t wa = reinterpret_cast<const uint32_t*>(ring)[sa & (rmask >> 2)];
+          const uint32_t wb = reinterpret_cast<const uint32_t*>(ring)[sb & (rmask >> 2)];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const uint32_t at = s[j] + a;
+            const uint32_t c = ((at >> 2 == sa ? wa : wb) >> 8 * (at & 3u) & 0xFFu) << 8 * j;
+            word |= wait >> j & 1u ? c : 0u;
+          }
+          wait = 0;
+          *slot = word;
+        }
+        if (__any_sync(kFull, mixed)) {
+          if (mixed) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              if (!(wait >> j & 1u)) continue;
+              const uint32_t at = s[j] + a;
+              if (at >> 2 == here) {  // earlier in this word
+                if (wait >> (at & 3u) & 1u) continue;
+                word |= (word >> 8 * (at & 3u) & 0xFFu) << 8 * j;
+              } else {
+                if (!there(at >> 2)) continue;
+                word |= (uint32_t)ring[at & rmask] << 8 * j;
+              }
+              wait &= ~(1u << j);
+            }
+            if (!wait) { mixed = false; *slot = word; }
+          }
+        }
+        done = __ballot_sync(kFull, !wait);
+        if (k > kMultiPoll) { dead = true; break; }
+      }
+      if (dead) break;
+      __syncwarp();
+      if (lane == 0) store_state(&state[w], (uint64_t)(ln + NW) << 32);
+      if (q0 >= 0 && q0 + 4 <= (int32_t)raw) {
+        *reinterpret_cast<uint32_t*>(o + q0) = word;
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (q0 + j >= 0 && q0 + j < (int32_t)raw) o[q0 + j] = (uint8_t)(word >> (8 * j));
+      }
+    }
+    __syncwarp();
+    if (lane == 0) store_state(&state[w], (uint64_t)0x7FFFFFFFu << 32);
+    if (dead && lane == 0) flag(A.err, b, E_TOKEN);
+  }
+}
+
 size_t fill_smem_bytes(uint32_t ring_log, uint32_t warps, uint32_t words) {
   return (size_t)warps * (fill_table_bytes(words) + (1u << ring_log) + fill_flag_bytes(words));
 }
@@ -448,16 +689,33 @@ cudaError_t prepare_fill() {
   return e;
 }
 
-void launch_decode_fill(const DecArgs& A, cudaStream_t st, Stages& S) {
+constexpr uint32_t kFillSms = 148;
+
+void launch_decode_fill(const DecArgs& args, cudaStream_t st, Stages& S) {
+  DecArgs A = args;
   if (!A.nb) return;
+  // A warp a block once ten blocks an SM keep it busy, else 4 to kMultiWarps warps a block, as many as the GPU holds
+  // (32 an SM).  lz_mix, block 18, ms with 1 / 4 / 8 / 16 warps: 256 blocks 1.99 / 0.75 / 0.56 / 0.52, 1024 blocks
+  // 2.18 / 1.62 / 1.73 / 1.66, 1600 blocks 2.35 / 2.37 / 2.46 / 2.61, 4096 blocks 3.70 / 5.57 / 6.19 / 6.54: sharing
+  // a block costs about 130 more warp instructions a line (366), so it pays while warps are few.
+  uint32_t nw = 1;
+  if (A.nb <= kFillSms * 10)
+    for (nw = 4; nw < kMultiWarps && 2 * nw * A.nb <= kFillSms * 32;) nw *= 2;
+  if (nw == 1) A.line = nullptr;
   launch_dec_streams(A, st, S);
   S.begin("k_dec_tokens", st);
   k_dec_tokens<<<A.nb, 1024, 0, st>>>(A);
   S.end(st);
+  cudaMemsetAsync(A.work, 0, sizeof(uint32_t), st);
+  if (nw > 1) {
+    S.begin("k_dec_fill", st);
+    k_dec_fill_multi<<<A.nb, 32 * nw, multi_smem(nw), st>>>(A);
+    S.end(st);
+    return;
+  }
   const uint32_t W = A.fill_warps;
   const size_t sm = fill_smem_bytes(A.ring_log, W, A.fill_words);
   const uint32_t grid = (A.nb + W - 1) / W;  // (as many warps as blocks; the counter balances them)
-  cudaMemsetAsync(A.work, 0, sizeof(uint32_t), st);
   S.begin("k_dec_fill", st);
   if (A.fill_words == 4) k_dec_fill<4><<<grid, 32 * W, sm, st>>>(A);
   else if (A.fill_words == 2) k_dec_fill<2><<<grid, 32 * W, sm, st>>>(A);

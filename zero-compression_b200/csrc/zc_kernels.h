@@ -40,13 +40,19 @@ struct DecArgs {
   // scratch, per block slot b: lit at b*B, tok / sym / grp at b*tok_cap(B), ext at b*ext_cap(B)
   uint8_t *s_lit, *s_tok, *s_sym, *s_grp, *s_ext;
   DecMeta* meta;
-  // the replay: per token (tok_cap(B) per block) its output start, match start, offset and literal start
-  uint32_t *tk_start, *tk_ms, *tk_d, *tk_lik;
+  // the replay: per token (tok_cap(B) per block) its row (output start, literal count, literal start) and offset
+  uint2* tk_pos;
+  uint32_t* tk_d;
+  // per 128-byte line of the output address (line_cap(B) per block): the token that holds its first byte, and a bit
+  // for each of its words in which another token starts
+  uint2* line;
   // the fill's shape: a ring of 2^ring_log recent output bytes per warp, fill_warps warps (blocks) per CTA,
   // fill_words output words a lane a round (1, 2 or 4)
   uint32_t ring_log, fill_warps, fill_words;
   uint32_t* work;             // the fill's device work counter (zeroed by the launcher)
 };
+
+__host__ __device__ inline uint32_t line_cap(uint32_t B) { return B / 128 + 2; }
 
 constexpr uint32_t kMinFillRingLog = 11, kMaxFillRingLog = 15, kMaxFillWarps = 8;
 constexpr size_t kMaxFillSmem = 227 * 1024;

@@ -49,7 +49,8 @@ size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // The scratch a call of nb blocks of B bytes takes: the fill's work counter, then per kind of buffer one
 // region of nb slots: literals (B), tok / sym / group streams (tok_cap each), ext bytes (ext_cap), the
-// framing records, and the four token tables (tok_cap words each).
+// framing records, and the token tables (four words for each of tok_cap tokens: three of its row and offset, and
+// room for the line table, which takes less than one).
 size_t scratch_need(uint32_t nb, uint32_t B) {
   const size_t TC = zc::tok_cap(B), EC = zc::ext_cap(B);
   return 256 + up256((size_t)nb * B) + 3 * up256((size_t)nb * TC) + up256((size_t)nb * EC) +
@@ -133,10 +134,9 @@ extern "C" int zc_decompress_noalloc(const uint8_t* d_comp, const uint64_t* d_co
   A.s_grp = at; at += up256((size_t)nb * TC);
   A.s_ext = at; at += up256((size_t)nb * EC);
   A.meta = reinterpret_cast<zc::DecMeta*>(at); at += up256((size_t)nb * sizeof(zc::DecMeta));
-  A.tk_start = reinterpret_cast<uint32_t*>(at); at += up256((size_t)nb * TC * 4);
-  A.tk_ms = reinterpret_cast<uint32_t*>(at); at += up256((size_t)nb * TC * 4);
+  A.tk_pos = reinterpret_cast<uint2*>(at); at += 2 * up256((size_t)nb * TC * 4);
   A.tk_d = reinterpret_cast<uint32_t*>(at); at += up256((size_t)nb * TC * 4);
-  A.tk_lik = reinterpret_cast<uint32_t*>(at);
+  A.line = reinterpret_cast<uint2*>(at);
   // the fill's launch shape: the default of the context-based calls (a ring of 4 KiB per warp, 4 warps a
   // CTA, a word a lane a round)
   A.ring_log = 12;
