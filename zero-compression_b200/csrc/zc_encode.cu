@@ -17,9 +17,9 @@
 //                  positions that a walk visits
 //   k_enc_parse    one CTA per block: segments re-walked from where the chain before them leaves until they
 //                  meet the first walk (rounds until no segment exit moves), then the tokens written
-//   k_enc_streams  one warp per block: group starts from a running maximum of per-token thresholds and a
-//                  next-start chain, recent offsets by shuffles from each group's start, tok / ext / sym /
-//                  group streams, offset bits packed by a word-segmented OR-scan, literals
+//   k_enc_streams  one CTA per block, a lane a token: group starts from a running maximum of per-token thresholds
+//                  and next-start chains, recent offsets from each group's start, tok / ext / sym / group streams
+//                  placed by scans, offset bits gathered in shared memory, literals
 //   k_enc_rans     one CTA per (block, stream): histogram, 12-bit normalisation with the reference's
 //                  tie-breaks, 64 lanes coding backwards (src/codec.h:41-147)
 //   k_enc_pack     one CTA per block: the payload (src/codec2.h:139-152), or "stored"
@@ -765,12 +765,12 @@ __global__ void __launch_bounds__(T, 1024 / T) k_enc_parse(EncArgs A) {
 constexpr uint32_t kWarpCopyRun = 32;
 
 // n bytes from src, a range of the codec's input (16-byte aligned, 64 readable bytes after its end), to
-// dst by the 32 lanes of a warp: 4-byte words stored aligned at dst, each built by a funnel shift from
+// dst by nth threads, this one thread t of them: 4-byte words stored aligned at dst, each built by a funnel shift from
 // the two aligned input words that cover it (those may reach a few bytes past the range, into the
-// input's slack, never before the input's start), four words a lane in flight.
-__device__ __forceinline__ void warp_copy_in(uint8_t* dst, const uint8_t* src, uint32_t n, uint32_t lane) {
+// input's slack, never before the input's start), four words a thread in flight.
+__device__ __forceinline__ void copy_in(uint8_t* dst, const uint8_t* src, uint32_t n, uint32_t t, uint32_t nth) {
   const uint32_t head = min(n, (4u - ((uint32_t)(uintptr_t)dst & 3u)) & 3u);
-  if (lane < head) dst[lane] = src[lane];
+  if (t < head) dst[t] = src[t];
   dst += head;
   src += head;
   n -= head;
@@ -779,36 +779,52 @@ __device__ __forceinline__ void warp_copy_in(uint8_t* dst, const uint8_t* src, u
   uint32_t* d = reinterpret_cast<uint32_t*>(dst);
   if (sh) {
 #pragma unroll 4
-    for (uint32_t w = lane; w < nw; w += 32) d[w] = __funnelshift_r(s[w], s[w + 1], 8u * sh);
+    for (uint32_t w = t; w < nw; w += nth) d[w] = __funnelshift_r(s[w], s[w + 1], 8u * sh);
   } else {
 #pragma unroll 4
-    for (uint32_t w = lane; w < nw; w += 32) d[w] = s[w];
+    for (uint32_t w = t; w < nw; w += nth) d[w] = s[w];
   }
-  const uint32_t t = nw << 2;
-  if (lane < n - t) dst[t + lane] = src[t + lane];
+  const uint32_t done = nw << 2;
+  if (t < n - done) dst[done + t] = src[done + t];
 }
 
-// Tokens -> streams, one warp per block, 32 tokens a round (the next 32 loaded while these are coded).
+// Tokens -> streams, a CTA of NW warps per block, 32 NW tokens a tile, a lane a token.
 //
 // Groups follow the rule of src/codec2.h:103-116: a group ends before a token whose match source starts before
-// the token's own output and reaches past the group's first output byte, or once it holds 255 tokens.  Within
-// a round, a group opened at token g is read by token k exactly when the output start of g lies below k's
-// source reach, and the output starts rise with the token index; so each token k whose source starts before
-// its output gets theta_k = how many of the round's tokens start their output below its reach (at most k),
-// and a group opened at g ends at the first token with theta > g.  With P the running maximum of theta over
-// the round, that is next(g) = the first k with P_k > g: a binary search over P by shuffles.  The group open
-// when the round starts ends at the first token that reads it (or would be its 256th); the round's later group
-// starts follow from there by next().  A token's recent-offset symbols (250..252) name the offsets of the
-// three tokens before its group's first token (src/codec2.h:121-137).
+// the token's own output and reaches past the group's first output byte, or once it holds 255 tokens.  A group
+// opened at token g is read by token k exactly when the output start of g lies below k's source reach, and the
+// output starts rise with the token index; so each token k whose source starts before its output gets
+// theta_k = how many tokens start their output below its reach (at most k; only the last 255 matter), and a group
+// opened at g ends at the first later token with theta > g, or at g + 255.  Within a warp's 32 tokens that is
+// next(g), by a binary search over the running maximum of theta; doubling next() gives, for each lane, the group
+// starts that follow if a group starts there, and the last of them.  One warp then goes through the tile's warps in
+// order: the group open before a warp ends at the warp's first token that reads it, and the last start that
+// follows from there is open after it.  A token's recent-offset symbols (250..252) name the offsets of the three
+// tokens before its group's first token (src/codec2.h:121-137).
 //
-// Offset bits (LSB first): each token's bits start at a running bit position.  The tokens are grouped by the
-// 32-bit output word their bits start in (the groups are runs of lanes), an OR-scan segmented by that word
-// collects each word's bits (64-bit values: a token's spill into the next word rides in the high half), and
-// the last lane of each run stores its completed word.  The partly filled last word carries to the next round.
-__global__ void __launch_bounds__(128) k_enc_streams(EncArgs A) {
-  const uint32_t lane = lane_id();
-  const uint32_t b = blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (b >= A.nb) return;
+// All positions in the streams come from two packed scans (literals and group starts; ext bytes and offset bits).
+// Offset bits (LSB first) are gathered in shared memory and stored as words, the last one carried to the next
+// tile.
+template <uint32_t NW>
+struct StreamTile {
+  static constexpr uint32_t NT = 32 * NW, RING = NT < 512 ? 1024 : 2 * NT;  // (a tile and the 257 tokens before it)
+  uint32_t op[RING], d[RING];          // output start and offset of token k at k % RING
+  uint32_t pm[NT];                     // running maximum of theta within the warp
+  uint8_t last[NT];                    // the last start of the warp that follows one here
+  uint32_t gin[NW], s1[NW];            // per warp: the group open before it, its first group start (32: none)
+  uint32_t sum0[NW], sum1[NW];         // per warp: literals | starts << 21, ext bytes | offset bits << 16
+  uint32_t bits[NT * 19 / 32 + 2];
+  uint32_t big[NW * 32][3], nbig;      // literal runs that the whole CTA copies: destination, source, length
+  uint32_t open;                       // the group open after the tile
+};
+constexpr uint32_t kCtaCopyRun = 2048;
+
+template <uint32_t NW>
+__global__ void __launch_bounds__(32 * NW, NW == 8 ? 8 : 1) k_enc_streams(EncArgs A) {
+  using T = StreamTile<NW>;
+  constexpr uint32_t NT = T::NT, RM = T::RING - 1;
+  __shared__ T S;
+  const uint32_t lane = lane_id(), w = threadIdx.x >> 5, tid = threadIdx.x, b = blockIdx.x;
   const uint32_t n = A.in_len[b], nt = A.bcnt[b * 8 + 0];
   const uint8_t* src = A.in + A.in_off[b];
   const size_t TC = tok_cap(A.B);
@@ -821,145 +837,147 @@ __global__ void __launch_bounds__(128) k_enc_streams(EncArgs A) {
   uint8_t* grp = A.s_grp + (size_t)b * TC;
   uint8_t* ext = A.s_ext + (size_t)b * ext_cap(A.B);
   uint32_t* bitw = reinterpret_cast<uint32_t*>(A.s_bits + (size_t)b * bits_cap(A.B));
-  const uint32_t upto = 0xFFFFFFFFu >> (31u - lane);  // lanes 0 .. lane
-  uint32_t op = 0;                    // output end of the tokens coded so far
-  uint32_t gpos = 0, gcnt = 0;        // the open group: its first output byte, its tokens so far
-  uint32_t ra = 1, rb = 4, rc = 8;    // the open group's recent offsets
-  uint32_t pa = 1, pb = 4, pc = 8;    // the offsets of the last three tokens before the round, nearest first
-  uint32_t ng = 0, ei = 0, li = 0;
-  uint64_t bp = 0, wbase = 0;         // bits written so far; the first bit of the word being filled
-  uint32_t cw = 0;                    // that word's bits [wbase, bp)
-  uint32_t ni = 0, nm = 4, nd = 1;
-  if (lane < nt) { ni = TI[lane]; nm = TM[lane]; nd = TD[lane]; }
-  for (uint32_t t0 = 0; t0 < nt; t0 += 32) {
-    const uint32_t c = min(32u, nt - t0);
-    const uint32_t q = t0 + lane;
-    const bool on = lane < c;
-    const uint32_t i = ni, m = nm, d = nd;
-    if (q + 32 < nt) { ni = TI[q + 32]; nm = TM[q + 32]; nd = TD[q + 32]; } else { ni = 0; nm = 4; nd = 1; }
-    const uint32_t endk = i + m;
-    const uint32_t up = __shfl_up_sync(kFull, endk, 1);
-    const uint32_t opk = lane == 0 ? op : up;
+  const uint32_t below = (1u << lane) - 1u;
+  uint32_t li = 0, ei = 0, ng = 0;      // literals, ext bytes, group starts after the first, of the tiles before
+  uint32_t bp = 0, cw = 0;              // offset bits of the tiles before, the last one's partly filled word
+  if (tid == 0) S.open = 0;
+  uint32_t ni = 0, nm = 4, nd = 1, ne = 0;  // the lane's token of the next tile, and the end of the one before it
+  auto fetch = [&](uint32_t k) {
+    ni = 0; nm = 4; nd = 1; ne = 0;
+    if (k < nt) {
+      ni = TI[k]; nm = TM[k]; nd = TD[k];
+      if (k) ne = TI[k - 1] + TM[k - 1];
+    }
+  };
+  fetch(tid);
+  for (uint32_t t0 = 0; t0 < nt; t0 += NT) {
+    const uint32_t k = t0 + tid;
+    const bool on = k < nt;
+    const uint32_t i = ni, m = nm, d = nd, opk = ne;
+    S.op[k & RM] = on ? opk : 0xFFFFFFFFu;
+    S.d[k & RM] = d;
+    if (tid == 0) S.nbig = 0;
+    for (uint32_t q = tid; q < sizeof S.bits / 4; q += NT) S.bits[q] = q ? 0u : cw;
+    fetch(k + NT);
+    __syncthreads();
+    // theta, its running maximum, next() and what follows from each lane
     const uint32_t L = on ? i - opk : 0u;
     const uint32_t reach = i - d + min(m, d);
-    const bool back = on && i - d < opk;  // the source starts before the token's own output
-    // theta: the round's tokens whose output starts below the reach (lanes past c compare as above all)
-    const uint32_t key = on ? opk : 0xFFFFFFFFu;
-    uint32_t below = 0;
-#pragma unroll
-    for (uint32_t s = 16; s; s >>= 1)
-      if (__shfl_sync(kFull, key, below + s - 1) < reach) below += s;
-    const uint32_t theta = back ? min(lane, below) : 0u;
-    // the open group ends at the first token that reads it, or that would be its 256th
-    const unsigned ends = __ballot_sync(kFull, on && ((back && reach > gpos) || gcnt + lane >= kMaxGroup));
-    const uint32_t s1 = ends ? (uint32_t)__ffs(ends) - 1u : c;
-    uint32_t pm = theta;  // running maximum of theta
+    uint32_t theta = 0;
+    if (on && i - d < opk) {  // tokens [lo, theta) start below the reach, of the last 255
+      uint32_t lo = k > 255u ? k - 255u : 0u, hi = k;
+      while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (S.op[mid & RM] < reach) lo = mid + 1; else hi = mid;
+      }
+      theta = lo;
+    }
+    uint32_t pm = theta;
 #pragma unroll
     for (uint32_t o = 1; o < 32; o <<= 1) {
       const uint32_t v = __shfl_up_sync(kFull, pm, o);
       if (lane >= o) pm = max(pm, v);
     }
-    uint32_t nx = 0;  // next(lane): the first token with pm > lane (32: none)
+    uint32_t nx = 0;  // the first lane with pm > k (32: none)
 #pragma unroll
     for (uint32_t s = 16; s; s >>= 1)
-      if (__shfl_sync(kFull, pm, nx + s - 1) <= lane) nx += s;
-    if (__shfl_sync(kFull, pm, nx) <= lane) nx = 32;
-    uint32_t starts = 0;  // the round's group starts (warp-uniform walk)
-    for (uint32_t s = s1; s < c; s = __shfl_sync(kFull, nx, s)) starts |= 1u << s;
-    // the token's group start gs (-1: the group open before the round) and its recent offsets
-    const uint32_t mine = starts & upto;
-    const int gs = mine ? 31 - __clz(mine) : -1;
-    const uint32_t x1 = __shfl_sync(kFull, d, max(gs - 1, 0)), x2 = __shfl_sync(kFull, d, max(gs - 2, 0)),
-                   x3 = __shfl_sync(kFull, d, max(gs - 3, 0));
-    uint32_t r0 = ra, r1 = rb, r2 = rc;
-    if (gs >= 0) {
-      r0 = gs >= 1 ? x1 : pa;
-      r1 = gs >= 2 ? x2 : gs == 1 ? pa : pb;
-      r2 = gs >= 3 ? x3 : gs == 2 ? pa : gs == 1 ? pb : pc;
+      if (__shfl_sync(kFull, pm, nx + s - 1) <= k) nx += s;
+    if (__shfl_sync(kFull, pm, nx) <= k) nx = 32;
+    uint32_t follow = 1u << lane, far = lane;  // the starts from this lane on, the last of them
+#pragma unroll
+    for (uint32_t o = 0; o < 5; ++o) {
+      const uint32_t f = __shfl_sync(kFull, follow, nx & 31u), l = __shfl_sync(kFull, far, nx & 31u),
+                     x = __shfl_sync(kFull, nx, nx & 31u);
+      if (nx < 32u) { follow |= f; far = l; nx = x; }
     }
+    S.pm[tid] = on ? pm : 0u;
+    S.last[tid] = (uint8_t)far;
+    __syncthreads();
+    if (w == 0) {  // the group that each warp meets, in order
+      uint32_t g = S.open, p = S.pm[lane];
+      for (uint32_t v = 0; v < NW; ++v) {
+        const uint32_t at = t0 + 32 * v + lane;
+        const unsigned e = __ballot_sync(kFull, at < nt && (p > g || at - g >= kMaxGroup) && at > g);
+        if (v + 1 < NW) p = S.pm[32 * (v + 1) + lane];
+        const uint32_t s = e ? (uint32_t)__ffs(e) - 1u : 32u;
+        if (lane == 0) { S.gin[v] = g; S.s1[v] = s; }
+        if (e) g = t0 + 32 * v + S.last[32 * v + s];
+      }
+      if (lane == 0) S.open = g;
+    }
+    __syncthreads();
+    const uint32_t g0 = S.gin[w], s1 = S.s1[w];
+    uint32_t starts = __shfl_sync(kFull, follow, s1 & 31u);
+    if (s1 == 32u) starts = 0;
+    starts &= __ballot_sync(kFull, on);
+    const uint32_t mine = starts & (below | 1u << lane);
+    const uint32_t gs = mine ? t0 + 32 * w + 31u - __clz(mine) : g0;
+    // the offsets of tokens gs - 1, gs - 2, gs - 3, then 1, 4, 8
+    const uint32_t r0 = gs >= 1 ? S.d[(gs - 1) & RM] : 1u;
+    const uint32_t r1 = gs >= 2 ? S.d[(gs - 2) & RM] : gs == 1 ? 1u : 4u;
+    const uint32_t r2 = gs >= 3 ? S.d[(gs - 3) & RM] : gs == 2 ? 1u : gs == 1 ? 4u : 8u;
     const uint32_t sv = d == r0 ? kSymRep : d == r1 ? kSymRep + 1 : d == r2 ? kSymRep + 2 : bitlen(d);
-    // group counts: the open group's (when it ends in this round), then each start's that ends in it
-    const uint32_t open_ends = s1 < c && gcnt + s1 > 0 ? 1u : 0u;
-    if (lane == 0 && open_ends) grp[ng] = (uint8_t)(gcnt + s1);
-    if (((starts >> lane) & 1u) && nx < c) grp[ng + open_ends + __popc(mine) - 1] = (uint8_t)(nx - lane);
-    ng += open_ends + (starts ? (uint32_t)__popc(starts) - 1u : 0u);
-    if (starts) {
-      const uint32_t last = 31u - __clz(starts);
-      gpos = __shfl_sync(kFull, opk, last);
-      gcnt = c - last;
-      ra = __shfl_sync(kFull, r0, last);
-      rb = __shfl_sync(kFull, r1, last);
-      rc = __shfl_sync(kFull, r2, last);
-    } else {
-      gcnt += c;
-    }
-    {  // (only a full round is followed by another)
-      const uint32_t a = __shfl_sync(kFull, d, 31), bq = __shfl_sync(kFull, d, 30), cq = __shfl_sync(kFull, d, 29);
-      pa = a; pb = bq; pc = cq;
-    }
     if (on) {
-      tok[q] = (uint8_t)((min(L, 15u) << 4) | min(m - 4u, 15u));
-      sym[q] = (uint8_t)sv;
+      tok[k] = (uint8_t)((min(L, 15u) << 4) | min(m - 4u, 15u));
+      sym[k] = (uint8_t)sv;
     }
     // ext bytes (src/codec2.h:120-121): L - 15 in 3 bytes when L >= 15, then m - 19 in 2 when m >= 19
     const uint32_t fl = on && L >= 15u, fm = on && m >= 19u;
-    const uint32_t nx_b = 3u * fl + 2u * fm;
-    const uint32_t xincl = warp_incl_scan(nx_b);
-    const uint32_t xq = ei + xincl - nx_b;
+    const uint32_t nbit = on && sv < kSymRep ? sv : 0u;
+    const uint32_t v0 = L | (starts >> lane & 1u) << 21, v1 = 3u * fl + 2u * fm | nbit << 16;
+    const uint32_t i0 = warp_incl_scan(v0), i1 = warp_incl_scan(v1);
+    if (lane == 31) { S.sum0[w] = i0; S.sum1[w] = i1; }
+    __syncthreads();
+    const uint32_t w0 = lane < NW ? S.sum0[lane] : 0u, w1 = lane < NW ? S.sum1[lane] : 0u;
+    const uint32_t c0 = warp_incl_scan(w0), c1 = warp_incl_scan(w1);
+    const uint32_t p0 = __shfl_sync(kFull, c0 - w0, w) + i0 - v0, p1 = __shfl_sync(kFull, c1 - w1, w) + i1 - v1;
+    const uint32_t all0 = __shfl_sync(kFull, c0, 31), all1 = __shfl_sync(kFull, c1, 31);
+    if (starts >> lane & 1u) {  // a start closes the group before it
+      const uint32_t before = starts & below;
+      grp[ng + (p0 >> 21)] = (uint8_t)(k - (before ? t0 + 32 * w + 31u - __clz(before) : g0));
+    }
+    const uint32_t xq = ei + (p1 & 0xFFFFu);
     if (fl) { const uint32_t v = L - 15u; ext[xq] = (uint8_t)v; ext[xq + 1] = (uint8_t)(v >> 8); ext[xq + 2] = (uint8_t)(v >> 16); }
     if (fm) { const uint32_t v = m - 19u, y = xq + 3u * fl; ext[y] = (uint8_t)v; ext[y + 1] = (uint8_t)(v >> 8); }
-    // offset bits
-    const uint32_t nbit = on && sv < kSymRep ? sv : 0u;
-    const uint32_t bincl = warp_incl_scan(nbit);
-    const uint32_t rel = (uint32_t)(bp - wbase) + bincl - nbit;  // (bp - wbase < 32)
-    const uint32_t wi = rel >> 5;
-    uint64_t acc = nbit ? (uint64_t)(d - (1u << nbit)) << (rel & 31u) : 0ull;
-#pragma unroll
-    for (uint32_t o = 1; o < 32; o <<= 1) {
-      const uint64_t v = __shfl_up_sync(kFull, acc, o);
-      const uint32_t vw = __shfl_up_sync(kFull, wi, o);
-      if (lane >= o && vw == wi) acc |= v;
+    if (nbit) {
+      const uint32_t at = (bp & 31u) + (p1 >> 16), x = d - (1u << nbit);
+      atomicOr(&S.bits[at >> 5], x << (at & 31u));
+      if ((at & 31u) + nbit > 32u) atomicOr(&S.bits[(at >> 5) + 1], x >> (32u - (at & 31u)));
     }
-    const uint32_t rel_end = (uint32_t)(bp - wbase) + __shfl_sync(kFull, bincl, 31);
-    const uint32_t full = rel_end >> 5;  // words completed by this round
-    const uint32_t wprev = __shfl_up_sync(kFull, wi, 1), wnext = __shfl_down_sync(kFull, wi, 1);
-    const unsigned firsts = __ballot_sync(kFull, lane == 0 || wprev != wi);
-    const uint32_t f = 31u - __clz(firsts & upto);  // the first lane of this lane's run
-    const uint32_t spill = (uint32_t)(__shfl_sync(kFull, acc, f ? f - 1u : 0u) >> 32);
-    const uint32_t word = (uint32_t)acc | (f ? spill : 0u) | (wi == 0 ? cw : 0u);
-    if ((lane == 31 || wnext != wi) && wi < full) bitw[(wbase >> 5) + wi] = word;
-    const uint32_t w31 = __shfl_sync(kFull, word, 31), s31 = (uint32_t)(__shfl_sync(kFull, acc, 31) >> 32);
-    cw = __shfl_sync(kFull, wi, 31) == full ? w31 : s31;
-    bp += __shfl_sync(kFull, bincl, 31);
-    wbase += 32ull * full;
-    // literals before each token: a lane copies its own short run; runs of kWarpCopyRun bytes or more
-    // (a long incompressible stretch) are copied by the whole warp, one after another
-    const uint32_t lincl = warp_incl_scan(L);
-    const uint32_t lik = li + lincl - L;
-    const bool longrun = L >= kWarpCopyRun;
-    if (!longrun)
-      for (uint32_t k = 0; k < L; ++k) lit[lik + k] = src[opk + k];
-    for (unsigned lb = __ballot_sync(kFull, longrun); lb; lb &= lb - 1) {
+    // literals before each token: a lane copies its own short run, the warp a longer one, the CTA the longest
+    const uint32_t lik = li + (p0 & 0x1FFFFFu);
+    if (L < kWarpCopyRun) {
+      for (uint32_t q = 0; q < L; ++q) lit[lik + q] = src[opk + q];
+    } else if (L >= kCtaCopyRun) {
+      const uint32_t q = atomicAdd(&S.nbig, 1u);
+      S.big[q][0] = lik; S.big[q][1] = opk; S.big[q][2] = L;
+    }
+    for (unsigned lb = __ballot_sync(kFull, L >= kWarpCopyRun && L < kCtaCopyRun); lb; lb &= lb - 1) {
       const uint32_t r = (uint32_t)__ffs(lb) - 1u;
       const uint32_t rL = __shfl_sync(kFull, L, r), rd = __shfl_sync(kFull, lik, r), rs = __shfl_sync(kFull, opk, r);
-      warp_copy_in(lit + rd, src + rs, rL, lane);
+      copy_in(lit + rd, src + rs, rL, lane, 32);
     }
-    li += __shfl_sync(kFull, lincl, 31);
-    ei += __shfl_sync(kFull, xincl, 31);
-    op = __shfl_sync(kFull, endk, c - 1);
+    __syncthreads();
+    for (uint32_t q = 0; q < S.nbig; ++q) copy_in(lit + S.big[q][0], src + S.big[q][1], S.big[q][2], tid, NT);
+    const uint32_t end = (bp & 31u) + (all1 >> 16), full = end >> 5;  // words completed by this tile
+    for (uint32_t q = tid; q < full; q += NT) bitw[(bp >> 5) + q] = S.bits[q];
+    cw = S.bits[full];
+    bp += all1 >> 16;
+    li += all0 & 0x1FFFFFu;
+    ng += all0 >> 21;
+    ei += all1 & 0xFFFFu;
+    __syncthreads();
   }
-  if (gcnt) {
-    if (lane == 0) grp[ng] = (uint8_t)gcnt;
-    ++ng;
-  }
-  warp_copy_in(lit + li, src + op, n - op, lane);
-  li += n - op;
-  if (bp > wbase && lane == 0) bitw[wbase >> 5] = cw;
-  if (lane == 0) {
-    A.bcnt[b * 8 + 1] = li;
+  __syncthreads();
+  const uint32_t op = nt ? TI[nt - 1] + TM[nt - 1] : 0u;
+  copy_in(lit + li, src + op, n - op, tid, NT);
+  if (tid == 0) {
+    if (nt) grp[ng] = (uint8_t)(nt - S.open);
+    if (bp & 31u) bitw[bp >> 5] = cw;
+    A.bcnt[b * 8 + 1] = li + n - op;
     A.bcnt[b * 8 + 2] = ei;
-    A.bcnt[b * 8 + 3] = (uint32_t)((bp + 7) / 8);
-    A.bcnt[b * 8 + 4] = ng;
+    A.bcnt[b * 8 + 3] = (bp + 7) / 8;
+    A.bcnt[b * 8 + 4] = nt ? ng + 1 : 0;
   }
 }
 
@@ -1319,7 +1337,13 @@ void launch_encode(const EncArgs& A, const CrcArgs& crc_in, cudaStream_t st, Sta
   else k_enc_parse<1024><<<A.nb, 1024, fin, st>>>(A);
   S.end(st);
   S.begin("k_enc_streams", st);
-  k_enc_streams<<<(A.nb + 3) / 4, 128, 0, st>>>(A);
+  // A tile's barriers and the walk over its warps cost the same for any width, so a block is faster in wide tiles and a
+  // full GPU in narrow ones.  ms with 32 / 16 / 8 warps: one text block 0.076 / 0.101 / 0.166, 64 MiB of text (256
+  // blocks) 0.24 / 0.19 / 0.29, 256 blocks of 1 MiB 0.43 / 0.36 / 0.58, 1 GiB of lz_mix (4096 blocks) 1.56 / 1.24 /
+  // 0.82.  (One warp a block, 32 tokens a round: 0.64, 1.09, 2.56 and 0.87.)
+  if (A.nb <= 148) k_enc_streams<32><<<A.nb, 1024, 0, st>>>(A);
+  else if (A.nb <= 3 * 148) k_enc_streams<16><<<A.nb, 512, 0, st>>>(A);
+  else k_enc_streams<8><<<A.nb, 256, 0, st>>>(A);
   S.end(st);
   S.begin("k_enc_rans", st);
   k_enc_rans<<<dim3(A.nb, 5), 64, 0, st>>>(A);
