@@ -39,6 +39,8 @@ constexpr zc::CrcTables cx_tables() {
     for (uint32_t i = 0; i < 256; ++i) T.t[k][i] = (T.t[k - 1][i] >> 8) ^ T.t[0][T.t[k - 1][i] & 0xFFu];
   uint32_t p = 0x00800000u;  // x^8
   for (int e = 0; e < 64; ++e) { T.pow2[e] = p; p = cx_mul(p, p); }
+  T.row[31] = 0x80000000u;  // x^0
+  for (int l = 30; l >= 0; --l) T.row[l] = cx_mul(T.row[l + 1], T.pow2[7]);
   return T;
 }
 
