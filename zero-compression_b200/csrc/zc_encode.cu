@@ -351,9 +351,9 @@ constexpr uint32_t kItems = 32 + 32 * kTasks;         // the most candidates tha
 constexpr uint32_t kBatch = 8;
 struct Finish {
   uint4 xw[32];                                       // the first 16 bytes at the request's position
-  uint32_t x[32], rt[32], key[32];                    // its position; its entry's place | tag << 20; best so far
-  uint32_t po[32], pw[32];                            // a candidate that matters has these 4 bytes at this offset
-  uint32_t ord[32];                                   // the requests' slots, one after the other
+  uint32_t x[32], key[32];                            // its position; best so far
+  uint4 req[32];  // the requests one after the other: the entry's place | tag << 20; position | an offset << 20; the 4
+                  // bytes there, which a candidate that matters has too; slot << 20
   uint32_t it[kItems], deep[kItems + 32], far[kItems + 32];  // not compared; equal for 16 bytes; for 32
   uint32_t batch[kBatch];
 };
@@ -407,6 +407,12 @@ __device__ __forceinline__ void finish_lists(const ParseBlock& P, Finish& W, uin
   const uint32_t g = lane >> 2, gl = lane & 3u;
   while (n3) {
     uint32_t m = 0, nb = 0, carry = 32;  // kept ones, this round's, the last kept one's slot
+    const uint32_t* batch = W.batch;
+    if (n3 <= kBatch) {  // (so few that all are extended)
+      batch = W.far;
+      nb = n3;
+      n3 = 0;
+    }
     for (uint32_t k = 0; k < n3; k += 32) {
       const bool on = k + lane < n3;
       const uint32_t c = on ? W.far[k + lane] : 0u, i = c >> 20, j = c & 0xFFFFFu;
@@ -433,7 +439,7 @@ __device__ __forceinline__ void finish_lists(const ParseBlock& P, Finish& W, uin
     n3 = m;
     if (!nb) break;  // (none was kept)
     bool act = g < nb;
-    const uint32_t c = act ? W.batch[g] : 0u, i = c >> 20, j = c & 0xFFFFFu;
+    const uint32_t c = act ? batch[g] : 0u, i = c >> 20, j = c & 0xFFFFFu;
     const uint32_t x = W.x[i], lim = min(kMaxMatch, P.n - x);
     const bool mine = act && gl == 0;
     uint32_t len = 32;
@@ -480,7 +486,7 @@ __device__ __forceinline__ void warp_finish(const ParseBlock& P, Finish& W, bool
   const uint32_t gl = lane & (G - 1u), NR = 32u / G;
   const bool on0 = act && m_is_sat(v), on1 = act && m_is_sat(v2);
   const uint32_t r2 = v2 & 0xFFFFFu;
-  uint32_t n2 = 0;
+  uint32_t n2 = 0, rt = 0;
   __syncwarp();
   if (__any_sync(kFull, on0)) {
     bool more = false;
@@ -489,7 +495,7 @@ __device__ __forceinline__ void warp_finish(const ParseBlock& P, Finish& W, bool
       const uint32_t r = v & 0xFFFFFu;
       const uint32_t e1 = P.srt[r - min(r, 1u)], e2 = P.srt[r - min(r, 2u)], e3 = P.srt[r - min(r, 3u)];
       const uint4 w = load16(P.in, P.base + p);
-      const uint32_t rt = r | (product(w.x) << 16 & 0xFFF00000u);
+      rt = r | (product(w.x) << 16 & 0xFFF00000u);
       const uint32_t tag = rt >> 20;
       const uint32_t e = e_tag(e1) == tag ? e1 : e_tag(e2) == tag ? e2 : e3;
       const uint32_t j = e_pos(e), lim = min(kMaxMatch, P.n - p);
@@ -502,96 +508,99 @@ __device__ __forceinline__ void warp_finish(const ParseBlock& P, Finish& W, bool
       c = lane << 20 | j;
       W.xw[lane] = w;
       W.x[lane] = p;
-      W.rt[lane] = rt;
       W.key[lane] = key;
     }
     const unsigned mm = __ballot_sync(kFull, more);
     if (more) W.deep[__popc(mm & below)] = c;
     n2 = (uint32_t)__popc(mm);
   }
+  finish_lists(P, W, 0, n2);
+  const uint32_t subs = P.depth > 32 ? 3u : 1u;  // chains are scanned 32 entries first, then the next 128, then the rest
   uint32_t need = 0;
 #pragma unroll 1
-  for (uint32_t ph = 0; ph < 3; ++ph) {
-    bool ask = false;
-    uint32_t at = 0;  // the length that a candidate must exceed (round 1), or reach less one (round 2)
-    if (ph == 1) {
-      if (on0) {
-        const uint32_t key = W.key[lane];
-        at = key ? k_len(key) : 0u;
-        ask = at < min(kMaxMatch, P.n - p);
-      }
-    } else if (ph == 2) {
+  for (uint32_t ph = 1; ph < 3; ++ph) {
+    const uint32_t x = p + ph - 1u, lim = min(kMaxMatch, P.n - x);
+    bool ask = on0;
+    uint32_t least = 0;
+    if (ph == 2) {
       if (on0) {
         const uint32_t key = W.key[lane];
         v = key ? m_pack(k_len(key), p - (key & 0xFFFFFu)) : M_NONE;
         P.minfo[p] = v;
       }
-      if (on1 && v != M_NONE) {
+      ask = on1 && v != M_NONE;
+      if (ask) {
         need = ((8u * m_len(v) + 8u - bitlen(m_dist(v))) >> 3) + 1u;
-        at = need - 1u;
-        ask = need <= min(kMaxMatch, P.n - p - 1u);
-      }
-    }
-    const unsigned am = __ballot_sync(kFull, ask);
-    if (ask) {
-      const uint32_t x = p + ph - 1u, po = max(at, 3u) - 3u;
-      if (ph == 2) {
+        least = need - 1u;
         const uint4 w = load16(P.in, P.base + x);
         W.xw[lane] = w;
         W.x[lane] = x;
-        W.rt[lane] = r2 | (product(w.x) << 16 & 0xFFF00000u);
         W.key[lane] = 0;
+        rt = r2 | (product(w.x) << 16 & 0xFFF00000u);
       }
-      W.po[lane] = po;
-      W.pw[lane] = load4(P.in, P.base + x + po);
-      W.ord[__popc(am & below)] = lane;
     }
-    __syncwarp();
-    const uint32_t nreq = (uint32_t)__popc(am);
-    const bool chunks = P.depth > 32;  // (then 8 chunks of 32 entries a request, four of them at a time)
-    const uint32_t nt = chunks ? nreq * (P.depth / 32) : (nreq + NR - 1) / NR;
-    uint32_t t = 0;
-    do {
-      uint32_t cnt = 0;
-      while (t < nt && cnt <= 32) {
-        uint32_t e[kTasks], s[kTasks], w[kTasks];
-        bool hit[kTasks];
-#pragma unroll
-        for (uint32_t u = 0; u < kTasks; ++u) {
-          const uint32_t k = chunks ? (t + u) / (P.depth / 32) : (t + u) * NR + lane / G;
-          const uint32_t q = chunks ? (t + u) % (P.depth / 32) * 32 + lane : gl;
-          s[u] = k < nreq ? W.ord[k] : 0u;
-          const uint32_t rt = k < nreq ? W.rt[s[u]] : 0u, r = rt & 0xFFFFFu;
-          e[u] = q < min(P.depth, r) ? P.srt[r - 1u - q] : ~rt;  // (else: another tag)
-          hit[u] = e[u] - (rt & 0xFFF00000u) < W.x[s[u]];         // the same tag and an earlier position
-        }
-#pragma unroll
-        for (uint32_t u = 0; u < kTasks; ++u)
-          w[u] = hit[u] ? load4(P.in, P.base + e_pos(e[u]) + W.po[s[u]]) : 0u;
-#pragma unroll
-        for (uint32_t u = 0; u < kTasks; ++u) {
-          const bool pass = hit[u] && w[u] == W.pw[s[u]];
-          const unsigned hm = __ballot_sync(kFull, pass);
-          if (pass) W.it[cnt + __popc(hm & below)] = s[u] << 20 | e_pos(e[u]);
-          cnt += (uint32_t)__popc(hm);
-        }
-        t += kTasks;
-        // a deep chain's second half is skipped when it ended in the first: at the order's start, or where the
-        // positions do not fall (entries of other hashes are harmless: their bytes differ)
-        if (chunks && t % (P.depth / 32)) {
-          bool end = false;
+#pragma unroll 1
+    for (uint32_t sub = 0; sub < subs; ++sub) {
+      // the requests whose chains go on, each with the 4 bytes that a candidate must have to be longer than the best
+      // so far (and than least)
+      uint32_t at = 0;
+      if (ask) {
+        const uint32_t key = W.key[lane];
+        at = max(least, key ? k_len(key) : 0u);
+        ask = at < lim;
+      }
+      const unsigned am = __ballot_sync(kFull, ask);
+      if (!am) break;
+      const uint32_t mine = __popc(am & below);
+      if (ask) {
+        const uint32_t po = max(at, 3u) - 3u;
+        W.req[mine] = make_uint4(rt, x | po << 20, load4(P.in, P.base + x + po), lane << 20);
+      }
+      __syncwarp();
+      const uint32_t nreq = (uint32_t)__popc(am);
+      // a load is NR requests' first entries (sub 0), or 32 entries of a request's next 128
+      const uint32_t from = sub == 0 ? 0u : 128u * sub - 96u, nt = sub ? nreq * kTasks : (nreq + NR - 1) / NR;
+      uint32_t t = 0, ended = 0;  // ended: a bit for each request whose chain does not go on
+      do {
+        uint32_t cnt = 0;
+        while (t < nt && cnt <= 32) {
+          uint32_t e[kTasks], xp[kTasks], pw[kTasks], w[kTasks], slot[kTasks];
+          bool hit[kTasks];
 #pragma unroll
           for (uint32_t u = 0; u < kTasks; ++u) {
-            const uint32_t up = __shfl_up_sync(kFull, e_pos(e[u]), 1);  // (every lane takes part)
-            if (lane > 0 && e_pos(e[u]) >= up) end = true;
+            const uint32_t k = sub ? t / kTasks : (t + u) * NR + lane / G;
+            const uint32_t q = sub ? from + 32 * u + lane : gl;
+            const uint4 rq = W.req[min(k, nreq - 1u)];
+            const uint32_t r = rq.x & 0xFFFFFu;
+            xp[u] = rq.y; pw[u] = rq.z; slot[u] = rq.w;
+            e[u] = k < nreq && q < min(P.depth, r) ? P.srt[r - 1u - q] : ~rq.x;  // (else: another tag)
+            hit[u] = e[u] - (rq.x & 0xFFF00000u) < (rq.y & 0xFFFFFu);             // the same tag and an earlier position
           }
-          const uint32_t r = W.rt[s[0]] & 0xFFFFFu;
-          if (__any_sync(kFull, end) || r <= 32 * kTasks) t += kTasks;
+#pragma unroll
+          for (uint32_t u = 0; u < kTasks; ++u)
+            w[u] = hit[u] ? load4(P.in, P.base + e_pos(e[u]) + (xp[u] >> 20)) : 0u;
+#pragma unroll
+          for (uint32_t u = 0; u < kTasks; ++u) {
+            const bool pass = hit[u] && w[u] == pw[u];
+            const unsigned hm = __ballot_sync(kFull, pass);
+            if (pass) W.it[cnt + __popc(hm & below)] = slot[u] | e_pos(e[u]);
+            cnt += (uint32_t)__popc(hm);
+          }
+          if (sub + 1 < subs) {  // where the positions do not fall, or the order's start is reached, a chain has ended
+                                 // (entries of other hashes that this misses are harmless: their bytes differ)
+#pragma unroll
+            for (uint32_t u = 0; u < kTasks; ++u) {
+              const uint32_t up = __shfl_up_sync(kFull, e_pos(e[u]), 1);
+              const uint32_t k = sub ? t / kTasks : t + u;
+              if (__any_sync(kFull, lane > 0 && e_pos(e[u]) >= up)) ended |= 1u << (k & 31u);
+            }
+          }
+          t += kTasks;
         }
-      }
-      finish_lists(P, W, cnt, n2);
-      n2 = 0;
-    } while (t < nt);
+        finish_lists(P, W, cnt, 0);
+      } while (t < nt);
+      ask = ask && !(ended >> mine & 1u);
+    }
   }
   if (on1) {
     v2 = M_NONE;
@@ -820,7 +829,7 @@ struct StreamTile {
 constexpr uint32_t kCtaCopyRun = 2048;
 
 template <uint32_t NW>
-__global__ void __launch_bounds__(32 * NW, NW == 8 ? 8 : 1) k_enc_streams(EncArgs A) {
+__global__ void __launch_bounds__(32 * NW, NW == 8 ? 8 : NW == 16 ? 2 : 1) k_enc_streams(EncArgs A) {
   using T = StreamTile<NW>;
   constexpr uint32_t NT = T::NT, RM = T::RING - 1;
   __shared__ T S;
