@@ -126,8 +126,8 @@ int ensure_enc(zc_ctx* c, uint32_t nb, uint32_t block_log) {
   Need need[] = {
       {&c->e_tmp, N * 4}, {&c->e_srt, N * 4}, {&c->e_minfo, N * 4},
       {&c->e_scnt, (size_t)nb * ((B + 4095) / 4096) * 256 * 4},
-      {&c->e_tk_seg, (size_t)nb * 3 * zc::seg_tok_cap((uint32_t)B) * 4}, {&c->e_seg, (size_t)nb * zc::kMaxSegs * 4},
-      {&c->e_tmp_d, N}, {&c->e_tk_i, nb * TC * 4}, {&c->e_tk_m, nb * TC * 4}, {&c->e_tk_d, nb * TC * 4},
+      {&c->e_tk_seg, (size_t)nb * 2 * zc::seg_tok_cap((uint32_t)B) * 8}, {&c->e_seg, (size_t)nb * zc::kMaxSegs * 8},
+      {&c->e_tmp_d, N}, {&c->e_tk, nb * TC * 8},
       {&c->e_bcnt, (size_t)nb * 8 * 4}, {&c->e_lit, N}, {&c->e_tok, nb * TC}, {&c->e_ext, nb * EC},
       {&c->e_sym, nb * TC}, {&c->e_grp, nb * TC}, {&c->e_bits, (size_t)nb * zc::bits_cap((uint32_t)B)},
       {&c->e_lanes, (size_t)nb * zc::lanes_per_block((uint32_t)B)}, {&c->e_freq, (size_t)nb * 5 * 256 * 2},
@@ -201,10 +201,10 @@ int encode_device(zc_ctx* c, const uint8_t* d_in, const uint64_t* d_off, const u
   A.B = 1u << block_log; A.block_log = block_log; A.depth = depth_for_level(level);
   A.tmp_e = c->e_tmp.as<uint32_t>(); A.tmp_d = c->e_tmp_d.as<uint8_t>(); A.srt = c->e_srt.as<uint32_t>();
   A.minfo = c->e_minfo.as<uint32_t>(); A.scnt = c->e_scnt.as<uint32_t>();
-  A.tk_seg = c->e_tk_seg.as<uint32_t>(); A.seg_exit = c->e_seg.as<uint32_t>();
+  A.tk_seg = c->e_tk_seg.as<uint2>(); A.seg_exit = c->e_seg.as<uint2>();
   A.nseg = enc_segments(nb, block_log);
   A.walk_segs = (uint64_t)nb * A.nseg < 4 * 148u * 1024u ? 32 : 64;  // (64: two a lane, once they fill the GPU twice)
-  A.tk_i = c->e_tk_i.as<uint32_t>(); A.tk_m = c->e_tk_m.as<uint32_t>(); A.tk_d = c->e_tk_d.as<uint32_t>();
+  A.tk = c->e_tk.as<uint2>();
   A.bcnt = c->e_bcnt.as<uint32_t>();
   A.s_lit = c->e_lit.as<uint8_t>(); A.s_tok = c->e_tok.as<uint8_t>(); A.s_ext = c->e_ext.as<uint8_t>();
   A.s_sym = c->e_sym.as<uint8_t>(); A.s_grp = c->e_grp.as<uint8_t>(); A.s_bits = c->e_bits.as<uint8_t>();
@@ -446,8 +446,8 @@ void zc_close(zc_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   if (c->cstream) cudaStreamSynchronize(c->cstream);
   drop_graphs(c);
-  for (DevBuf* b : {&c->e_tmp, &c->e_tmp_d, &c->e_srt, &c->e_minfo, &c->e_scnt, &c->e_tk_seg, &c->e_seg, &c->e_tk_i,
-                    &c->e_tk_m, &c->e_tk_d, &c->e_bcnt, &c->e_lit, &c->e_tok, &c->e_ext, &c->e_sym, &c->e_grp,
+  for (DevBuf* b : {&c->e_tmp, &c->e_tmp_d, &c->e_srt, &c->e_minfo, &c->e_scnt, &c->e_tk_seg, &c->e_seg, &c->e_tk,
+                    &c->e_bcnt, &c->e_lit, &c->e_tok, &c->e_ext, &c->e_sym, &c->e_grp,
                     &c->e_bits, &c->e_lanes, &c->e_freq, &c->e_lanelen, &c->e_sinfo, &c->e_slab, &c->d_lit, &c->d_tok,
                     &c->d_sym, &c->d_grp, &c->d_ext, &c->d_meta, &c->d_tkp, &c->d_tkd, &c->d_line, &c->s_in, &c->s_blk, &c->s_out, &c->s_meta, &c->work,
                     &c->a_desc, &c->a_work})

@@ -89,7 +89,7 @@ struct zc_ctx {
   zch::StageRecords records;
   zc::CrcTables* d_crct = nullptr;
   // encoder scratch (sized by capacity: any block size whose blocks fit)
-  zch::DevBuf e_tmp, e_tmp_d, e_srt, e_minfo, e_scnt, e_tk_seg, e_seg, e_tk_i, e_tk_m, e_tk_d, e_bcnt, e_lit, e_tok,
+  zch::DevBuf e_tmp, e_tmp_d, e_srt, e_minfo, e_scnt, e_tk_seg, e_seg, e_tk, e_bcnt, e_lit, e_tok,
       e_ext, e_sym, e_grp, e_bits, e_lanes, e_freq, e_lanelen, e_sinfo, e_slab;
   // decoder scratch (likewise)
   zch::DevBuf d_lit, d_tok, d_sym, d_grp, d_ext, d_meta, d_tkp, d_tkd, d_line;

@@ -84,11 +84,11 @@ struct EncArgs {
   uint32_t *tmp_e, *srt, *minfo;  // sort entries after pass 0 and in order; match records
   uint8_t* tmp_d;                 // the entries' digits of pass 1, beside tmp_e
   uint32_t* scnt;                 // sort: per block ceil(B / 4096) * 256 tile digit counts / starts
-  uint32_t *tk_i, *tk_m, *tk_d;   // tokens, tok_cap(B) per block
-  uint32_t* tk_seg;               // the parse's per-segment token slots: 3 * seg_tok_cap(B) per block
+  uint2* tk;                      // tokens, tok_cap(B) per block
+  uint2* tk_seg;                  // per-segment token slots, of the first walk and of the re-walk: 2 * seg_tok_cap(B) per block
   uint32_t nseg;                  // segments a block is parsed in: 256, 512 or 1024
   uint32_t walk_segs;             // of those, how many a warp of k_enc_walk takes: 32 or 64
-  uint32_t* seg_exit;             // where each segment's first walk leaves it: nseg per block
+  uint2* seg_exit;                // where each segment's first walk leaves it, and its tokens: nseg per block
   uint32_t* bcnt;                 // per block [8]: nt, nl, ne, nob, ng, payload size, method
   uint8_t *s_lit, *s_tok, *s_ext, *s_sym, *s_grp, *s_bits;
   uint8_t* lanes;                 // rANS lane scratch, lanes_per_block(B) per block
