@@ -63,14 +63,14 @@ def test_finished_matches(codec, name, level):
 
 @pytest.mark.parametrize("level", [1, 5])
 def test_segment_counts(codec, level):
-    """One launch of 2048 and one of 2560 blocks of 64 KiB (fewer segments a block, 32 and 64 a warp) against launches
-    of 64 blocks (1024 segments a block): the blocks repeat, so their payloads must."""
+    """One launch of 512 blocks of 256 KiB (256-byte segments) and one of 1408 (512-byte segments) against launches of 16
+    blocks: the blocks repeat, so their payloads must."""
     import datagen as G
-    block_log, nb, reps = 16, 512, 9
+    block_log, nb, reps = 18, 128, 15
     tile = G.lz_mix(nb << block_log, block_log, 3)
     small = []
-    for k in range(0, nb, 64):
-        m, n, _, p, o = codec.compress_arrays(tile[k << block_log:(k + 64) << block_log], block_log, level=level)
+    for k in range(0, nb, 16):
+        m, n, _, p, o = codec.compress_arrays(tile[k << block_log:(k + 16) << block_log], block_log, level=level)
         small += [p[int(a): int(a) + int(b)].tobytes() for a, b in zip(o, n)]
         assert m.all()
     m, n, _, p, o = codec.compress_arrays(np.tile(tile, reps), block_log, level=level)

@@ -158,14 +158,13 @@ uint32_t dec_blocks_per_launch(uint32_t block_log) {
   return (uint32_t)std::min<size_t>(((size_t)4 << 30) >> block_log, 1u << 20);
 }
 
-// segments a block is parsed in: 1 KiB each, a lane's walk, where that fills the GPU (148 SMs x 1024 walks);
-// fewer blocks are cut finer, down to 1024 segments, so that the walks spread over more SMs
-// (64 MiB of text, 256 blocks of 256 KiB: the walks take 5.7 ms at 256 segments a block, 3.1 at 512, 1.7 at 1024;
-// 1 GiB of lz_mix: 14.3, 14.0, 15.0 ms with the parse, whose re-walks grow with the segments)
+// segments a block is parsed in: 512 bytes each, a lane's walk; 256 in launches whose 256-byte segments would not
+// keep every SM's 1024 walks busy eight times over, so that the walks end sooner.  Shorter ones cost more re-walked
+// steps.  ms of walks and parse: 1 GiB of lz_mix, block 18, in 1024 / 512 / 256 bytes 11.7 / 11.0 / 11.6; 571 blocks of
+// files 6.0 / 3.0 / 2.5; 256 blocks of text 5.4 / 2.2 / 2.0.
 uint32_t enc_segments(uint32_t nb, uint32_t block_log) {
-  uint32_t s = std::min(std::max((1u << block_log) / 1024u, 256u), zc::kMaxSegs);
-  while (s < zc::kMaxSegs && (uint64_t)nb * s < 148u * 1024u) s *= 2;
-  return s;
+  const uint32_t bytes = ((uint64_t)nb << block_log) < 8ull * 148 * 1024 * 256 ? 256 : 512;
+  return std::min(std::max((1u << block_log) / bytes, 256u), zc::kMaxSegs);
 }
 
 // The test injector (src/safe_codec.h:17 has the reference's): with ZC_FAIL_AFTER=n in the environment
@@ -203,7 +202,6 @@ int encode_device(zc_ctx* c, const uint8_t* d_in, const uint64_t* d_off, const u
   A.minfo = c->e_minfo.as<uint32_t>(); A.scnt = c->e_scnt.as<uint32_t>();
   A.tk_seg = c->e_tk_seg.as<uint2>(); A.seg_exit = c->e_seg.as<uint2>();
   A.nseg = enc_segments(nb, block_log);
-  A.walk_segs = (uint64_t)nb * A.nseg < 4 * 148u * 1024u ? 32 : 64;  // (64: two a lane, once they fill the GPU twice)
   A.tk = c->e_tk.as<uint2>();
   A.bcnt = c->e_bcnt.as<uint32_t>();
   A.s_lit = c->e_lit.as<uint8_t>(); A.s_tok = c->e_tok.as<uint8_t>(); A.s_ext = c->e_ext.as<uint8_t>();

@@ -87,7 +87,6 @@ struct EncArgs {
   uint2* tk;                      // tokens, tok_cap(B) per block
   uint2* tk_seg;                  // per-segment token slots, of the first walk and of the re-walk: 2 * seg_tok_cap(B) per block
   uint32_t nseg;                  // segments a block is parsed in: 256, 512 or 1024
-  uint32_t walk_segs;             // of those, how many a warp of k_enc_walk takes: 32 or 64
   uint2* seg_exit;                // where each segment's first walk leaves it, and its tokens: nseg per block
   uint32_t* bcnt;                 // per block [8]: nt, nl, ne, nob, ng, payload size, method
   uint8_t *s_lit, *s_tok, *s_ext, *s_sym, *s_grp, *s_bits;
