@@ -1097,9 +1097,10 @@ __global__ void __launch_bounds__(64) k_enc_rans(EncArgs A) {
   const uint32_t LC = lane_cap(A.B, s);
   uint8_t* end = A.lanes + (size_t)b * lanes_per_block(A.B) + lane_base(A.B, s) + (size_t)(k + 1) * LC;
   uint8_t* ptr = end;
-  // output bytes go down from the lane's (16-byte aligned) end; they are gathered four at a time, the
-  // first at bits 31..24, and stored as aligned words
-  uint32_t acc = 0, pend = 0;
+  // output bytes go down from the lane's (16-byte aligned) end; they are gathered in acc, the first of its `pend` bytes
+  // highest, and stored as aligned words
+  uint64_t acc = 0;
+  uint32_t pend = 0;
   uint32_t x = kRansLow;
   // The stream in chunks of kRansChunk symbols (a whole number of rounds of the 64 lanes), last chunk
   // first: the CTA stages a chunk in shared memory with coalesced loads, then lane k codes its symbols
@@ -1122,26 +1123,33 @@ __global__ void __launch_bounds__(64) k_enc_rans(EncArgs A) {
       // x' = (x / f) * 4096 + x % f + cum = x + cum + q * (4096 - f), with q = x / f by an exact
       // reciprocal: for x < 2^31 and s = ceil(log2 f), floor(x * ceil(2^(31+s) / f) / 2^(31+s)) = x / f
       // (the product's error is below x / 2^(31+s) < 2^-s <= 1/f, less than the gap to the next integer)
-      for (int32_t t = (int32_t)(k + (cn - 1 - k) / kLanes * kLanes); t >= 0; t -= (int32_t)kLanes) {
-        const uint32_t c = stage[t], e = fc[c], m = rcp[c];
-        const uint32_t f = e & 0x1FFFu;
-        const uint32_t xmax = f << (23 - kScaleBits + 8);
-        while (x >= xmax) {
-          acc |= (x & 0xFFu) << (24u - 8u * pend);
-          x >>= 8;
-          if (++pend == 4u) {
-            ptr -= 4;
-            *reinterpret_cast<uint32_t*>(ptr) = acc;
-            acc = 0;
-            pend = 0;
-          }
+      // A symbol emits the state's low byte when it is at least f << 19, two when its upper bytes are too (never more:
+      // x < 2^31).  Only that, the product and the sum are on the state's chain: the next symbol's table entries are
+      // looked up before this one is coded.
+      int32_t t = (int32_t)(k + (cn - 1 - k) / kLanes * kLanes);
+      uint32_t e = fc[stage[t]], m = rcp[stage[t]];
+      for (;;) {
+        const uint32_t ce = e, cm = m;
+        t -= (int32_t)kLanes;
+        if (t >= 0) { e = fc[stage[t]]; m = rcp[stage[t]]; }
+        const uint32_t f = ce & 0x1FFFu, xmax = f << (23 - kScaleBits + 8);
+        const bool one = x >= xmax, two = x >> 8 >= xmax;
+        const uint32_t b1 = x & 0xFFu, b2 = __byte_perm(x, 0, 0x4401);
+        acc = two ? acc << 16 | b2 : one ? acc << 8 | b1 : acc;
+        pend += (uint32_t)one + two;
+        x = two ? x >> 16 : one ? x >> 8 : x;
+        if (pend >= 4u) {
+          pend -= 4u;
+          ptr -= 4;
+          *reinterpret_cast<uint32_t*>(ptr) = (uint32_t)(acc >> (8u * pend));
         }
-        const uint32_t q = f == 1 ? x : __umulhi(x, m) >> (e >> 25);
-        x += ((e >> 13) & 0xFFFu) + q * (kScale - f);
+        const uint32_t q = f == 1 ? x : __umulhi(x, cm) >> (ce >> 25);
+        x += ((ce >> 13) & 0xFFFu) + q * (kScale - f);
+        if (t < 0) break;
       }
     }
   }
-  for (uint32_t i = 0; i < pend; ++i) *--ptr = (uint8_t)(acc >> (24u - 8u * i));  // the bytes still gathered
+  for (uint32_t i = pend; i > 0; --i) *--ptr = (uint8_t)(acc >> (8u * (i - 1u)));  // the bytes still gathered
   ptr -= 4;
   st32(ptr, x);
   const uint32_t ll = (uint32_t)(end - ptr);
