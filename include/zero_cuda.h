@@ -289,7 +289,7 @@ int zc_archive_write_range(zc_ctx *ctx, const uint8_t *d_range, uint64_t range_o
 
 /* The same from host memory into host memory (synchronous): solid holds the files' bytes in entry order;
  * *out_len gets the archive's length and entries[i].crc each entry's CRC.  The stream goes through the GPU
- * in chunks (128 MiB, then 512 MiB): a chunk's upload and the previous chunk's records coming down
+ * in chunks (64, 128, then 256 MiB): a chunk's upload and the previous chunk's records coming down
  * overlap the chunk's kernels.  out_cap = zc_archive_bound is always enough. */
 int zc_archive_write(zc_ctx *ctx, const uint8_t *solid, uint32_t block_log, int level, zc_entry *entries,
                      uint32_t n_entries, uint8_t *out, uint64_t out_cap, uint64_t *out_len);

@@ -63,17 +63,27 @@ def test_finished_matches(codec, name, level):
 
 @pytest.mark.parametrize("level", [1, 5])
 def test_segment_counts(codec, level):
-    """One launch of 512 blocks of 256 KiB (256-byte segments) and one of 1408 (512-byte segments) against launches of 16
-    blocks: the blocks repeat, so their payloads must."""
+    """One device launch of 1408 blocks of 256 KiB (512-byte segments) against launches of 16 blocks (256-byte segments):
+    the blocks repeat, so their payloads must."""
     import datagen as G
-    block_log, nb, reps = 18, 128, 15
+    import torch
+    block_log, nb, reps = 18, 128, 11
+    B = 1 << block_log
     tile = G.lz_mix(nb << block_log, block_log, 3)
     small = []
     for k in range(0, nb, 16):
         m, n, _, p, o = codec.compress_arrays(tile[k << block_log:(k + 16) << block_log], block_log, level=level)
         small += [p[int(a): int(a) + int(b)].tobytes() for a, b in zip(o, n)]
         assert m.all()
-    m, n, _, p, o = codec.compress_arrays(np.tile(tile, reps), block_log, level=level)
+    total = nb * reps
+    z = lambda k, t: torch.zeros(k, dtype=t, device="cuda")  # noqa: E731
+    d_in = z(total * B + 64, torch.uint8)
+    d_in[: total * B] = torch.from_numpy(tile).cuda().repeat(reps)
+    offs, lens = torch.arange(total, device="cuda") * B, torch.full((total,), B, dtype=torch.int32, device="cuda")
+    m, n, crc, out, at, end = (z(total, torch.uint8), z(total, torch.int32), z(total, torch.int32), z(total * B, torch.uint8),
+                               z(total, torch.int64), z(1, torch.int64))
+    codec.compress_device(d_in, offs, lens, total, block_log, m, n, crc, out, at, end, level=level)
+    m, n, at, out = m.cpu().numpy(), n.cpu().numpy(), at.cpu().numpy(), out[: int(end.item())].cpu().numpy()
     assert m.all()
-    for b in range(nb * reps):
-        assert p[int(o[b]): int(o[b]) + int(n[b])].tobytes() == small[b % nb], f"block {b}"
+    for b in range(total):
+        assert out[int(at[b]): int(at[b]) + int(n[b])].tobytes() == small[b % nb], f"block {b}"

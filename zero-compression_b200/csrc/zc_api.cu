@@ -243,10 +243,12 @@ int decode_device(zc_ctx* c, const uint8_t* d_comp, const uint64_t* d_comp_offs,
   return check_launch(c, "decoder launch");
 }
 
-// blocks in chunk `i` of a host-pointer call: 128 MiB first (so the first kernels start early and the
-// copies left exposed are short), then 512 MiB, so that a large call's copies overlap kernels
+// blocks in chunk `i` of a host-pointer call: 64, 128, then 256 MiB, so that a large call's copies overlap kernels
+// and the copies left exposed, the first chunk's upload and the last one's results, are short.  ms to compress and
+// decompress lz_mix at block 18, level 5 (kernels that fill the GPU with few blocks made smaller chunks pay): 256 MiB
+// 18.5 in 128 MiB chunks, 16.9 in these; 1 GiB 64.9 in 128, then 512 MiB, 62.3 in 64, then 128, 61.4 in 64, then 256
 uint32_t host_chunk_blocks(uint32_t block_log, uint32_t per_launch, uint32_t i) {
-  const size_t bytes = (size_t)(i == 0 ? 128 : 512) << 20;
+  const size_t bytes = (size_t)(i == 0 ? 64 : i == 1 ? 128 : 256) << 20;
   return std::max<uint32_t>(1, std::min<uint32_t>(per_launch, (uint32_t)(bytes >> block_log)));
 }
 

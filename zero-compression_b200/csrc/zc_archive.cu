@@ -583,7 +583,7 @@ void pieces_in(const Pieces& P, uint64_t lo, uint64_t hi, uint32_t& q0, uint32_t
   q1 = (uint32_t)(std::lower_bound(P.part_off.begin(), P.part_off.end(), hi) - P.part_off.begin());
 }
 
-// Host-pointer archive write.  The solid stream goes up in chunks of whole blocks (128 MiB, then 512 MiB)
+// Host-pointer archive write.  The solid stream goes up in chunks of whole blocks (64, 128, then 256 MiB)
 // through the context's two stages: a chunk's upload and the previous chunk's records coming down (copy
 // stream) overlap the chunk's kernels.  Each chunk's records are written from the start of its stage
 // buffer; the partial file pieces inside the chunk get their CRCs while it is resident.  At the end the

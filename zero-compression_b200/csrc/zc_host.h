@@ -119,7 +119,7 @@ int fail(zc_ctx* c, int code, const std::string& msg);
 int cuda_fail(zc_ctx* c, cudaError_t e, const char* what);
 cudaError_t grow(DevBuf& b, size_t bytes);
 cudaError_t grow_host(HostBuf& b, size_t bytes);  // pinned
-// blocks in chunk `i` of a host-pointer call: 128 MiB first, then 512 MiB (at most per_launch)
+// blocks in chunk `i` of a host-pointer call: 64, 128, then 256 MiB (at most per_launch)
 uint32_t host_chunk_blocks(uint32_t block_log, uint32_t per_launch, uint32_t i);
 bool bad_block_log(uint32_t bl);
 uint32_t enc_blocks_per_launch(uint32_t block_log);
