@@ -22,7 +22,7 @@
 //                  placed by scans, offset bits gathered in shared memory, literals
 //   k_enc_rans     one CTA per (block, stream): histogram, 12-bit normalisation with the reference's
 //                  tie-breaks, 64 lanes coding backwards (src/codec.h:41-147)
-//   k_enc_pack     one CTA per block: the payload (src/codec2.h:139-152), or "stored"
+//   k_enc_pack     one CTA per (block, part): the payload (src/codec2.h:139-152), or "stored"
 //   k_enc_scan / k_enc_emit: record sizes -> offsets, payloads packed back to back
 #include "zc_internal.cuh"
 #include "zc_kernels.h"
@@ -784,7 +784,7 @@ __global__ void __launch_bounds__(T, 1024 / T) k_enc_parse(EncArgs A) {
 // ---------------------------------------------------------------- 4. tokens -> streams
 constexpr uint32_t kWarpCopyRun = 32;
 
-// n bytes from src, a range of the codec's input (16-byte aligned, 64 readable bytes after its end), to
+// n bytes from src, a range of the codec's input (16-byte aligned, 64 readable bytes after its end) or scratch, to
 // dst by nth threads, this one thread t of them: 4-byte words stored aligned at dst, each built by a funnel shift from
 // the two aligned input words that cover it (those may reach a few bytes past the range, into the
 // input's slack, never before the input's start), four words a thread in flight.
@@ -1172,70 +1172,67 @@ __global__ void __launch_bounds__(64) k_enc_rans(EncArgs A) {
 }
 
 // ---------------------------------------------------------------- 6. the payload
+// A CTA per (block, part): parts 0..4 are the streams' sections, part 5 the counts and the offset bits; each finds its
+// place from the five sections' lengths.  Bytes are copied as aligned words (copy_in).  (One CTA per block, a byte a
+// thread: 0.046 ms for one text block against 0.013, 0.39 for 1000 files against 0.10.)
 __global__ void __launch_bounds__(256) k_enc_pack(EncArgs A) {
-  const uint32_t b = blockIdx.x, tid = threadIdx.x;
+  const uint32_t b = blockIdx.x, s = blockIdx.y, tid = threadIdx.x;
   const uint32_t n = A.in_len[b];
   uint32_t* c = A.bcnt + b * 8;
   const uint32_t nob = c[3];
-  uint64_t off[6];
-  off[0] = kHdrBytes;
-  for (uint32_t s = 0; s < 5; ++s) off[s + 1] = off[s] + 5 + A.sinfo[(size_t)(b * 5 + s) * 4 + 1];
-  const uint64_t total = off[5] + nob;
-  if (total >= n) {  // stored (src/codec2.h:152, src/archive.h:394)
-    if (tid == 0) { c[5] = n; c[6] = 0; }
+  uint64_t at = kHdrBytes, total = kHdrBytes + (uint64_t)nob;
+  for (uint32_t k = 0; k < 5; ++k) {
+    const uint32_t len = 5 + A.sinfo[(size_t)(b * 5 + k) * 4 + 1];
+    if (k < s) at += len;
+    total += len;
+  }
+  const bool stored = total >= n;  // (src/codec2.h:152, src/archive.h:394)
+  uint8_t* o = A.slab + (size_t)b * A.B;
+  if (s == 5) {
+    if (tid == 0) { c[5] = stored ? n : (uint32_t)total; c[6] = stored ? 0 : 1; }
+    if (stored) return;
+    if (tid == 0) { st32(o, c[0]); st32(o + 4, c[1]); st32(o + 8, c[2]); st32(o + 12, nob); st32(o + 16, c[4]); }
+    copy_in(o + at, A.s_bits + (size_t)b * bits_cap(A.B), nob, tid, 256);
     return;
   }
-  uint8_t* o = A.slab + (size_t)b * A.B;
-  if (tid == 0) {
-    st32(o, c[0]); st32(o + 4, c[1]); st32(o + 8, c[2]); st32(o + 12, nob); st32(o + 16, c[4]);
-    c[5] = (uint32_t)total; c[6] = 1;
-  }
+  if (stored) return;
   __shared__ uint32_t lofs[kLanes + 1];
   __shared__ uint32_t wcnt[8];
-  for (uint32_t s = 0; s < 5; ++s) {
-    const uint32_t g = b * 5 + s;
-    const uint32_t* info = A.sinfo + (size_t)g * 4;
-    const uint32_t kind = info[0], len = info[1], np = info[2], ns = info[3];
-    uint8_t* d = o + off[s];
-    if (tid == 0) { d[0] = (uint8_t)kind; st32(d + 1, len); }
-    const uint8_t* sym = stream_syms(A, b, s);
-    if (kind == 0) {
-      for (uint32_t i = tid; i < ns; i += blockDim.x) d[5 + i] = sym[i];
-      continue;
-    }
-    const uint16_t* fq = A.freq + (size_t)g * 256;
-    // present bitmap, then the frequencies of the present symbols in symbol order
-    const uint32_t f = fq[tid];
-    const uint32_t pres = f != 0;
-    const unsigned bal = __ballot_sync(kFull, pres);
-    if ((tid & 7u) == 0) d[5 + (tid >> 3)] = (uint8_t)((bal >> (tid & 31u)) & 0xFFu);
-    if ((tid & 31u) == 0) wcnt[tid >> 5] = __popc(bal);
-    __syncthreads();
-    uint32_t idx = __popc(bal & ((1u << (tid & 31u)) - 1u));
-    for (uint32_t k = 0; k < (tid >> 5); ++k) idx += wcnt[k];
-    if (pres) { d[5 + 32 + 2 * idx] = (uint8_t)f; d[5 + 32 + 2 * idx + 1] = (uint8_t)(f >> 8); }
-    const uint32_t* ll = A.lanelen + (size_t)g * kLanes;
-    if (tid < kLanes) st32(d + 5 + 32 + 2 * np + 4 * tid, ll[tid]);
-    if (tid < 32) {
-      const uint32_t a = ll[2 * tid], bb = ll[2 * tid + 1];
-      const uint32_t inc = warp_incl_scan(a + bb);
-      lofs[2 * tid] = inc - a - bb;
-      lofs[2 * tid + 1] = inc - bb;
-    }
-    __syncthreads();
-    const uint32_t data0 = 5 + 32 + 2 * np + 4 * kLanes;
-    const uint32_t LC = lane_cap(A.B, s);
-    const uint8_t* lb = A.lanes + (size_t)b * lanes_per_block(A.B) + lane_base(A.B, s);
-    for (uint32_t jl = tid >> 5; jl < kLanes; jl += blockDim.x >> 5) {
-      const uint32_t len_j = ll[jl];
-      const uint8_t* srcp = lb + (size_t)(jl + 1) * LC - len_j;
-      uint8_t* dst = d + data0 + lofs[jl];
-      for (uint32_t i = lane_id(); i < len_j; i += 32) dst[i] = srcp[i];
-    }
-    __syncthreads();
+  const uint32_t g = b * 5 + s;
+  const uint32_t* info = A.sinfo + (size_t)g * 4;
+  const uint32_t kind = info[0], len = info[1], np = info[2], ns = info[3];
+  uint8_t* d = o + at;
+  if (tid == 0) { d[0] = (uint8_t)kind; st32(d + 1, len); }
+  if (kind == 0) {
+    copy_in(d + 5, stream_syms(A, b, s), ns, tid, 256);
+    return;
   }
-  const uint8_t* bits = A.s_bits + (size_t)b * bits_cap(A.B);
-  for (uint32_t i = tid; i < nob; i += blockDim.x) o[off[5] + i] = bits[i];
+  const uint16_t* fq = A.freq + (size_t)g * 256;
+  // present bitmap, then the frequencies of the present symbols in symbol order
+  const uint32_t f = fq[tid];
+  const uint32_t pres = f != 0;
+  const unsigned bal = __ballot_sync(kFull, pres);
+  if ((tid & 7u) == 0) d[5 + (tid >> 3)] = (uint8_t)((bal >> (tid & 31u)) & 0xFFu);
+  if ((tid & 31u) == 0) wcnt[tid >> 5] = __popc(bal);
+  const uint32_t* ll = A.lanelen + (size_t)g * kLanes;
+  if (tid < 32) {
+    const uint32_t a = ll[2 * tid], bb = ll[2 * tid + 1];
+    const uint32_t inc = warp_incl_scan(a + bb);
+    lofs[2 * tid] = inc - a - bb;
+    lofs[2 * tid + 1] = inc - bb;
+  }
+  __syncthreads();
+  uint32_t idx = __popc(bal & ((1u << (tid & 31u)) - 1u));
+  for (uint32_t k = 0; k < (tid >> 5); ++k) idx += wcnt[k];
+  if (pres) { d[5 + 32 + 2 * idx] = (uint8_t)f; d[5 + 32 + 2 * idx + 1] = (uint8_t)(f >> 8); }
+  if (tid < kLanes) st32(d + 5 + 32 + 2 * np + 4 * tid, ll[tid]);
+  const uint32_t data0 = 5 + 32 + 2 * np + 4 * kLanes;
+  const uint32_t LC = lane_cap(A.B, s);
+  const uint8_t* lb = A.lanes + (size_t)b * lanes_per_block(A.B) + lane_base(A.B, s);
+  for (uint32_t jl = tid >> 5; jl < kLanes; jl += 8) {
+    const uint32_t len_j = ll[jl];
+    copy_in(d + data0 + lofs[jl], lb + (size_t)(jl + 1) * LC - len_j, len_j, lane_id(), 32);
+  }
 }
 
 // ---------------------------------------------------------------- 7. record bodies back to back
@@ -1379,7 +1376,7 @@ void launch_encode(const EncArgs& A, const CrcArgs& crc_in, cudaStream_t st, Sta
   k_enc_rans<<<dim3(A.nb, 5), 64, 0, st>>>(A);
   S.end(st);
   S.begin("k_enc_pack", st);
-  k_enc_pack<<<A.nb, 256, 0, st>>>(A);
+  k_enc_pack<<<dim3(A.nb, 6), 256, 0, st>>>(A);
   S.end(st);
   S.begin("k_enc_scan", st);
   k_enc_scan<<<1, 1024, 0, st>>>(A);
