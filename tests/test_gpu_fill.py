@@ -58,3 +58,18 @@ def test_whole_blocks(codec, block_log):
     data = np.concatenate([material(3 * B, 5), material(B, 6)])
     lens = np.array([77, B, B, B - 1, 1], np.uint32)
     round_trip(codec, data, np.cumsum(np.concatenate([[0], lens[:-1]])).astype(np.uint64), lens, block_log)
+
+
+@pytest.mark.parametrize("copies", [0, 1, 3, 4, 5, 2047, 2048, 2049, 4097, 9000])
+def test_token_counts(codec, copies):
+    """About as many tokens as copies: on both sides of the token scan's four a thread and 2048 a tile, with groups of up
+    to 255 tokens and offsets that repeat (recent-offset symbols naming tokens of this tile and earlier ones)."""
+    r = np.random.default_rng(copies + 1)
+    src = r.integers(0, 256, 3000, dtype=np.uint8)
+    out = [src]
+    for k in range(copies):
+        at = int(r.integers(0, 2900)) if k % 3 else 40 * (k % 7)
+        out += [src[at: at + int(r.integers(5, 25))], r.integers(0, 256, int(r.integers(0, 2)), dtype=np.uint8)]
+    data = np.concatenate(out)
+    assert data.size < 1 << 18
+    round_trip(codec, data, np.zeros(1, np.uint64), np.array([data.size], np.uint32), 18)

@@ -1,11 +1,11 @@
 // zc_decode_fill.cu -- the ZB2 LZ replay in two kernels (src/codec2.h:155-203):
 //
-//   k_dec_tokens  one CTA of 1024 threads per block: every token's literal run and match length (ext
+//   k_dec_tokens  one CTA per block: every token's literal run and match length (ext
 //                 bytes), offset (offset bits), output start and literal start, from block-wide scans, in
 //                 parallel over the tokens; which token holds each 128-byte line's first byte; then the groups
 //                 (a scan of their counts) and the recent-offset symbols (each names an earlier token's offset,
-//                 src/codec2.h:180-192), resolved by pointer jumping over all tokens at once.  Every check of the
-//                 reference decoder is made here; a failing one records a status and the block is not replayed.
+//                 src/codec2.h:180-192), resolved by pointer jumping within each tile.  Every check of the reference
+//                 decoder is made here; a failing one records a status and the block is not replayed.
 //   k_dec_fill    one warp per block: fills the block in rounds of 128 output bytes (a 4-byte word a lane)
 //                 straight through, group boundaries or not: a byte whose source lies earlier in the same
 //                 round is passed along by shuffles once known; the token table is a 64-row ring in shared
@@ -24,27 +24,53 @@ namespace {
 
 __device__ __forceinline__ void flag(uint32_t* err, uint32_t b, uint32_t code) { atomicCAS(err + b, 0u, code); }
 
-// exclusive scan over the CTA (blockDim.x == 1024); returns the prefix, `total` gets the sum.  ws: 32 words
-__device__ __forceinline__ uint32_t cta_scan(uint32_t v, uint32_t* ws, uint32_t& total) {
-  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-  const uint32_t inc = warp_incl_scan(v);
-  if (lane == 31) ws[w] = inc;
-  __syncthreads();
-  if (w == 0) {
-    const uint32_t x = ws[lane];
-    const uint32_t xi = warp_incl_scan(x);
-    ws[lane] = xi - x;
-    if (lane == 31) ws[32] = xi;
+// Scans over a CTA of 32 NW threads with one barrier each: every warp scans all the warps' totals for itself, and a
+// scan's totals lie in the row of ws that the scan before it did not use, so none can still be read when they are
+// written.
+template <uint32_t NW>
+struct CtaScan {
+  uint64_t (*sums)[NW];
+  uint32_t (*maxs)[NW];
+  uint32_t row = 0;
+  __device__ CtaScan(uint64_t (*s)[NW], uint32_t (*m)[NW]) : sums(s), maxs(m) {}
+  // the sum over the threads before this one (`total`: over all), and the maximum of `top` over them
+  __device__ __forceinline__ uint64_t operator()(uint64_t v, uint64_t& total, uint32_t top, uint32_t& top_before,
+                                                 uint32_t& top_all) {
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    uint64_t inc = v;
+    uint32_t mx = top;
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+      const uint64_t y = __shfl_up_sync(kFull, inc, o);
+      const uint32_t z = __shfl_up_sync(kFull, mx, o);
+      if (lane >= o) { inc += y; mx = max(mx, z); }
+    }
+    if (lane == 31) { sums[row][w] = inc; maxs[row][w] = mx; }
+    __syncthreads();
+    const uint64_t x = lane < NW ? sums[row][lane] : 0ull;
+    const uint32_t xm = lane < NW ? maxs[row][lane] : 0u;
+    uint64_t xi = x;
+    uint32_t mi = xm;
+#pragma unroll
+    for (uint32_t o = 1; o < NW; o <<= 1) {
+      const uint64_t y = __shfl_up_sync(kFull, xi, o);
+      const uint32_t z = __shfl_up_sync(kFull, mi, o);
+      if (lane >= o) { xi += y; mi = max(mi, z); }
+    }
+    row ^= 1u;
+    total = __shfl_sync(kFull, xi, NW - 1);
+    top_all = __shfl_sync(kFull, mi, NW - 1);
+    const uint32_t warps = __shfl_sync(kFull, mi, w ? w - 1u : 0u), up = __shfl_up_sync(kFull, mx, 1);
+    top_before = max(w ? warps : 0u, lane ? up : 0u);
+    return __shfl_sync(kFull, xi - x, w) + inc - v;
   }
-  __syncthreads();
-  const uint32_t r = ws[w] + inc - v;
-  total = ws[32];
-  __syncthreads();
-  return r;
-}
+  __device__ __forceinline__ uint64_t operator()(uint64_t v, uint64_t& total) {
+    uint32_t a, b;
+    return (*this)(v, total, 0u, a, b);
+  }
+};
 
-constexpr uint32_t kRepMark = 0x80000000u;  // a recent-offset symbol not resolved yet: kRepMark | index
-constexpr uint32_t kGrpStart = 0x40000000u; // (while groups are scanned) the first token of a group
+constexpr uint32_t kRepMark = 0x80000000u;  // a recent-offset symbol not resolved yet: kRepMark | the token it names
 
 // A token's row: its output start and its literals' start before it (21 bits each: start - literal start is never
 // negative), and its literal count (21 bits, split over the two words' upper bits).
@@ -55,46 +81,45 @@ __device__ __forceinline__ uint32_t row_start(const uint2& r) { return r.x & 0x1
 __device__ __forceinline__ uint32_t row_back(const uint2& r) { return r.y & 0x1FFFFFu; }  // start - literal start
 __device__ __forceinline__ uint32_t row_lits(const uint2& r) { return r.x >> 21 | r.y >> 21 << 11; }
 
-// inclusive max over the CTA in thread order (blockDim.x == 1024); `total` gets the CTA's max.  ws: 33 words
-__device__ __forceinline__ uint32_t cta_max_incl(uint32_t v, uint32_t* ws, uint32_t& total) {
-  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-  uint32_t x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(kFull, x, o);
-    if (lane >= (uint32_t)o) x = max(x, y);
-  }
-  if (lane == 31) ws[w] = x;
-  __syncthreads();
-  if (w == 0) {
-    uint32_t z = ws[lane];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(kFull, z, o);
-      if (lane >= (uint32_t)o) z = max(z, y);
-    }
-    ws[lane] = z;  // inclusive over warps
-  }
-  __syncthreads();
-  const uint32_t r = w ? max(x, ws[w - 1]) : x;
-  total = ws[31];
-  __syncthreads();
-  return r;
+// `n` <= 26 bits from bit `at` of p on, from the one or two aligned words that hold them
+__device__ __forceinline__ uint32_t bits_at(const uint8_t* p, uint32_t at, uint32_t n) {
+  const uint8_t* q = p + (at >> 3);
+  const uint32_t sh = (uint32_t)(uintptr_t)q & 3u, from = 8u * sh + (at & 7u);
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(q - sh);
+  uint64_t v = __ldg(w);
+  if (from + n > 32u) v |= (uint64_t)__ldg(w + 1) << 32;
+  return (uint32_t)(v >> from) & ((1u << n) - 1u);
 }
 
 }  // namespace
 
-__global__ void __launch_bounds__(1024, 2) k_dec_tokens(DecArgs A) {
+// A CTA of 512 threads per block, 2048 tokens a tile, four consecutive ones a thread (one load for their four bytes of
+// a stream, vector stores for their rows).  A tile is a chain of loads and barriers whatever its size: its streams'
+// bytes, the scan that places its ext bytes and offset bits, those, the scan that places its literals and output, and
+// the offsets that its recent-offset symbols name.  (One token a thread, groups and recent offsets in passes of their
+// own over the block's tokens in global memory: 0.49 ms per GiB of lz_mix at block 18 against 0.33, one text block 0.058
+// against 0.037.)
+//
+// Recent offsets (src/codec2.h:179-199): symbol r of a group whose first token is gs names the offset of token
+// gs - 1 - r (the last three offsets before the group, nearest first), or the initial 1, 4, 8 when r >= gs.  The group
+// counts' scan sets a bit for each group's first token; the maximum of those up to a token is its gs.  A token named
+// in an earlier tile is resolved; within the tile, by pointer jumping in shared memory (a chain halves each round).
+constexpr uint32_t kTokThreads = 512, kTokPer = 4, kTokTile = kTokThreads * kTokPer;
+
+__global__ void __launch_bounds__(kTokThreads, 2) k_dec_tokens(DecArgs A) {
+  constexpr uint32_t NW = kTokThreads / 32;
   const uint32_t b = blockIdx.x, tid = threadIdx.x;
   if (A.method[b] != 1 || A.raw_len[b] > A.B || A.err[b]) return;
-  __shared__ uint32_t ws[33];
-  __shared__ uint32_t any_bad;
+  __shared__ uint64_t sums[2][NW];
+  __shared__ uint32_t maxs[2][NW];
+  __shared__ uint32_t gbits[(1u << kMaxBlockLog) / 4 / 32 + 1];  // a bit for each group's first token
+  __shared__ __align__(16) uint32_t jump[kTokTile];
   const DecMeta m = A.meta[b];
   const uint32_t raw = A.raw_len[b], B = A.B;
   const size_t TC = tok_cap(B), EC = ext_cap(B);
-  const uint8_t* tok = A.s_tok + (size_t)b * TC;
-  const uint8_t* sym = A.s_sym + (size_t)b * TC;
-  const uint8_t* grp = A.s_grp + (size_t)b * TC;
+  const uint32_t* tok = reinterpret_cast<const uint32_t*>(A.s_tok + (size_t)b * TC);  // (four symbols a word)
+  const uint32_t* sym = reinterpret_cast<const uint32_t*>(A.s_sym + (size_t)b * TC);
+  const uint32_t* grp = reinterpret_cast<const uint32_t*>(A.s_grp + (size_t)b * TC);
   const uint8_t* ext = A.s_ext + (size_t)b * EC;
   const uint8_t* bits = A.comp + A.comp_off[b] + m.bits_off;
   const uint64_t nbits = 8ull * m.nob;
@@ -102,132 +127,142 @@ __global__ void __launch_bounds__(1024, 2) k_dec_tokens(DecArgs A) {
   uint32_t* Td = A.tk_d + (size_t)b * TC;
   uint2* line = A.line ? A.line + (size_t)b * line_cap(B) : nullptr;  // (none for one warp a block)
   const uint32_t al = (uint32_t)(uintptr_t)(A.out + A.out_off[b]) & 127u;  // output byte q lies in line (q + al) / 128
-  if (line)
-    for (uint32_t k = tid; k < (raw + al + 127u) >> 7; k += 1024) line[k] = make_uint2(0, 0);
-  if (tid == 0) any_bad = 0;
-  __syncthreads();
-  // ---- lengths, offsets and positions, 1024 tokens a tile
-  uint32_t ei = 0, bp = 0, op = 0, li = 0;
   bool bad = false;
-  for (uint32_t t0 = 0; t0 < m.nt; t0 += 1024) {
-    const uint32_t t = t0 + tid;
-    const bool on = t < m.nt;
-    const uint32_t tv = on ? tok[t] : 0u, sv = on ? sym[t] : 0u;
-    const uint32_t fl = on && (tv >> 4) == 15u, fm = on && (tv & 15u) == 15u;
-    const uint32_t nx = 3u * fl + 2u * fm;
-    const uint32_t nbit = (on && sv <= 19u) ? sv : 0u;
-    if (on && sv > 19u && (sv < kSymRep || sv > kSymRep + 2)) bad = true;
-    uint32_t tsum;
-    const uint32_t pre = cta_scan(nx | nbit << 16, ws, tsum);  // (each part of a tile's sum fits 16 bits)
-    const uint32_t xq = ei + (pre & 0xFFFFu), bq = bp + (pre >> 16);
-    ei += tsum & 0xFFFFu;
-    bp += tsum >> 16;
-    if (on && (uint64_t)xq + nx > m.ne) bad = true;
-    if (on && (uint64_t)bq + nbit > nbits) bad = true;
-    uint32_t L = tv >> 4, M = on ? (tv & 15u) + 4u : 0u;
-    if (!bad && fl) L += (uint32_t)ext[xq] | (uint32_t)ext[xq + 1] << 8 | (uint32_t)ext[xq + 2] << 16;
-    if (!bad && fm) { const uint32_t q = xq + 3u * fl; M += (uint32_t)ext[q] | (uint32_t)ext[q + 1] << 8; }
-    uint32_t D = 0;
-    if (on && !bad) {
-      if (sv >= kSymRep) {
-        D = kRepMark | (sv - kSymRep);
-      } else {
-        uint32_t x = 0;
-        if (nbit) {
-          const uint32_t j0 = bq >> 3, j1 = (bq + nbit - 1) >> 3;
-          uint64_t w = 0;
-          for (uint32_t j = j0; j <= j1; ++j) w |= (uint64_t)bits[j] << (8 * (j - j0));
-          x = (uint32_t)(w >> (bq & 7u)) & ((1u << nbit) - 1u);
-        }
-        D = (1u << sv) + x;
+  CtaScan<NW> scan(sums, maxs);
+  uint64_t sum;
+  if (line)
+    for (uint32_t k = tid; k < (raw + al + 127u) >> 7; k += kTokThreads) line[k] = make_uint2(0, 0);
+  for (uint32_t k = tid; k < (m.nt >> 5) + 1; k += kTokThreads) gbits[k] = 0;
+  __syncthreads();
+  // ---- the groups' first tokens
+  {
+    uint32_t at = 0;
+    for (uint32_t g0 = 0; g0 < m.ng; g0 += kTokTile) {
+      const uint32_t g = g0 + kTokPer * tid, c4 = g < m.ng ? grp[g >> 2] : 0u;
+      uint32_t c[kTokPer], mine = 0;
+#pragma unroll
+      for (uint32_t j = 0; j < kTokPer; ++j) {
+        c[j] = g + j < m.ng ? c4 >> 8 * j & 0xFFu : 0u;
+        mine += c[j];
       }
-    }
-    uint32_t lsum, osum;
-    const uint32_t lpre = cta_scan(L, ws, lsum);
-    const uint32_t opre = cta_scan(L + M, ws, osum);
-    const uint32_t opk = op + opre, lik = li + lpre;
-    if (on && ((uint64_t)lik + L > m.nl || (uint64_t)opk + L + M > raw)) bad = true;
-    if (on) { Tp[t] = tok_row(opk, L, lik); Td[t] = D; }
-    if (line && on && !bad) {  // the lines whose first byte the token holds, and its own start inside a line
-      for (uint32_t k = (opk + al + 127u) >> 7; k < (opk + L + M + al + 127u) >> 7; ++k) line[k].x = t;
-      if (t && ((opk + al) & 127u)) atomicOr(&line[(opk + al) >> 7].y, 1u << ((opk + al) >> 2 & 31u));
-    }
-    op += osum;
-    li += lsum;
-  }
-  if (bad) any_bad = 1;
-  __syncthreads();
-  if (tid == 0) { Tp[m.nt] = tok_row(op, raw - op, li); Td[m.nt] = 1; }  // token nt: the literal tail
-  if (line && !any_bad && op < raw) {  // the literal tail's lines and start (a line 0 that starts before the output: token 0)
-    for (uint32_t k = ((op + al + 127u) >> 7) + tid; k < (raw + al + 127u) >> 7; k += 1024) line[k].x = m.nt;
-    if (tid == 0 && op && ((op + al) & 127u)) atomicOr(&line[(op + al) >> 7].y, 1u << ((op + al) >> 2 & 31u));
-  }
-  // ---- groups and recent offsets (src/codec2.h:179-199).  A recent-offset symbol r of a group whose first
-  //      token is gs names the offset of token gs - 1 - r (the last three offsets before the group,
-  //      nearest first), or the initial 1, 4, 8 when r >= gs.  So: group starts (a scan of the group
-  //      counts) flag their first tokens; a max-scan gives each token its group's start; each recent-
-  //      offset token then points at the token it names, and pointer jumping resolves chains of them.
-  __syncthreads();
-  if (!any_bad) {
-    uint32_t gbase = 0;
-    for (uint32_t g0 = 0; g0 < m.ng; g0 += 1024) {
-      const uint32_t g = g0 + tid;
-      const uint32_t c = g < m.ng ? grp[g] : 0u;
-      uint32_t tot;
-      const uint32_t at = gbase + cta_scan(c, ws, tot);
-      if (g < m.ng && (c == 0 || (uint64_t)at + c > m.nt)) bad = true;
-      else if (g < m.ng) Td[at] |= kGrpStart;
-      gbase += tot;
-    }
-    if (gbase != m.nt) bad = true;
-  }
-  if (bad) any_bad = 1;
-  __syncthreads();
-  if (!any_bad) {
-    uint32_t carry = 0;
-    for (uint32_t t0 = 0; t0 < m.nt; t0 += 1024) {
-      const uint32_t t = t0 + tid;
-      const bool on = t < m.nt;
-      uint32_t v = on ? Td[t] : 0u;
-      uint32_t tmax;
-      const uint32_t gs = max(carry, cta_max_incl(on && (v & kGrpStart) ? t : 0u, ws, tmax));
-      carry = max(carry, tmax);
-      if (on) {
-        v &= ~kGrpStart;
-        if (v & kRepMark) {
-          const uint32_t r = v & 3u;
-          v = r < gs ? kRepMark | (gs - 1u - r) : (r - gs == 0 ? 1u : r - gs == 1 ? 4u : 8u);
+      uint32_t s = at + (uint32_t)scan(mine, sum);
+#pragma unroll
+      for (uint32_t j = 0; j < kTokPer; ++j) {
+        if (g + j < m.ng) {
+          if (c[j] == 0 || s + c[j] > m.nt) bad = true;  // (at most 2^20 counts of at most 255)
+          else atomicOr(&gbits[s >> 5], 1u << (s & 31u));
         }
-        Td[t] = v;
+        s += c[j];
       }
+      at += (uint32_t)sum;
     }
+    if (at != m.nt) bad = true;
   }
   __syncthreads();
-  if (!any_bad) {
-    for (int round = 0; round < 32; ++round) {  // (a chain halves each round: at most 20 for 2^20 tokens)
-      bool more = false;
-      for (uint32_t t = tid; t < m.nt; t += 1024) {
-        const uint32_t v = Td[t];
-        if (v & kRepMark) {
-          const uint32_t w = Td[v & ~kRepMark];
-          Td[t] = w;
-          more |= (w & kRepMark) != 0;
+  // ---- the tokens
+  uint32_t ei = 0, bp = 0, op = 0, li = 0, carry = 0;
+  uint32_t ntv = 0, nsv = 0;  // the next tile's tokens and symbols
+  if (kTokPer * tid < m.nt) { ntv = tok[tid]; nsv = sym[tid]; }
+  for (uint32_t t0 = 0; t0 < m.nt; t0 += kTokTile) {
+    const uint32_t t = t0 + kTokPer * tid;  // the thread's first token
+    const uint32_t n = t < m.nt ? min(kTokPer, m.nt - t) : 0u;
+    const uint32_t tv4 = ntv, sv4 = nsv;
+    ntv = 0; nsv = 0;
+    if (t + kTokTile < m.nt) { ntv = tok[(t + kTokTile) >> 2]; nsv = sym[(t + kTokTile) >> 2]; }
+    const uint32_t starts = n ? gbits[t >> 5] >> (t & 31u) & ((1u << n) - 1u) : 0u;
+    uint32_t mine = 0;  // ext bytes | offset bits << 16 of the thread (each part of a tile's sum fits 16 bits)
+#pragma unroll
+    for (uint32_t j = 0; j < kTokPer; ++j) {
+      if (j >= n) continue;
+      const uint32_t tv = tv4 >> 8 * j & 0xFFu, sv = sv4 >> 8 * j & 0xFFu;
+      if (sv > 19u && (sv < kSymRep || sv > kSymRep + 2)) bad = true;
+      mine += ((tv >> 4) == 15u ? 3u : 0u) + ((tv & 15u) == 15u ? 2u : 0u) + (sv <= 19u ? sv << 16 : 0u);
+    }
+    uint32_t gbefore, gall;
+    const uint32_t pre = (uint32_t)scan(mine, sum, starts ? t + 31u - __clz(starts) : 0u, gbefore, gall);
+    uint32_t xq = ei + (pre & 0xFFFFu), bq = bp + (pre >> 16);
+    ei += (uint32_t)sum & 0xFFFFu;
+    bp += (uint32_t)sum >> 16;
+    uint32_t L[kTokPer], M[kTokPer], D[kTokPer];
+    uint64_t len = 0;  // literals, and output << 32 (a sum past 32 bits only where a token is bad by itself)
+#pragma unroll
+    for (uint32_t j = 0; j < kTokPer; ++j) {
+      L[j] = 0; M[j] = 0; D[j] = 0;
+      if (j >= n) continue;
+      const uint32_t tv = tv4 >> 8 * j & 0xFFu, sv = sv4 >> 8 * j & 0xFFu;
+      const uint32_t fl = (tv >> 4) == 15u, fm = (tv & 15u) == 15u, nx = 3u * fl + 2u * fm, nbit = sv <= 19u ? sv : 0u;
+      if ((uint64_t)xq + nx > m.ne || (uint64_t)bq + nbit > nbits) bad = true;
+      L[j] = tv >> 4;
+      M[j] = (tv & 15u) + 4u;
+      if (!bad) {
+        if (fl) L[j] += (uint32_t)ext[xq] | (uint32_t)ext[xq + 1] << 8 | (uint32_t)ext[xq + 2] << 16;
+        if (fm) { const uint32_t q = xq + 3u * fl; M[j] += (uint32_t)ext[q] | (uint32_t)ext[q + 1] << 8; }
+        if (sv < kSymRep) {
+          D[j] = (1u << sv) + (nbit ? bits_at(bits, bq, nbit) : 0u);
+        } else {
+          const uint32_t own = starts & (2u << j) - 1u, r = sv - kSymRep;
+          const uint32_t gs = own ? t + 31u - __clz(own) : max(carry, gbefore);
+          D[j] = r < gs ? kRepMark | (gs - 1u - r) : r - gs == 0 ? 1u : r - gs == 1 ? 4u : 8u;
+          if (r < gs && gs - 1u - r < t0) D[j] = Td[gs - 1u - r];
         }
+      }
+      xq += nx;
+      bq += nbit;
+      len += (uint64_t)(L[j] + M[j]) << 32 | L[j];
+    }
+    carry = max(carry, gall);
+    *reinterpret_cast<uint4*>(&jump[kTokPer * tid]) = make_uint4(D[0], D[1], D[2], D[3]);
+    const uint64_t at = scan(len, sum);  // (its barrier also publishes jump)
+    uint32_t opk = op + (uint32_t)(at >> 32), lik = li + (uint32_t)at;
+    op += (uint32_t)(sum >> 32);
+    li += (uint32_t)sum;
+    uint2 row[kTokPer];
+    uint32_t ms[kTokPer];
+#pragma unroll
+    for (uint32_t j = 0; j < kTokPer; ++j) {
+      row[j] = tok_row(opk, L[j], lik);
+      ms[j] = opk + L[j];
+      if (j >= n) continue;
+      if ((uint64_t)lik + L[j] > m.nl || (uint64_t)opk + L[j] + M[j] > raw) bad = true;
+      const uint32_t end = opk + L[j] + M[j];
+      if (line && !bad) {  // the lines whose first byte the token holds, and its own start inside a line
+        for (uint32_t k = (opk + al + 127u) >> 7; k < (end + al + 127u) >> 7; ++k) line[k].x = t + j;
+        if (t + j && ((opk + al) & 127u)) atomicOr(&line[(opk + al) >> 7].y, 1u << ((opk + al) >> 2 & 31u));
+      }
+      opk = end;
+      lik += L[j];
+    }
+    for (;;) {  // (every thread has read jump before any writes it again)
+      uint32_t more = 0;
+#pragma unroll
+      for (uint32_t j = 0; j < kTokPer; ++j) {
+        if (D[j] & kRepMark) D[j] = jump[(D[j] & ~kRepMark) - t0];
+        more |= D[j] & kRepMark;
       }
       if (!__syncthreads_or(more)) break;
+      *reinterpret_cast<uint4*>(&jump[kTokPer * tid]) = make_uint4(D[0], D[1], D[2], D[3]);
+      __syncthreads();
     }
-    for (uint32_t t = tid; t < m.nt; t += 1024) {
-      const uint32_t D = Td[t];
-      const uint2 r = Tp[t];
-      if ((D & kRepMark) || D == 0 || D > row_start(r) + row_lits(r)) bad = true;
+    if (n) {
+#pragma unroll
+      for (uint32_t j = 0; j < kTokPer; ++j)
+        if (j < n && (D[j] == 0 || D[j] > ms[j])) bad = true;
+      *reinterpret_cast<uint4*>(Tp + t) = make_uint4(row[0].x, row[0].y, row[1].x, row[1].y);
+      *reinterpret_cast<uint4*>(Tp + t + 2) = make_uint4(row[2].x, row[2].y, row[3].x, row[3].y);
+      *reinterpret_cast<uint4*>(Td + t) = make_uint4(D[0], D[1], D[2], D[3]);
     }
-    if (bad) any_bad = 1;
   }
-  __syncthreads();
+  const int any_bad = __syncthreads_or(bad);
   if (tid == 0) {
+    Tp[m.nt] = tok_row(op, raw - op, li);  // token nt: the literal tail
+    Td[m.nt] = 1;
     if (any_bad || op + (m.nl - li) != raw) flag(A.err, b, E_TOKEN);
     A.meta[b].op_total = op;
     A.meta[b].li_total = li;
+  }
+  if (line && !any_bad && op < raw) {  // the literal tail's lines and start (a line 0 that starts before the output: token 0)
+    for (uint32_t k = ((op + al + 127u) >> 7) + tid; k < (raw + al + 127u) >> 7; k += kTokThreads) line[k].x = m.nt;
+    if (tid == 0 && op && ((op + al) & 127u)) atomicOr(&line[(op + al) >> 7].y, 1u << ((op + al) >> 2 & 31u));
   }
 }
 
@@ -704,7 +739,7 @@ void launch_decode_fill(const DecArgs& args, cudaStream_t st, Stages& S) {
   if (nw == 1) A.line = nullptr;
   launch_dec_streams(A, st, S);
   S.begin("k_dec_tokens", st);
-  k_dec_tokens<<<A.nb, 1024, 0, st>>>(A);
+  k_dec_tokens<<<A.nb, kTokThreads, 0, st>>>(A);
   S.end(st);
   cudaMemsetAsync(A.work, 0, sizeof(uint32_t), st);
   if (nw > 1) {
