@@ -1031,18 +1031,29 @@ __global__ void __launch_bounds__(64) k_enc_rans(EncArgs A) {
   }
   const uint8_t* sym = stream_syms(A, b, s);
   // per symbol: fc = freq | cum << 13 | (ceil(log2 freq) - 1) << 25, rcp = ceil(2^(31 + ceil(log2 freq)) / freq)
-  __shared__ uint32_t hist[256], fc[256], rcp[256], red[3];
+  __shared__ uint32_t hist[2][256], fc[256], rcp[256], red[3];
   __shared__ __align__(16) uint8_t stage[kRansChunk];
-  for (uint32_t i = k; i < 256; i += 64) hist[i] = 0;
+  for (uint32_t i = k; i < 512; i += 64) (&hist[0][0])[i] = 0;
   __syncthreads();
-  for (uint32_t i = k; i < ns; i += 64) atomicAdd(&hist[sym[i]], 1u);
+  {  // counts, a warp's in its own half: 16 symbols a load (a byte a load was half the kernel's time on long streams)
+    uint32_t* h = hist[k >> 5];
+    const uint32_t nv = ((uintptr_t)sym & 15u) == 0 ? ns >> 4 : 0u;
+#pragma unroll 4
+    for (uint32_t i = k; i < nv; i += 64) {
+      const uint4 v = reinterpret_cast<const uint4*>(sym)[i];
+      const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int j = 0; j < 16; ++j) atomicAdd(&h[u[j >> 2] >> (8 * (j & 3)) & 0xFFu], 1u);
+    }
+    for (uint32_t i = 16 * nv + k; i < ns; i += 64) atomicAdd(&h[sym[i]], 1u);
+  }
   __syncthreads();
   // normalisation (src/codec.h:41-66) by warp 0: lane l holds symbols 8l .. 8l+7
   if (k < 32) {
     uint32_t f[8], sum = 0, np = 0;
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-      const uint32_t c = hist[k * 8 + q];
+      const uint32_t c = hist[0][k * 8 + q] + hist[1][k * 8 + q];
       f[q] = c ? max(1u, (uint32_t)(((uint64_t)c << kScaleBits) / ns)) : 0u;
       sum += f[q];
       np += c != 0;
@@ -1109,19 +1120,28 @@ __global__ void __launch_bounds__(64) k_enc_rans(EncArgs A) {
   // first: the CTA stages a chunk in shared memory with coalesced loads, then lane k codes its symbols
   // c0 + k + 64 j of it, j descending -- the order of the whole-stream loop, without a global load on
   // the state's dependency chain.
-  const bool al4 = ((uintptr_t)sym & 3u) == 0;
-  for (int32_t ch = (int32_t)((ns - 1) / kRansChunk); ch >= 0; --ch) {
+  // (16-byte aligned streams: a chunk is loaded into registers while the one after it is coded)
+  constexpr int kVecs = kRansChunk / 16 / kLanes;
+  const bool al16 = ((uintptr_t)sym & 15u) == 0;
+  const int32_t last = (int32_t)((ns - 1) / kRansChunk);
+  uint4 ahead[kVecs];
+  for (int32_t ch = last; ch >= 0; --ch) {
     const uint32_t c0 = (uint32_t)ch * kRansChunk, cn = min(kRansChunk, ns - c0);
     __syncthreads();  // (the previous chunk is coded)
-    uint32_t t0 = 0;
-    if (al4) {
-      const uint32_t n4 = cn >> 2;
+    if (al16 && ch != last) {
+#pragma unroll
+      for (int j = 0; j < kVecs; ++j) reinterpret_cast<uint4*>(stage)[j * kLanes + k] = ahead[j];
+    } else {
+      const uint32_t n4 = ((uintptr_t)sym & 3u) == 0 ? cn >> 2 : 0u;
       for (uint32_t t = k; t < n4; t += kLanes)
         reinterpret_cast<uint32_t*>(stage)[t] = reinterpret_cast<const uint32_t*>(sym + c0)[t];
-      t0 = n4 << 2;
+      for (uint32_t t = 4 * n4 + k; t < cn; t += kLanes) stage[t] = sym[c0 + t];
     }
-    for (uint32_t t = t0 + k; t < cn; t += kLanes) stage[t] = sym[c0 + t];
     __syncthreads();
+    if (al16 && ch > 0) {
+#pragma unroll
+      for (int j = 0; j < kVecs; ++j) ahead[j] = reinterpret_cast<const uint4*>(sym + c0 - kRansChunk)[j * kLanes + k];
+    }
     if (k < cn) {
       // x' = (x / f) * 4096 + x % f + cum = x + cum + q * (4096 - f), with q = x / f by an exact
       // reciprocal: for x < 2^31 and s = ceil(log2 f), floor(x * ceil(2^(31+s) / f) / 2^(31+s)) = x / f
