@@ -683,6 +683,16 @@ __global__ void __launch_bounds__(32, 32) k_enc_walk(EncArgs A) {
   A.seg_exit[(size_t)b * A.nseg + q] = make_uint2(p, cnt);
 }
 
+// how many of a walk's n tokens lie before position c
+__device__ __forceinline__ uint32_t tk_after(const uint2* toks, uint32_t n, uint32_t c) {
+  uint32_t lo = 0;
+  while (lo < n) {
+    const uint32_t mid = (lo + n) >> 1;
+    if (tk_i(toks[mid]) < c) lo = mid + 1; else n = mid;
+  }
+  return lo;
+}
+
 // One CTA per block, a lane a segment.  Rounds re-walk each segment from where the chain before it leaves, until
 // that walk meets the previous one (a two-pointer merge), and end when no segment's exit moves.  Then every
 // segment's tokens are its first walk's (k_enc_walk) from where the walk from its true entry meets that one, after
@@ -705,6 +715,12 @@ __global__ void __launch_bounds__(T, 1024 / T) k_enc_parse(EncArgs A) {
   ent[q] = s;
   const uint2 first = A.seg_exit[(size_t)b * T + q];  // the first walk's exit, its tokens
   ex[q] = first.x;
+  // the segment's tokens: cnt of its own slots, then the first walk's from the from-th on
+  const uint32_t slots = S / 4 + 2;
+  const uint2* old = A.tk_seg + (size_t)b * 2 * seg_tok_cap(A.B) + (size_t)q * slots;
+  uint2* own = A.tk_seg + ((size_t)b * 2 + 1) * seg_tok_cap(A.B) + (size_t)q * slots;
+  uint32_t cnt = 0, from = 0;
+  bool again = false;  // the entry moved twice: the tokens are taken after the rounds
   // rounds: each segment re-walked from where the chain before it leaves, until it meets its old walk
   for (;;) {
     __syncthreads();
@@ -717,18 +733,26 @@ __global__ void __launch_bounds__(T, 1024 / T) k_enc_parse(EncArgs A) {
     int mode = 0;
     uint32_t a = want, c = old_ent, nx = old_ex;
     if (want != old_ent) {
+      again = old_ent != s;  // (its path was the first walk's: the tokens until the walks meet are taken here)
+      cnt = 0;
+      from = first.y;
       if (want >= e) nx = want;
       else mode = old_ent >= e ? 1 : 2;
     }
     while (__any_sync(kFull, mode != 0)) {
       const bool adv_a = mode == 1 || (mode == 2 && a < c);
       const uint32_t y = warp_step(P, W, adv_a ? a : c, e, mode != 0, t, ta, tc, td);
+      if (t && adv_a && !again) own[cnt++] = tk_pack(ta, tc, td);
       if (mode == 1) {
         a = y;
         if (a >= e) { nx = a; mode = 0; }
       } else if (mode == 2) {
         if (adv_a) a = y; else c = y;
-        if (a == c) { nx = old_ex; mode = 0; }
+        if (a == c) {
+          nx = old_ex;
+          mode = 0;
+          if (!again) from = tk_after(old, first.y, c);
+        }
         else if (a >= e && c >= e) { nx = a; mode = 0; }
       }
     }
@@ -738,14 +762,10 @@ __global__ void __launch_bounds__(T, 1024 / T) k_enc_parse(EncArgs A) {
     }
     if (!__syncthreads_or(changed)) break;
   }
-  const uint32_t slots = S / 4 + 2;
-  const uint2* old = A.tk_seg + (size_t)b * 2 * seg_tok_cap(A.B) + (size_t)q * slots;
-  uint2* own = A.tk_seg + ((size_t)b * 2 + 1) * seg_tok_cap(A.B) + (size_t)q * slots;
-  uint32_t cnt = 0, from = first.y;  // tokens before the walks meet, the first walk's from there on
   {
     uint32_t a = ent[q], c = s;
-    if (a == c) from = 0;
-    bool on = a != c && a < e;
+    if (again) { cnt = 0; from = a == c ? 0u : first.y; }
+    bool on = again && a != c && a < e;
     while (__any_sync(kFull, on)) {
       const bool adv_a = a < c;
       const uint32_t y = warp_step(P, W, adv_a ? a : c, e, on, t, ta, tc, td);
@@ -757,14 +777,7 @@ __global__ void __launch_bounds__(T, 1024 / T) k_enc_parse(EncArgs A) {
           c = y;
         }
         on = a != c && (a < e || c < e);
-        if (a == c) {  // the first walk's tokens from here on
-          uint32_t hi = from;
-          from = 0;
-          while (from < hi) {
-            const uint32_t mid = (from + hi) >> 1;
-            if (tk_i(old[mid]) < c) from = mid + 1; else hi = mid;
-          }
-        }
+        if (a == c) from = tk_after(old, first.y, c);
       }
     }
   }
