@@ -626,21 +626,25 @@ __device__ __forceinline__ uint32_t warp_step(const ParseBlock& P, Finish& W, ui
                                               bool& tok, uint32_t& ti, uint32_t& tm, uint32_t& td) {
   uint32_t v = M_NONE, v2 = M_NONE;
   if (act) {
+    // eight records at a time, from two aligned loads: the first that is not NONE ends the run (a load a record, or
+    // four, made a step wait for two to four times as many); its own and the next one's come from the L1 then
     const uint32_t* m = P.minfo;
-    v = m[p];
-    if (v == M_NONE) {
-      ++p;
-      while (p + 4 <= lim) {
-        const uint32_t q0 = m[p], q1 = m[p + 1], q2 = m[p + 2], q3 = m[p + 3];
-        if (q0 != M_NONE) break;
-        if (q1 != M_NONE) { p += 1; break; }
-        if (q2 != M_NONE) { p += 2; break; }
-        if (q3 != M_NONE) { p += 3; break; }
-        p += 4;
+    while (p < lim) {
+      const uint32_t at = p & ~3u;
+      const uint4 a = *reinterpret_cast<const uint4*>(m + at);
+      uint4 c = make_uint4(0, 0, 0, 0);
+      if (at + 4 < P.n) c = *reinterpret_cast<const uint4*>(m + at + 4);
+      uint32_t some = (a.x != M_NONE ? 1u : 0u) | (a.y != M_NONE ? 2u : 0u) | (a.z != M_NONE ? 4u : 0u) |
+                      (a.w != M_NONE ? 8u : 0u) | (c.x != M_NONE ? 16u : 0u) | (c.y != M_NONE ? 32u : 0u) |
+                      (c.z != M_NONE ? 64u : 0u) | (c.w != M_NONE ? 128u : 0u);
+      some >>= p & 3u;
+      if (some) {
+        p = min(p + (uint32_t)__ffs(some) - 1u, lim);
+        break;
       }
-      while (p < lim && m[p] == M_NONE) ++p;
-      if (p < lim) v = m[p];
+      p = min(at + 8, lim);
     }
+    if (p < lim) v = m[p];
     if (v != M_NONE && p + 1 < P.n) v2 = m[p + 1];
     if (m_is_below(v2)) v2 = M_NONE;  // (of no use to p's lazy test)
   }
