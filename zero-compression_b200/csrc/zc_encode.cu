@@ -160,24 +160,44 @@ __global__ void __launch_bounds__(256) k_sort_count(EncArgs A) {
   A.scnt[((size_t)b * sort_tiles(A.B) + t) * 256 + tid] = sum;
 }
 
-// per block: counts -> each tile's start per digit (digit-major order over the block's tiles)
-__global__ void __launch_bounds__(256) k_sort_scan(EncArgs A) {
-  const uint32_t b = blockIdx.x, d = threadIdx.x, lane = lane_id(), w = d >> 5;
-  __shared__ uint32_t ws[8];
-  const uint32_t T = sort_tiles(A.B);
-  uint32_t* c = A.scnt + (size_t)b * T * 256;
+// per block: counts -> each tile's start per digit (digit-major order over the block's tiles).  A thread a digit, or
+// kScanParts of them over more than 16 tiles, each with a run of tiles: sums of the runs, then the starts, four tiles'
+// counts in flight a thread.  (One thread a digit, a tile after the other: 0.42 ms per GiB for both passes at block
+// 18 against 0.23, 0.19 for 256 blocks of 1 MiB against 0.07; at 16 tiles 0.030 against 0.034 with four.)
+constexpr uint32_t kScanParts = 4;
+
+__global__ void __launch_bounds__(256 * kScanParts) k_sort_scan(EncArgs A) {
+  const uint32_t b = blockIdx.x, d = threadIdx.x & 255u, part = threadIdx.x >> 8, lane = lane_id();
+  __shared__ uint32_t sums[kScanParts][256], ws[8];
+  const uint32_t T = sort_tiles(A.B), parts = blockDim.x >> 8, per = (T + parts - 1) / parts;
+  const uint32_t t0 = min(part * per, T), t1 = min(t0 + per, T);
+  uint32_t* c = A.scnt + (size_t)b * T * 256 + d;
   uint32_t run = 0;
-  for (uint32_t t = 0; t < T; ++t) {
-    const uint32_t v = c[t * 256 + d];
-    c[t * 256 + d] = run;
-    run += v;
-  }
-  const uint32_t inc = warp_incl_scan(run);
-  if (lane == 31) ws[w] = inc;
+#pragma unroll 4
+  for (uint32_t t = t0; t < t1; ++t) run += c[t * 256];
+  sums[part][d] = run;
   __syncthreads();
-  uint32_t base = inc - run;
-  for (uint32_t k = 0; k < w; ++k) base += ws[k];
-  for (uint32_t t = 0; t < T; ++t) c[t * 256 + d] += base;
+  uint32_t before = 0, total = 0;  // of the digit: the tiles before this run, all tiles
+  for (uint32_t k = 0; k < parts; ++k) {
+    const uint32_t v = sums[k][d];
+    if (k < part) before += v;
+    total += v;
+  }
+  const uint32_t inc = warp_incl_scan(total);
+  if (part == 0 && lane == 31) ws[d >> 5] = inc;
+  __syncthreads();
+  uint32_t at = before + inc - total;
+  for (uint32_t k = 0; k < (d >> 5); ++k) at += ws[k];
+  for (uint32_t t = t0; t < t1; t += 4) {
+    uint32_t v[4];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) v[k] = t + k < t1 ? c[(t + k) * 256] : 0u;
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+      if (t + k < t1) c[(t + k) * 256] = at;
+      at += v[k];
+    }
+  }
 }
 
 template <int PASS>
@@ -1370,11 +1390,12 @@ void launch_encode(const EncArgs& A, const CrcArgs& crc_in, cudaStream_t st, Sta
   if (!A.nb) return;
   launch_crc(crc_in, st, S, "k_crc_in");
   const dim3 sg((A.B + kSortTile - 1) / kSortTile, A.nb);
+  const uint32_t scan_threads = sg.x > 16 ? 256 * kScanParts : 256;
   S.begin("k_sort_count", st);
   k_sort_count<0><<<sg, 256, 0, st>>>(A);
   S.end(st);
   S.begin("k_sort_scan", st);
-  k_sort_scan<<<A.nb, 256, 0, st>>>(A);
+  k_sort_scan<<<A.nb, scan_threads, 0, st>>>(A);
   S.end(st);
   S.begin("k_sort_scatter", st);
   k_sort_scatter<0><<<sg, kSortThreads, 0, st>>>(A);
@@ -1383,7 +1404,7 @@ void launch_encode(const EncArgs& A, const CrcArgs& crc_in, cudaStream_t st, Sta
   k_sort_count<1><<<sg, 256, 0, st>>>(A);
   S.end(st);
   S.begin("k_sort_scan", st);
-  k_sort_scan<<<A.nb, 256, 0, st>>>(A);
+  k_sort_scan<<<A.nb, scan_threads, 0, st>>>(A);
   S.end(st);
   S.begin("k_sort_scatter", st);
   k_sort_scatter<1><<<sg, kSortThreads, 0, st>>>(A);
