@@ -147,9 +147,11 @@ int zc_reserve(zc_ctx *ctx, uint32_t block_log, uint32_t nb);
  *   fill_ring_log   decoder fill: each warp keeps its last 2^fill_ring_log output bytes in shared memory
  *                   (11..15), so a match nearer than that reads shared instead of global memory
  *   fill_warps      decoder fill: blocks (warps) per CTA, 1, 2, 4 or 8; fill_warps * (2^fill_ring_log +
- *                   1408 * fill_words) bytes of shared memory per CTA, at most 227 KiB
+ *                   1536 * fill_words) bytes of shared memory per CTA, at most 227 KiB
  *   fill_words      decoder fill: output words each lane fills per round (1, 2 or 4: rounds of 128,
  *                   256 or 512 bytes, whose loads are in flight together)
+ *                   (the fill_* fields shape launches of more than 888 blocks: with fewer, several warps share
+ *                   a block in a form of its own)
  *   match_cap (8..32), match_tile (256, 512 or 1024), match_dense (0..1025), match_defer (0..4)
  *                   kept and checked, without effect: they shaped a match pass that compared every position's
  *                   candidates; the parse now computes matches where it needs them

@@ -40,7 +40,7 @@ def round_trip(codec, data, offs, lens, block_log):
     assert np.array_equal(raw, want)
 
 
-@pytest.mark.parametrize("nb", [1, 2, 296, 297, 592, 593, 1480, 1481])
+@pytest.mark.parametrize("nb", [1, 2, 296, 297, 592, 593, 888, 889, 1480, 1481])
 def test_block_counts(codec, nb):
     data = material(1 << 20, nb)
     r = np.random.default_rng(nb)
@@ -48,6 +48,23 @@ def test_block_counts(codec, nb):
     lens[:: 7] = r.integers(0, 140, lens[:: 7].size)
     offs = r.integers(0, data.size - 6000, nb).astype(np.uint64)
     round_trip(codec, data, offs, lens, 16)
+
+
+@pytest.mark.parametrize("words", [1, 2, 4])
+@pytest.mark.parametrize("ring_log,warps", [(11, 8), (13, 4), (15, 1)])
+def test_shapes_of_one_warp_a_block(codec, ring_log, warps, words):
+    """More blocks than the form with several warps a block takes, in each shape of the other one."""
+    default = codec.get_shape(16, 5)
+    codec.set_shape(16, 5, fill_ring_log=ring_log, fill_warps=warps, fill_words=words)
+    try:
+        data = material(1 << 20, 7)
+        r = np.random.default_rng(8)
+        lens = r.integers(0, 6000, 900).astype(np.uint32)
+        lens[:: 90] = 65536
+        offs = r.integers(0, data.size - 65536, 900).astype(np.uint64)
+        round_trip(codec, data, offs, lens, 16)
+    finally:
+        codec.set_shape(16, 5, **default)
 
 
 @pytest.mark.parametrize("block_log", [16, 18, 20])

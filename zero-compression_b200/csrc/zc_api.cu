@@ -220,7 +220,7 @@ int encode_device(zc_ctx* c, const uint8_t* d_in, const uint64_t* d_off, const u
 
 int decode_device(zc_ctx* c, const uint8_t* d_comp, const uint64_t* d_comp_offs, const uint32_t* d_comp_lens,
                   const uint8_t* d_methods, const uint32_t* d_raw_lens, uint32_t nb, uint32_t block_log, uint8_t* d_out,
-                  const uint64_t* d_out_offs, uint32_t* d_crcs, uint32_t* d_err, cudaStream_t st) {
+                  const uint64_t* d_out_offs, uint32_t* d_crcs, uint32_t* d_err, cudaStream_t st, bool shaped) {
   if (bad_block_log(block_log)) return fail(c, ZC_E_ARG, "block size must be 2^16 .. 2^20 bytes");
   if (int r = ensure_dec(c, std::max(nb, 1u), block_log)) return r;
   ZC_CUDA(cudaMemsetAsync(d_err, 0, (size_t)nb * 4, st));
@@ -229,7 +229,7 @@ int decode_device(zc_ctx* c, const uint8_t* d_comp, const uint64_t* d_comp_offs,
   A.nb = nb; A.B = 1u << block_log; A.out = d_out; A.out_off = d_out_offs; A.err = d_err;
   A.s_lit = c->d_lit.as<uint8_t>(); A.s_tok = c->d_tok.as<uint8_t>(); A.s_sym = c->d_sym.as<uint8_t>();
   A.s_grp = c->d_grp.as<uint8_t>(); A.s_ext = c->d_ext.as<uint8_t>(); A.meta = c->d_meta.as<zc::DecMeta>();
-  A.tk_pos = c->d_tkp.as<uint2>(); A.tk_d = c->d_tkd.as<uint32_t>(); A.line = c->d_line.as<uint2>();
+  A.tk_pos = c->d_tkp.as<uint2>(); A.tk_d = c->d_tkd.as<uint32_t>(); A.line = shaped ? nullptr : c->d_line.as<uint2>();
   const Shape& sh = c->shape[block_log - zc::kMinBlockLog][level_class(c->level)];
   A.ring_log = sh.ring_log; A.fill_warps = sh.fill_warps; A.fill_words = sh.fill_words;
   A.work = c->work.as<uint32_t>() + 1;
@@ -626,8 +626,8 @@ int zc_set_shape(zc_ctx* c, uint32_t block_log, int level, const zc_shape* in) {
   return ZC_OK;
 }
 
-// Times every candidate shape of the fill on the sample (whole blocks of it, up to one encoder launch) and
-// keeps the fastest for (block_log, level).  Each candidate runs once untimed and then `reps` times; its time
+// Times every candidate shape of the fill on the sample (whole blocks of it, up to one encoder launch; in the shaped
+// form even where the sample has few blocks) and keeps the fastest for (block_log, level).  Each candidate runs once untimed and then `reps` times; its time
 // is the smallest.
 int zc_autotune(zc_ctx* c, const uint8_t* sample, size_t n, uint32_t block_log, int level, zc_shape* chosen) {
   if (!c || (!sample && n)) return ZC_E_ARG;
@@ -692,7 +692,8 @@ int zc_autotune(zc_ctx* c, const uint8_t* sample, size_t n, uint32_t block_log, 
                          d_coff, d_tot, 1, st);
   };
   auto decode = [&]() {
-    return decode_device(c, d_comp, d_coff, d_clen, d_meth, d_ilen, nb, block_log, d_raw, d_ioff, nullptr, d_err, st);
+    return decode_device(c, d_comp, d_coff, d_clen, d_meth, d_ilen, nb, block_log, d_raw, d_ioff, nullptr, d_err, st,
+                         true);
   };
   do {
     cudaError_t e = cudaEventCreate(&e0);

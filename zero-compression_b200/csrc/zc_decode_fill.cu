@@ -8,12 +8,13 @@
 //                 decoder is made here; a failing one records a status and the block is not replayed.
 //   k_dec_fill    one warp per block: fills the block in rounds of 128 output bytes (a 4-byte word a lane)
 //                 straight through, group boundaries or not: a byte whose source lies earlier in the same
-//                 round is passed along by shuffles once known; the token table is a 64-row ring in shared
-//                 memory, refilled 32 tokens at a time from registers loaded one window ahead.
+//                 round is read from the round's staged bytes once known; the token table is a 64-row ring in
+//                 shared memory, refilled 32 tokens at a time from registers loaded one window ahead.
 //   k_dec_fill_multi  the same with several warps a block, a line each, for launches of few blocks: words wait for
 //                 their source words, which are published in shared memory.
 // Stored blocks are copied by the fill.  The rANS streams come from k_dec_streams (zc_decode.cu).
 #include <algorithm>
+#include <type_traits>
 
 #include "zc_internal.cuh"
 #include "zc_kernels.h"
@@ -271,17 +272,18 @@ namespace {
 // The warp's token table: a ring of TR rows, token t in row t % TR.  start = the token's output start;
 // tk = {match start, literal start - output start (mod 2^32), offset D, the reciprocal ceil(2^32 / D)
 // for D >= 2 (0 for D = 1)}.  Token nt (one past the last) is the block's literal tail: it starts where
-// the tokens' output ends and is literals up to the block's end; later rows start at 0xFFFFFFFF.
+// the tokens' output ends and is literals up to the block's end; later rows start at kNoToken.
+constexpr uint32_t kNoToken = 0x7FFFFFFFu;
 template <uint32_t TR>
 struct FillTable {
   uint32_t start[TR];
   uint4 tk[TR];
 };
 // per warp, for WPL output words a lane a round: the table's rows (a round's tokens and the one carried
-// in), its bytes, and the round's byte flags (which bytes are not known yet)
+// in), its bytes, and the round's staged bytes
 __host__ __device__ constexpr uint32_t fill_rows(uint32_t wpl) { return 64 * wpl; }
 __host__ __device__ constexpr uint32_t fill_table_bytes(uint32_t wpl) { return 20 * fill_rows(wpl); }
-__host__ __device__ constexpr uint32_t fill_flag_bytes(uint32_t wpl) { return 128 * wpl; }
+__host__ __device__ constexpr uint32_t fill_stage_bytes(uint32_t wpl) { return 256 * wpl; }
 
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
@@ -306,8 +308,13 @@ __device__ inline void copy_bytes(uint8_t* d, const uint8_t* s, uint32_t n, uint
 // comes from its token's literals, from output before the round (the warp's shared-memory ring of the last
 // R bytes, or global memory), or from an earlier byte of the same round.  The lanes first fill every byte
 // of the first two kinds with their loads in flight together; the bytes of the third kind then read their
-// sources from the round's words staged in the ring, pass after pass until all are known (each source lies
+// sources from the round's bytes, staged 16 bits each, pass after pass until all are known (each source lies
 // before its byte, so this ends; the format's groups keep those chains short).
+//
+// Bound by instruction issue, so the work of a byte is kept short: a round that lies wholly inside the block tests no
+// bounds, ring loads are apart from loads of literals and far output (one generic load made the ring's slower), a
+// byte's source stays as it was computed, and a staged byte carries its own flag.  lz_mix, 1 GiB, block 18: 3.69 ms
+// with packed sources, bounds, generic loads and a flag array; 2.85 ms now.
 //
 // A token is at least 4 bytes long, so an aligned word holds at most one token start: a line's token
 // starts form a 32-bit word mask (one OR-reduction), and a lane's bytes belong to the last token starting at
@@ -316,7 +323,7 @@ __device__ inline void copy_bytes(uint8_t* d, const uint8_t* s, uint32_t n, uint
 // multiply-high by the reciprocal, exact to one step, which a compare corrects.
 template <uint32_t WPL, uint32_t TR>
 __device__ __forceinline__ void fill_block(const DecArgs& A, uint32_t b, FillTable<TR>& T, uint8_t* ring,
-                                           uint8_t* flags) {
+                                           uint16_t* stage) {
   const uint32_t R = 1u << A.ring_log, rmask = R - 1u;
   const uint32_t lane = lane_id();
   const uint32_t raw = A.raw_len[b], method = A.method[b], clen = A.comp_len[b], B = A.B;
@@ -344,7 +351,7 @@ __device__ __forceinline__ void fill_block(const DecArgs& A, uint32_t b, FillTab
   uint32_t loaded = 0, ns, nm, nd, nl;
   auto fetch = [&](uint32_t base) {
     const uint32_t t = base + lane;
-    ns = 0xFFFFFFFFu; nm = 0xFFFFFFFFu; nd = 1; nl = 0;
+    ns = kNoToken; nm = kNoToken; nd = 1; nl = 0;
     if (t < nt) {
       const uint2 r = Tp[t];
       nd = Td[t];
@@ -378,58 +385,61 @@ __device__ __forceinline__ void fill_block(const DecArgs& A, uint32_t b, FillTab
     }
     const int32_t rlo = lb - (int32_t)R;  // the ring holds output [lb - R, lb)
     uint32_t w[WPL], pend = 0;            // pend: bit 4h + j, byte j of word h is not known yet
-    uint64_t srcs[WPL];                   // its source's offset in the round, 16 bits a byte
+    uint32_t srcs[WPL][4];                // its source
     uint32_t bh = before;
 #pragma unroll
     for (uint32_t h = 0; h < WPL; ++h) {
       const int32_t lh = lb + 128 * (int32_t)h;
       const uint32_t ts = T.start[(bh + lane) % TR];
       const int32_t rel = (int32_t)(ts - (uint32_t)lh);
-      const uint32_t mask = __reduce_or_sync(kFull, ts != 0xFFFFFFFFu && rel >= 0 && rel < 128 ? 1u << (rel >> 2) : 0u);
+      const uint32_t mask = __reduce_or_sync(kFull, (uint32_t)rel < 128u ? 1u << (rel >> 2) : 0u);
       const uint32_t t1 = bh + __popc(mask & upto) - 1u, t0 = t1 - 1u;  // (mod 2^32: token -1 is row TR - 1)
       const uint32_t st1 = T.start[t1 % TR], st0 = T.start[t0 % TR];
       const uint4 a1 = T.tk[t1 % TR], a0 = T.tk[t0 % TR];
       bh += __popc(mask);
       const int32_t q0 = lh + 4 * (int32_t)lane;
       w[h] = 0;
-      srcs[h] = 0;
+      auto bytes = [&](auto whole) {
+        constexpr bool inside = decltype(whole)::value;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {  // every choice a select, the load predicated
-        const int32_t qi = q0 + j;
-        const bool valid = qi >= 0 && qi < (int32_t)raw;
-        const uint32_t q = (uint32_t)qi;
-        const bool hi = q >= st1;
-        const uint32_t opk = hi ? st1 : st0, ms = hi ? a1.x : a0.x, ld = hi ? a1.y : a0.y, D = hi ? a1.z : a0.z,
-                       mg = hi ? a1.w : a0.w;
-        const uint32_t x = q - ms;
-        uint32_t r = x - __umulhi(x, mg) * D;
-        r = (int32_t)r < 0 ? r + D : r;
-        r = mg ? r : 0u;
-        const uint32_t s = q >= ms ? ms - D + r : q;
-        const bool own = s >= opk;
-        const bool inr = !own && (int32_t)s >= lb;
-        const uint8_t* src = own ? lit + (s + ld) : (int32_t)s >= rlo ? ring + ((ob + s) & rmask) : o + s;
-        const bool take = valid && inr;
-        pend |= (uint32_t)take << (4 * h + j);
-        srcs[h] |= take ? (uint64_t)(s - (uint32_t)lb) << (16 * j) : 0ull;
-        uint32_t v = 0;
-        if (valid && !inr) v = *src;
-        w[h] |= v << (8 * j);
-      }
+        for (int j = 0; j < 4; ++j) {  // every choice a select, the load predicated
+          const int32_t qi = q0 + j;
+          const bool valid = inside || (qi >= 0 && qi < (int32_t)raw);
+          const uint32_t q = (uint32_t)qi;
+          const bool hi = q >= st1;
+          const uint32_t opk = hi ? st1 : st0, ms = hi ? a1.x : a0.x, ld = hi ? a1.y : a0.y, D = hi ? a1.z : a0.z,
+                         mg = hi ? a1.w : a0.w;
+          const uint32_t x = q - ms;
+          uint32_t r = x - __umulhi(x, mg) * D;
+          r = (int32_t)r < 0 ? r + D : r;
+          r = mg ? r : 0u;
+          const uint32_t s = q >= ms ? ms - D + r : q;
+          const bool own = s >= opk;
+          const bool inr = !own && (int32_t)s >= lb;
+          const bool near = !own && (int32_t)s >= rlo;
+          const uint8_t* src = (own ? lit : o) + (own ? s + ld : s);
+          const bool take = valid && inr;
+          pend |= (uint32_t)take << (4 * h + j);
+          srcs[h][j] = s;
+          uint32_t v = 0;
+          if (valid && !near) v = *src;
+          if (valid && near && !inr) v = ring[(ob + s) & rmask];
+          w[h] |= v << (8 * j);
+        }
+      };
+      if (lh >= 0 && lh + 128 <= (int32_t)raw) bytes(std::true_type{}); else bytes(std::false_type{});
     }
-    // bytes from earlier in the round: the round's words staged in their ring slots (the ring's older
-    // bytes there are no longer needed: every load from the ring was made above), with a flag per byte
-    // still unknown; each pass takes the bytes whose sources are known
+    // bytes from earlier in the round: the round's bytes staged, 16 bits each, bit 8 set while one is not known; each
+    // pass takes the bytes whose sources are known
     __syncwarp();  // (every lane's loads from the ring come before any lane's stores into it)
     if (__any_sync(kFull, pend)) {
       for (;;) {
 #pragma unroll
         for (uint32_t h = 0; h < WPL; ++h) {
-          const uint32_t q0 = (uint32_t)(lb + 128 * (int32_t)h + 4 * (int32_t)lane);
-          *reinterpret_cast<uint32_t*>(ring + ((ob + q0) & rmask)) = w[h];
-          const uint32_t f = (pend >> (4 * h)) & 15u;
-          *reinterpret_cast<uint32_t*>(flags + 128 * h + 4 * lane) =
-              (f & 1u) | (f & 2u) << 7 | (f & 4u) << 14 | (f & 8u) << 21;
+          const uint32_t f = (pend >> (4 * h)) & 15u;  // (bits 0, 1 to bits 8, 24, then bits 2, 3)
+          const uint32_t lo = __byte_perm(w[h], 0, 0x4140) | ((f & 3u) * 0x00800100u & 0x01000100u);
+          const uint32_t hi = __byte_perm(w[h], 0, 0x4342) | ((f >> 2) * 0x00800100u & 0x01000100u);
+          *reinterpret_cast<uint2*>(stage + 128 * h + 4 * lane) = make_uint2(lo, hi);
         }
         __syncwarp();
         uint32_t left = pend;
@@ -438,9 +448,9 @@ __device__ __forceinline__ void fill_block(const DecArgs& A, uint32_t b, FillTab
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             if (!((pend >> (4 * h + j)) & 1u)) continue;
-            const uint32_t sp = (uint32_t)(srcs[h] >> (16 * j)) & 0xFFFFu;
-            if (flags[sp]) continue;
-            w[h] |= (uint32_t)ring[(ob + (uint32_t)lb + sp) & rmask] << (8 * j);
+            const uint32_t c = stage[srcs[h][j] - (uint32_t)lb];
+            if (c >> 8) continue;
+            w[h] |= c << (8 * j);
             left &= ~(1u << (4 * h + j));
           }
         }
@@ -469,7 +479,7 @@ __device__ __forceinline__ void fill_block(const DecArgs& A, uint32_t b, FillTab
 
 // Fed by a device work queue: every warp takes the next block from the work counter until none is left,
 // so blocks of uneven sizes (a batch of many files) balance across warps.  A CTA holds blockDim.x / 32
-// warps, each with its table, a ring of 2^ring_log bytes and its byte flags in dynamic shared memory.
+// warps, each with its table, a ring of 2^ring_log bytes and its staged bytes in dynamic shared memory.
 // The ring is read only at positions the warp has written in its current block.
 template <uint32_t WPL>
 __global__ void __maxnreg__(72) k_dec_fill(DecArgs A) {  // (72 registers: 28 warps an SM with 4-warp CTAs)
@@ -477,24 +487,24 @@ __global__ void __maxnreg__(72) k_dec_fill(DecArgs A) {  // (72 registers: 28 wa
   extern __shared__ __align__(16) uint8_t fsm[];
   const uint32_t R = 1u << A.ring_log;
   const uint32_t wid = threadIdx.x >> 5;
-  const size_t per = (size_t)fill_table_bytes(WPL) + R + fill_flag_bytes(WPL);
+  const size_t per = (size_t)fill_table_bytes(WPL) + R + fill_stage_bytes(WPL);
   uint8_t* mine = fsm + (size_t)wid * per;
   FillTable<TR>& T = *reinterpret_cast<FillTable<TR>*>(mine);
   uint8_t* ring = mine + fill_table_bytes(WPL);
-  uint8_t* flags = ring + R;
+  uint16_t* stage = reinterpret_cast<uint16_t*>(ring + R);
   for (;;) {
     uint32_t b = 0;
     if (lane_id() == 0) b = atomicAdd(A.work, 1u);
     b = __shfl_sync(kFull, b, 0);
     if (b >= A.nb) break;
-    fill_block<WPL>(A, b, T, ring, flags);
+    fill_block<WPL>(A, b, T, ring, stage);
     __syncwarp();
   }
 }
 
 // ---- several warps a block
 // With fewer blocks than the GPU has room for warps, one warp a block leaves it idle and takes a block's 2^block_log
-// / 128 rounds one after the other (about 0.8 us each: 1.6 ms for 256 KiB).  Here the CTA's NW warps share a block:
+// / 128 rounds one after the other (about 0.55 us each: 1.1 ms for 256 KiB).  Here the CTA's NW warps share a block:
 // warp w fills the 128-byte lines w, w + NW, ..., each looked up by itself in the token table (DecArgs.line gives
 // the token that holds a line's first byte).  A word's bytes from literals and from lines that are complete are
 // loaded at once; the others wait for their source words.  state[v] is the line that warp v is at, with a bit for
@@ -618,21 +628,25 @@ __global__ void __launch_bounds__(32 * kMultiWarps, 2) k_dec_fill_multi(DecArgs 
         }
       }
       const int32_t lows = (int32_t)(low << 7) - (int32_t)a;  // the first output byte that may not be there
+      auto bytes = [&](auto whole) {  // (a line inside the block needs no bounds)
+        constexpr bool inside = decltype(whole)::value;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int32_t qi = q0 + j;
-        const bool valid = qi >= 0 && qi < (int32_t)raw;
-        const bool hi = (uint32_t)qi >= st1;
-        const bool own = s[j] >= (hi ? st1 : st0);
-        const bool later = !own && (int32_t)s[j] >= lows;
-        const bool near = !own && (int32_t)s[j] >= rlo;
-        wait |= (uint32_t)(valid && later) << j;
-        v[j] = 0;
-        const uint8_t* from = own ? lit : o;
-        const uint32_t off = own ? s[j] - (hi ? bk1 : bk0) : s[j];
-        if (valid && !near) v[j] = from[off];
-        if (valid && near && !later) v[j] = ring[(s[j] + a) & rmask];
-      }
+        for (int j = 0; j < 4; ++j) {
+          const int32_t qi = q0 + j;
+          const bool valid = inside || (qi >= 0 && qi < (int32_t)raw);
+          const bool hi = (uint32_t)qi >= st1;
+          const bool own = s[j] >= (hi ? st1 : st0);
+          const bool later = !own && (int32_t)s[j] >= lows;
+          const bool near = !own && (int32_t)s[j] >= rlo;
+          wait |= (uint32_t)(valid && later) << j;
+          v[j] = 0;
+          const uint8_t* from = own ? lit : o;
+          const uint32_t off = own ? s[j] - (hi ? bk1 : bk0) : s[j];
+          if (valid && !near) v[j] = from[off];
+          if (valid && near && !later) v[j] = ring[(s[j] + a) & rmask];
+        }
+      };
+      if (lb >= 0 && lb + 128 <= (int32_t)raw) bytes(std::true_type{}); else bytes(std::false_type{});
       uint32_t word = v[0] | v[1] << 8 | v[2] << 16 | v[3] << 24;
       uint32_t* const slot = reinterpret_cast<uint32_t*>(ring + (((ln << 7) + 4 * lane) & rmask));
       if (!wait) *slot = word;
@@ -713,7 +727,7 @@ __global__ void __launch_bounds__(32 * kMultiWarps, 2) k_dec_fill_multi(DecArgs 
 }
 
 size_t fill_smem_bytes(uint32_t ring_log, uint32_t warps, uint32_t words) {
-  return (size_t)warps * (fill_table_bytes(words) + (1u << ring_log) + fill_flag_bytes(words));
+  return (size_t)warps * (fill_table_bytes(words) + (1u << ring_log) + fill_stage_bytes(words));
 }
 
 cudaError_t prepare_fill() {
@@ -729,12 +743,13 @@ constexpr uint32_t kFillSms = 148;
 void launch_decode_fill(const DecArgs& args, cudaStream_t st, Stages& S) {
   DecArgs A = args;
   if (!A.nb) return;
-  // A warp a block once ten blocks an SM keep it busy, else 4 to kMultiWarps warps a block, as many as the GPU holds
-  // (32 an SM).  lz_mix, block 18, ms with 1 / 4 / 8 / 16 warps: 256 blocks 1.99 / 0.75 / 0.56 / 0.52, 1024 blocks
-  // 2.18 / 1.62 / 1.73 / 1.66, 1600 blocks 2.35 / 2.37 / 2.46 / 2.61, 4096 blocks 3.70 / 5.57 / 6.19 / 6.54: sharing
-  // a block costs about 130 more warp instructions a line (366), so it pays while warps are few.
+  // A warp a block beyond six blocks an SM, else 4 to kMultiWarps warps a block, as many as the GPU holds (32 an SM).
+  // Block 18, ms with 1 / 4 / 8 / 16 warps, lz_mix: 256 blocks 1.16 / 0.76 / 0.56 / 0.51, 1024 blocks 1.41 / 1.57 /
+  // 1.55 / 1.65, 1600 blocks 1.63 / 2.27 / 2.55 / 2.56; block 16, 768 blocks: lz_mix 0.34 / 0.36 / 0.35 / 0.38, text
+  // 0.43 / 0.34 / 0.35 / 0.43; 1200 blocks: text 0.49 / 0.47 / 0.52 / 0.63.  Sharing a block costs waits on its
+  // source words, so it pays while warps are few: the line lies where lz_mix loses as little as text gains.
   uint32_t nw = 1;
-  if (A.nb <= kFillSms * 10)
+  if (A.line && A.nb <= kFillSms * 6)
     for (nw = 4; nw < kMultiWarps && 2 * nw * A.nb <= kFillSms * 32;) nw *= 2;
   if (nw == 1) A.line = nullptr;
   launch_dec_streams(A, st, S);

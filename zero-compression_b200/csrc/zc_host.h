@@ -139,9 +139,10 @@ int encode_device(zc_ctx* c, const uint8_t* d_in, const uint64_t* d_off, const u
                   uint8_t* d_out, size_t out_cap, uint64_t* d_out_offs, uint64_t* d_total, int emit_stored,
                   cudaStream_t st, const uint64_t* rec_base = nullptr);
 // the decoder over nb device-resident blocks; d_crcs (may be NULL) gets each output's CRC-32
+// (`shaped`: the fill in its form of one warp a block, whatever the block count)
 int decode_device(zc_ctx* c, const uint8_t* d_comp, const uint64_t* d_comp_offs, const uint32_t* d_comp_lens,
                   const uint8_t* d_methods, const uint32_t* d_raw_lens, uint32_t nb, uint32_t block_log, uint8_t* d_out,
-                  const uint64_t* d_out_offs, uint32_t* d_crcs, uint32_t* d_err, cudaStream_t st);
+                  const uint64_t* d_out_offs, uint32_t* d_crcs, uint32_t* d_err, cudaStream_t st, bool shaped = false);
 
 }  // namespace zch
 
