@@ -87,3 +87,24 @@ def test_segment_counts(codec, level):
     assert m.all()
     for b in range(total):
         assert out[int(at[b]): int(at[b]) + int(n[b])].tobytes() == small[b % nb], f"block {b}"
+
+
+def test_walks_a_warp(codec):
+    """Launches whose warps take 2, 4, 8, 16 and 32 walks each give the same blocks the same payloads, which are the
+    CPU codec's."""
+    import datagen as G
+    import oracle as O
+    block_log, B = 16, 1 << 16
+    data = np.concatenate([G.text_mix(256 * B, 1), G.lz_mix(256 * B, block_log, 2)])[::-1].copy()
+    want = {}
+    for nb in (1, 32, 64, 128, 256, 512):  # (256 walks a block; 4736 warps at most, or 2 walks a warp)
+        m, n, _, p, o = codec.compress_arrays(data[: nb * B], block_log, level=5)
+        for b in range(nb):
+            got = p[int(o[b]): int(o[b]) + int(n[b])].tobytes() if m[b] else None
+            if b not in want:
+                want[b] = got
+                if b in (0, 31, 300):
+                    blk = data[b * B:(b + 1) * B].tobytes()
+                    ref = O.Port.compress_block(blk, O.depth_for_level(5))
+                    assert got == (ref if len(ref) < len(blk) else None)
+            assert got == want[b], (nb, b)

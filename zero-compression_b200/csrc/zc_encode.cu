@@ -683,13 +683,16 @@ __device__ __forceinline__ uint32_t warp_step(const ParseBlock& P, Finish& W, ui
 
 // The parse is a chain 0 -> next(0) -> ... cut into A.nseg segments of each block.  Every segment's walk from its
 // own start, a lane a walk: it leaves the exact records of the positions that it visits in minfo, its tokens in the
-// segment's slots, and where it leaves the segment, with the count, in seg_exit.  A warp, a CTA of its own, takes 32
-// consecutive segments; no warp waits for another, so a launch of few blocks spreads over the whole GPU.  (Two or
-// four segments a lane, handed out as lanes got done, kept more lanes busy, but the fewer warps took longer: 10.5,
-// 10.8, 11.5 ms for 1 GiB of lz_mix in 512-byte segments.)
-__global__ void __launch_bounds__(32, 32) k_enc_walk(EncArgs A) {
+// segment's slots, and where it leaves the segment, with the count, in seg_exit.  A warp, a CTA of its own, takes `walks`
+// (2 to 32) consecutive segments, its other lanes helping to finish records; no warp waits for another, so a launch
+// of few blocks spreads over the whole GPU.  (Two or four segments a lane, handed out as lanes got done, kept more
+// lanes busy, but the fewer warps took longer: 10.5, 10.8, 11.5 ms for 1 GiB of lz_mix in 512-byte segments.)
+// Text in 512-byte segments is bound by L2 misses: 32 warps an SM are then in 296 blocks' candidate orders, 1.25 MiB
+// each, 103 bytes read from memory a byte of input; lz_mix has few candidates and does not mind.
+__global__ void __launch_bounds__(32, 32) k_enc_walk(EncArgs A, uint32_t walks) {
   __shared__ Finish W;
-  const uint32_t per = A.nseg / 32, b = blockIdx.x / per, q = blockIdx.x % per * 32 + lane_id();
+  const uint32_t per = A.nseg / walks, b = blockIdx.x / per, q = blockIdx.x % per * walks + lane_id();
+  const bool mine = lane_id() < walks;
   const uint32_t n = A.in_len[b];
   const size_t so = (size_t)b * A.B;
   ParseBlock P;
@@ -697,14 +700,14 @@ __global__ void __launch_bounds__(32, 32) k_enc_walk(EncArgs A) {
   P.minfo = A.minfo + so; P.srt = A.srt + so;
   const uint32_t S = seg_bytes(n, A.nseg), slots = S / 4 + 2;  // (a token takes at least 4 bytes: S / 4 + 1 at most)
   uint2* toks = A.tk_seg + (size_t)b * 2 * seg_tok_cap(A.B) + (size_t)q * slots;
-  uint32_t p = min(q * S, n), cnt = 0;
+  uint32_t p = mine ? min(q * S, n) : n, cnt = 0;
   const uint32_t e = min(p + S, n);
   bool t; uint32_t ta, tc, td;
   while (__any_sync(kFull, p < e)) {
     p = warp_step(P, W, p, e, p < e, t, ta, tc, td);
     if (t) toks[cnt++] = tk_pack(ta, tc, td);
   }
-  A.seg_exit[(size_t)b * A.nseg + q] = make_uint2(p, cnt);
+  if (mine) A.seg_exit[(size_t)b * A.nseg + q] = make_uint2(p, cnt);
 }
 
 // how many of a walk's n tokens lie before position c
@@ -809,13 +812,26 @@ __global__ void __launch_bounds__(T, 1024 / T) k_enc_parse(EncArgs A) {
   const uint32_t incl = warp_incl_scan(cnt + rest);
   if (lane_id() == 31) wsum[q >> 5] = incl;
   __syncthreads();
-  uint32_t off = incl - cnt - rest;
-  for (uint32_t k = 0; k < (q >> 5); ++k) off += wsum[k];
+  // the warp's 32 segments' tokens lie one after another in the list: a lane a token, whose segment is the first with
+  // a higher inclusive count
+  uint32_t off = warp_sum(lane_id() < (q >> 5) ? wsum[lane_id()] : 0u);
   uint2* to = A.tk + (size_t)b * tok_cap(A.B) + off;
-  for (uint32_t k = 0; k < cnt; ++k) to[k] = own[k];
+  const uint32_t all = __shfl_sync(kFull, incl, 31);
+  const uint2* own0 = own - (size_t)lane_id() * slots;
+  const uint2* old0 = old - (size_t)lane_id() * slots;
 #pragma unroll 4
-  for (uint32_t k = 0; k < rest; ++k) to[cnt + k] = old[from + k];
-  if (q == T - 1) A.bcnt[b * 8 + 0] = off + cnt + rest;
+  for (uint32_t k0 = 0; k0 < all; k0 += 32) {
+    const uint32_t k = k0 + lane_id();
+    uint32_t l = 0;
+#pragma unroll
+    for (uint32_t h = 16; h; h >>= 1) l += __shfl_sync(kFull, incl, l + h - 1) <= k ? h : 0u;
+    const uint32_t before = __shfl_sync(kFull, incl, l ? l - 1 : 0u), mine = __shfl_sync(kFull, cnt, l),
+                   skip = __shfl_sync(kFull, from, l);
+    const uint32_t j = k - (l ? before : 0u);
+    const uint2* src = j < mine ? own0 + j : old0 + skip + (j - mine);
+    if (k < all) to[k] = src[(size_t)l * slots];
+  }
+  if (q == T - 1) A.bcnt[b * 8 + 0] = off + all;
 }
 
 // ---------------------------------------------------------------- 4. tokens -> streams
@@ -1413,7 +1429,13 @@ void launch_encode(const EncArgs& A, const CrcArgs& crc_in, cudaStream_t st, Sta
   k_enc_chain<<<dim3((A.B + kChainTile - 1) / kChainTile, A.nb), 256, 0, st>>>(A);
   S.end(st);
   S.begin("k_enc_walk", st);
-  k_enc_walk<<<A.nb * (A.nseg / 32), 32, 0, st>>>(A);
+  // Walks a warp: 32, or fewer while the launch has too few for every SM's 32 warps; a step takes as long as the chains
+  // of its warp's walks together.  ms with 32 / 16 / 8 / 4 / 2: one block of text 0.38 / 0.25 / 0.17 / 0.13 / 0.12,
+  // 16 blocks 0.41 / 0.29 / 0.22 / 0.21 / 0.32, 64 blocks 0.57 / 0.50 / 0.54 / 0.66 / 1.03, 128 blocks 0.82 / 0.87 /
+  // 0.95 / 1.2 / 1.9.
+  uint32_t walks = 32;
+  while (walks > 2 && 2 * (A.nb * A.nseg / walks) <= 148 * 32) walks /= 2;
+  k_enc_walk<<<A.nb * (A.nseg / walks), 32, 0, st>>>(A, walks);
   S.end(st);
   S.begin("k_enc_parse", st);
   const size_t fin = A.nseg / 32 * sizeof(Finish);
