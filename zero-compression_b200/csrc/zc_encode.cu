@@ -98,19 +98,6 @@ constexpr uint32_t kSortTile = 4096, kSortThreads = 512, kSortPer = kSortTile / 
 
 __device__ __forceinline__ uint32_t sort_tiles(uint32_t B) { return (B + kSortTile - 1) / kSortTile; }
 
-// the entry's word and its 16-bit hash (pass 1: its high byte alone, in the high byte's place)
-template <int PASS>
-__device__ __forceinline__ void sort_load(const EncArgs& A, uint32_t b, uint32_t i, uint32_t& e, uint32_t& h) {
-  if (PASS == 0) {
-    const uint32_t x = product(load4(A.in, A.in_off[b] + i));
-    e = entry(i, x);
-    h = x >> 16;
-  } else {
-    const size_t so = (size_t)b * A.B;
-    e = A.tmp_e[so + i];
-    h = (uint32_t)A.tmp_d[so + i] << 8;
-  }
-}
 template <int PASS>
 __device__ __forceinline__ uint32_t sort_digit(uint32_t h) { return PASS == 0 ? (h & 0xFFu) : (h >> 8); }
 
@@ -200,79 +187,127 @@ __global__ void __launch_bounds__(256 * kScanParts) k_sort_scan(EncArgs A) {
   }
 }
 
+// The tile's entries ranked per digit, reordered and written: latency, shared memory and instruction issue about evenly,
+// so 64 warps an SM matter most (tiles of 8192, with 48, took 12.0 ms for both passes over 1 GiB of lz_mix at block 18
+// where these took 9.9).  The warps' digit counts are 16 bits, cleared by one store a thread and summed two digits a
+// word (32-bit words: 10.8 ms).  Now 9.6 ms, 64 MiB of text 0.63 (0.83 before), 1000 files 1.68 (2.10).
 template <int PASS>
 __global__ void __launch_bounds__(kSortThreads, 4) k_sort_scatter(EncArgs A) {
   constexpr uint32_t NW = kSortThreads / 32;
-  __shared__ uint32_t cw[NW][256];  // per-warp digit counts, then the warp's start within the digit
-  __shared__ uint32_t st_e[kSortTile];
+  __shared__ __align__(16) uint16_t cw[NW][256];  // per-warp digit counts, then the warp's start within the digit
+  __shared__ __align__(16) uint32_t st_e[kSortTile];  // (while entries are ranked: the warps' masks)
   __shared__ uint16_t st_h[kSortTile];
-  __shared__ uint32_t dst[256], ws[8];  // (dst: where a digit's run goes, less its start in the tile)
+  __shared__ uint32_t dst[256], ws[4];  // (dst: where a digit's run goes, less its start in the tile)
+  static_assert(sizeof(cw) == 16 * kSortThreads && kSortTile <= 0xFFFF, "16 bytes a thread; counts of 16 bits");
+  static_assert(kSortTile >= 256 * NW, "the masks lie in the tile's array");
   const uint32_t b = blockIdx.y, t = blockIdx.x, tid = threadIdx.x, lane = lane_id(), w = tid >> 5;
   const uint32_t n = A.in_len[b], count = n >= 4 ? n - 3 : 0;
   const uint32_t i0 = t * kSortTile;
   if (i0 >= count) return;
   const uint32_t tn = min(kSortTile, count - i0);
   const size_t so = (size_t)b * A.B;
-  for (uint32_t k = tid; k < NW * 256; k += kSortThreads) (&cw[0][0])[k] = 0;
-  __syncthreads();
+  reinterpret_cast<uint4*>(&cw[0][0])[tid] = make_uint4(0, 0, 0, 0);
+  if (PASS == 0)
+    for (uint32_t k = tid; k < kSortTile / 4; k += kSortThreads) reinterpret_cast<uint4*>(st_e)[k] = make_uint4(0, 0, 0, 0);
   // ranks: warp w holds the tile's entries [kSortPer * 32 w, kSortPer * 32 (w + 1)), 32 per round, in order
   // (all of a thread's entries are loaded first: the ranking's warp syncs would otherwise keep each load
   // behind the previous entry's ranking)
-  uint32_t ke[kSortPer], kh[kSortPer], kr[kSortPer];
+  uint32_t ke[kSortPer], kh[kSortPer];  // kh: the hash, and above it the entry's rank among its warp's of the digit
+  const uint32_t l0 = w * (32 * kSortPer) + lane;
+  if (PASS == 0) {  // (32 positions are 8 words: a thread's loads lie at one address and constants from it)
+    const uint64_t x0 = A.in_off[b] + i0 + l0;
+    const uint32_t* in = reinterpret_cast<const uint32_t*>(A.in) + (x0 >> 2);
+    const uint32_t sh = (uint32_t)(x0 & 3u) * 8u;
 #pragma unroll
-  for (uint32_t j = 0; j < kSortPer; ++j) {
-    const uint32_t li = w * (32 * kSortPer) + j * 32 + lane;
-    ke[j] = 0; kh[j] = 0;
-    if (li < tn) sort_load<PASS>(A, b, i0 + li, ke[j], kh[j]);
-  }
-#pragma unroll
-  for (uint32_t j = 0; j < kSortPer; ++j) {
-    const uint32_t li = w * (32 * kSortPer) + j * 32 + lane;
-    const bool on = li < tn;
-    const uint32_t d = sort_digit<PASS>(kh[j]);
-    const unsigned act = __ballot_sync(kFull, on);
-    uint32_t rk = 0xFFFFFFFFu;
-    if (on) {
-      const unsigned peers = __match_any_sync(act, d);
-      const uint32_t c = cw[w][d];
-      rk = c + __popc(peers & ((1u << lane) - 1u));
-      __syncwarp(act);
-      if ((peers & ((1u << lane) - 1u)) == 0) cw[w][d] = c + __popc(peers);
+    for (uint32_t j = 0; j < kSortPer; ++j) {
+      ke[j] = 0; kh[j] = 0;
+      if (l0 + j * 32 < tn) {
+        const uint32_t x = product(__funnelshift_r(__ldg(in + 8 * j), __ldg(in + 8 * j + 1), sh));
+        ke[j] = entry(i0 + l0 + j * 32, x);
+        kh[j] = x >> 16;
+      }
     }
-    __syncwarp();
-    kr[j] = rk;
+  } else {  // (of the hash, the high byte alone, in the high byte's place)
+#pragma unroll
+    for (uint32_t j = 0; j < kSortPer; ++j) {
+      ke[j] = 0; kh[j] = 0;
+      if (l0 + j * 32 < tn) {
+        ke[j] = A.tmp_e[so + i0 + l0 + j * 32];
+        kh[j] = (uint32_t)A.tmp_d[so + i0 + l0 + j * 32] << 8;
+      }
+    }
   }
   __syncthreads();
-  uint32_t run = 0, inc = 0;  // per digit: the tile's count, and the digits' before it in the warp
-  if (tid < 256) {
+  // Pass 0: the lanes with a lane's digit are a mask a digit and warp, or-ed together in shared memory and cleared by
+  // its first lane (not where all 32 have one digit: 32 lanes would wait for one word).  match_any takes two of an SM's
+  // cycles for each different value in the warp, and the low bytes of a hash in position order are nearly all
+  // different (64 MiB of text: both passes 0.77 ms with it, 0.63 now); among pass 1's fewer different ones it is the
+  // faster (1 GiB of lz_mix: 9.7 ms, 10.7 with masks in both).
+  uint32_t* mask = st_e + 256 * w;
 #pragma unroll
-    for (uint32_t k = 0; k < NW; ++k) run += cw[k][tid];
-    inc = warp_incl_scan(run);
+  for (uint32_t j = 0; j < kSortPer; ++j) {
+    const bool on = l0 + j * 32 < tn;
+    const uint32_t d = on ? sort_digit<PASS>(kh[j]) : 256u;
+    uint32_t peers;
+    if (PASS == 0) {
+      int one;
+      __match_all_sync(kFull, d, &one);
+      peers = kFull;
+      if (!one) {
+        if (on) atomicOr(&mask[d], 1u << lane);
+        __syncwarp();
+        peers = on ? mask[d] : 0u;
+      }
+    } else {
+      peers = __match_any_sync(kFull, d);
+    }
+    const uint32_t lower = peers & ((1u << lane) - 1u), c = on ? cw[w][d] : 0u;
+    __syncwarp();
+    if (on && !lower) {
+      cw[w][d] = (uint16_t)(c + __popc(peers));
+      if (PASS == 0) mask[d] = 0;
+    }
+    __syncwarp();
+    kh[j] |= (c + __popc(lower)) << 16;
+  }
+  __syncthreads();
+  // two digits a thread (a word of counts): the tile's counts, and those of the digits before them in the warp
+  uint32_t run = 0, inc = 0, both = 0;
+  uint32_t* cw2 = reinterpret_cast<uint32_t*>(&cw[0][0]) + tid;
+  if (tid < 128) {
+#pragma unroll 8
+    for (uint32_t k = 0; k < NW; ++k) run += cw2[k * 128];
+    both = (run & 0xFFFFu) + (run >> 16);
+    inc = warp_incl_scan(both);
     if (lane == 31) ws[w] = inc;
   }
   __syncthreads();
-  if (tid < 256) {  // each warp's start of the digit in the reordered tile
-    uint32_t at = inc - run;
+  if (tid < 128) {  // each warp's starts of the digits in the reordered tile
+    uint32_t at = inc - both;
     for (uint32_t k = 0; k < w; ++k) at += ws[k];
-    dst[tid] = A.scnt[((size_t)b * sort_tiles(A.B) + t) * 256 + tid] - at;
-#pragma unroll
-    for (uint32_t k = 0; k < NW; ++k) { const uint32_t c = cw[k][tid]; cw[k][tid] = at; at += c; }
+    at |= (at + (run & 0xFFFFu)) << 16;
+    const uint2 g = *reinterpret_cast<const uint2*>(A.scnt + ((size_t)b * sort_tiles(A.B) + t) * 256 + 2 * tid);
+    dst[2 * tid] = g.x - (at & 0xFFFFu);
+    dst[2 * tid + 1] = g.y - (at >> 16);
+#pragma unroll 8
+    for (uint32_t k = 0; k < NW; ++k) { const uint32_t c = cw2[k * 128]; cw2[k * 128] = at; at += c; }
   }
   __syncthreads();
 #pragma unroll
   for (uint32_t j = 0; j < kSortPer; ++j) {
-    if (kr[j] == 0xFFFFFFFFu) continue;
-    const uint32_t at = cw[w][sort_digit<PASS>(kh[j])] + kr[j];
+    if (l0 + j * 32 >= tn) continue;
+    const uint32_t h = kh[j] & 0xFFFFu, at = cw[w][sort_digit<PASS>(h)] + (kh[j] >> 16);
     st_e[at] = ke[j];
-    st_h[at] = (uint16_t)kh[j];
+    st_h[at] = (uint16_t)h;
   }
   __syncthreads();
-  uint32_t* oe = PASS == 0 ? A.tmp_e : A.srt;
+  uint32_t* oe = (PASS == 0 ? A.tmp_e : A.srt) + so;
+  uint8_t* od = A.tmp_d + so;
+#pragma unroll 4
   for (uint32_t i = tid; i < tn; i += kSortThreads) {
-    const uint32_t h = st_h[i], d = sort_digit<PASS>(h);
-    const size_t dest = so + (dst[d] + i);
+    const uint32_t h = st_h[i], dest = dst[sort_digit<PASS>(h)] + i;
     oe[dest] = st_e[i];
-    if (PASS == 0) A.tmp_d[dest] = (uint8_t)(h >> 8);
+    if (PASS == 0) od[dest] = (uint8_t)(h >> 8);
   }
 }
 
