@@ -418,7 +418,7 @@ struct Finish {
   uint32_t x[32], key[32];                            // its position; best so far
   uint4 req[32];  // the requests one after the other: the entry's place | tag << 20; position | an offset << 20; the 4
                   // bytes there, which a candidate that matters has too; slot << 20
-  uint32_t it[kItems], deep[kItems + 32], far[kItems + 32];  // not compared; equal for 16 bytes; for 32
+  uint32_t it[kItems], deep[kItems];  // not compared, then those equal for 32 bytes; equal for 16
   uint32_t batch[kBatch];
 };
 
@@ -426,9 +426,11 @@ struct Finish {
 __device__ __forceinline__ uint32_t k_len(uint32_t key) { return (key >> 20) + 1u; }
 
 // Works the lists off: cnt candidates not compared (W.it), n2 equal for 16 bytes (W.deep), into the slots' keys.
+// (One of the two counts is 0, so no list grows over kItems.)
 __device__ __forceinline__ void finish_lists(const ParseBlock& P, Finish& W, uint32_t cnt, uint32_t n2) {
   const uint32_t lane = lane_id(), below = (1u << lane) - 1u;
   const uint64_t base = P.base;
+  uint32_t* const far = W.it;  // (equal for 32 bytes: written when W.it has been worked off)
   __syncwarp();
   // the first 16 bytes, a lane a candidate
   for (uint32_t k = 0; k < cnt; k += 32) {
@@ -461,7 +463,7 @@ __device__ __forceinline__ void finish_lists(const ParseBlock& P, Finish& W, uin
       more = l == 16u && lim > 32u;
     }
     const unsigned mm = __ballot_sync(kFull, more);
-    if (more) W.far[n3 + __popc(mm & below)] = c;
+    if (more) far[n3 + __popc(mm & below)] = c;
     n3 += (uint32_t)__popc(mm);
   }
   __syncwarp();
@@ -474,13 +476,13 @@ __device__ __forceinline__ void finish_lists(const ParseBlock& P, Finish& W, uin
     uint32_t m = 0, nb = 0, carry = 32;  // kept ones, this round's, the last kept one's slot
     const uint32_t* batch = W.batch;
     if (n3 <= kBatch) {  // (so few that all are extended)
-      batch = W.far;
+      batch = far;
       nb = n3;
       n3 = 0;
     }
     for (uint32_t k = 0; k < n3; k += 32) {
       const bool on = k + lane < n3;
-      const uint32_t c = on ? W.far[k + lane] : 0u, i = c >> 20, j = c & 0xFFFFFu;
+      const uint32_t c = on ? far[k + lane] : 0u, i = c >> 20, j = c & 0xFFFFFu;
       const uint32_t x = W.x[i], key = W.key[i], lim = min(kMaxMatch, P.n - x);
       const bool best = j == (key & 0xFFFFFu);  // (the best is here only until it has been extended)
       const uint32_t at = k_len(key) - (j > (key & 0xFFFFFu) ? 1u : 0u);
@@ -495,7 +497,7 @@ __device__ __forceinline__ void finish_lists(const ParseBlock& P, Finish& W, uin
       const bool sel = first && fk < kBatch;
       if (sel) W.batch[fk] = c;
       const unsigned rm = km & ~__ballot_sync(kFull, sel);
-      if (rm >> lane & 1u) W.far[m + __popc(rm & below)] = c;
+      if (rm >> lane & 1u) far[m + __popc(rm & below)] = c;
       m += (uint32_t)__popc(rm);
       nb = min(kBatch, nb + (uint32_t)__popc(fm));
       if (km) carry = __shfl_sync(kFull, i, 31u - __clz(km));
@@ -726,15 +728,21 @@ __device__ __forceinline__ uint32_t warp_step(const ParseBlock& P, Finish& W, ui
 
 // The parse is a chain 0 -> next(0) -> ... cut into A.nseg segments of each block.  Every segment's walk from its
 // own start, a lane a walk: it leaves the exact records of the positions that it visits in minfo, its tokens in the
-// segment's slots, and where it leaves the segment, with the count, in seg_exit.  A warp, a CTA of its own, takes `walks`
-// (2 to 32) consecutive segments, its other lanes helping to finish records; no warp waits for another, so a launch
+// segment's slots, and where it leaves the segment, with the count, in seg_exit.  A warp takes `walks` (2 to 32)
+// consecutive segments, its other lanes helping to finish records; no warp waits for another, so a launch
 // of few blocks spreads over the whole GPU.  (Two or four segments a lane, handed out as lanes got done, kept more
 // lanes busy, but the fewer warps took longer: 10.5, 10.8, 11.5 ms for 1 GiB of lz_mix in 512-byte segments.)
 // Text in 512-byte segments is bound by L2 misses: 32 warps an SM are then in 296 blocks' candidate orders, 1.25 MiB
 // each, 103 bytes read from memory a byte of input; lz_mix has few candidates and does not mind.
-__global__ void __launch_bounds__(32, 32) k_enc_walk(EncArgs A, uint32_t walks) {
-  __shared__ Finish W;
-  const uint32_t per = A.nseg / walks, b = blockIdx.x / per, q = blockIdx.x % per * walks + lane_id();
+// The walks' own loads live on the L1, which has what 32 warps' lists leave of an SM's 256 KiB: two warps a CTA and
+// 2688 bytes of lists a warp leave 128 KiB (1 GiB of lz_mix 8.7 ms, 64 MiB of text 1.62, 256 MiB at depth 256 6.5);
+// one, and 3584 bytes, left 64 (8.8, 1.68, 6.8).  40 or 48 warps in as many registers as that leaves: 8.9 and 9.4, text
+// 1.9 and 2.5.
+__global__ void __launch_bounds__(64, 16) k_enc_walk(EncArgs A, uint32_t walks) {
+  __shared__ Finish Ws[2];
+  Finish& W = Ws[threadIdx.x >> 5];
+  const uint32_t per = A.nseg / walks, wi = blockIdx.x * 2 + (threadIdx.x >> 5);  // (per is even: 8 or more)
+  const uint32_t b = wi / per, q = wi % per * walks + lane_id();
   const bool mine = lane_id() < walks;
   const uint32_t n = A.in_len[b];
   const size_t so = (size_t)b * A.B;
@@ -1478,7 +1486,7 @@ void launch_encode(const EncArgs& A, const CrcArgs& crc_in, cudaStream_t st, Sta
   // 0.95 / 1.2 / 1.9.
   uint32_t walks = 32;
   while (walks > 2 && 2 * (A.nb * A.nseg / walks) <= 148 * 32) walks /= 2;
-  k_enc_walk<<<A.nb * (A.nseg / walks), 32, 0, st>>>(A, walks);
+  k_enc_walk<<<A.nb * (A.nseg / walks) / 2, 64, 0, st>>>(A, walks);
   S.end(st);
   S.begin("k_enc_parse", st);
   const size_t fin = A.nseg / 32 * sizeof(Finish);
