@@ -95,6 +95,7 @@ __device__ __forceinline__ uint32_t lcp16(const uint4& a, const uint4& b) {
 // position in all (22 with the hash beside the position in both passes).  The counts array holds
 // tiles_per_block(B) * 256 words per block.
 constexpr uint32_t kSortTile = 4096, kSortThreads = 512, kSortPer = kSortTile / kSortThreads;
+constexpr int kCrowd = 3;
 
 __device__ __forceinline__ uint32_t sort_tiles(uint32_t B) { return (B + kSortTile - 1) / kSortTile; }
 
@@ -190,7 +191,7 @@ __global__ void __launch_bounds__(256 * kScanParts) k_sort_scan(EncArgs A) {
 // The tile's entries ranked per digit, reordered and written: latency, shared memory and instruction issue about evenly,
 // so 64 warps an SM matter most (tiles of 8192, with 48, took 12.0 ms for both passes over 1 GiB of lz_mix at block 18
 // where these took 9.9).  The warps' digit counts are 16 bits, cleared by one store a thread and summed two digits a
-// word (32-bit words: 10.8 ms).  Now 9.6 ms, 64 MiB of text 0.63 (0.83 before), 1000 files 1.68 (2.10).
+// word (32-bit words: 10.8 ms).  Now 9.3 ms, 64 MiB of text 0.62 (0.83 before), 1000 files 1.66 (2.10).
 template <int PASS>
 __global__ void __launch_bounds__(kSortThreads, 4) k_sort_scatter(EncArgs A) {
   constexpr uint32_t NW = kSortThreads / 32;
@@ -239,21 +240,22 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_sort_scatter(EncArgs A) {
   }
   __syncthreads();
   // Pass 0: the lanes with a lane's digit are a mask a digit and warp, or-ed together in shared memory and cleared by
-  // its first lane (not where all 32 have one digit: 32 lanes would wait for one word).  match_any takes two of an SM's
-  // cycles for each different value in the warp, and the low bytes of a hash in position order are nearly all
-  // different (64 MiB of text: both passes 0.77 ms with it, 0.63 now); among pass 1's fewer different ones it is the
-  // faster (1 GiB of lz_mix: 9.7 ms, 10.7 with masks in both).
+  // its first lane.  match_any takes two of an SM's cycles for each different value in the warp, and the low bytes of a
+  // hash in position order are nearly all different (64 MiB of text: both passes 0.77 ms with it, 0.62 now).  Where a
+  // digit had more than kCrowd lanes, as in short periods and runs, the next round takes match_any: equal digits wait
+  // for one word of shared memory (1 GiB of lz_mix 9.6 ms with masks alone, 9.3 now, 9.4 with a line at 10 lanes).
+  // Pass 1 has match_any alone (with masks, by the same rule, 9.7, but 1000 files 1.48 for 1.66).
   uint32_t* mask = st_e + 256 * w;
+  bool crowded = false;
 #pragma unroll
   for (uint32_t j = 0; j < kSortPer; ++j) {
     const bool on = l0 + j * 32 < tn;
     const uint32_t d = on ? sort_digit<PASS>(kh[j]) : 256u;
     uint32_t peers;
     if (PASS == 0) {
-      int one;
-      __match_all_sync(kFull, d, &one);
-      peers = kFull;
-      if (!one) {
+      if (crowded) {
+        peers = __match_any_sync(kFull, d);
+      } else {
         if (on) atomicOr(&mask[d], 1u << lane);
         __syncwarp();
         peers = on ? mask[d] : 0u;
@@ -265,8 +267,9 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_sort_scatter(EncArgs A) {
     __syncwarp();
     if (on && !lower) {
       cw[w][d] = (uint16_t)(c + __popc(peers));
-      if (PASS == 0) mask[d] = 0;
+      if (PASS == 0 && !crowded) mask[d] = 0;
     }
+    if (PASS == 0) crowded = __any_sync(kFull, __popc(peers) > kCrowd);
     __syncwarp();
     kh[j] |= (c + __popc(lower)) << 16;
   }
