@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(256 * kScanParts) k_sort_scan(EncArgs A) {
 // The tile's entries ranked per digit, reordered and written: latency, shared memory and instruction issue about evenly,
 // so 64 warps an SM matter most (tiles of 8192, with 48, took 12.0 ms for both passes over 1 GiB of lz_mix at block 18
 // where these took 9.9).  The warps' digit counts are 16 bits, cleared by one store a thread and summed two digits a
-// word (32-bit words: 10.8 ms).  Now 9.3 ms, 64 MiB of text 0.62 (0.83 before), 1000 files 1.66 (2.10).
+// word (32-bit words: 10.8 ms).  Now 9.3 ms, 64 MiB of text 0.62 (0.83 before), 1000 files 1.44 (2.10).
 template <int PASS>
 __global__ void __launch_bounds__(kSortThreads, 4) k_sort_scatter(EncArgs A) {
   constexpr uint32_t NW = kSortThreads / 32;
@@ -208,8 +208,6 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_sort_scatter(EncArgs A) {
   const uint32_t tn = min(kSortTile, count - i0);
   const size_t so = (size_t)b * A.B;
   reinterpret_cast<uint4*>(&cw[0][0])[tid] = make_uint4(0, 0, 0, 0);
-  if (PASS == 0)
-    for (uint32_t k = tid; k < kSortTile / 4; k += kSortThreads) reinterpret_cast<uint4*>(st_e)[k] = make_uint4(0, 0, 0, 0);
   // ranks: warp w holds the tile's entries [kSortPer * 32 w, kSortPer * 32 (w + 1)), 32 per round, in order
   // (all of a thread's entries are loaded first: the ranking's warp syncs would otherwise keep each load
   // behind the previous entry's ranking)
@@ -239,37 +237,32 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_sort_scatter(EncArgs A) {
     }
   }
   __syncthreads();
-  // Pass 0: the lanes with a lane's digit are a mask a digit and warp, or-ed together in shared memory and cleared by
-  // its first lane.  match_any takes two of an SM's cycles for each different value in the warp, and the low bytes of a
-  // hash in position order are nearly all different (64 MiB of text: both passes 0.77 ms with it, 0.62 now).  Where a
-  // digit had more than kCrowd lanes, as in short periods and runs, the next round takes match_any: equal digits wait
-  // for one word of shared memory (1 GiB of lz_mix 9.6 ms with masks alone, 9.3 now, 9.4 with a line at 10 lanes).
-  // Pass 1 has match_any alone (with masks, by the same rule, 9.7, but 1000 files 1.48 for 1.66).
+  // The lanes with a lane's digit: a mask a digit and warp, or-ed together in shared memory, or match_any, which takes
+  // two of an SM's cycles for each different value in the warp; in masks equal digits wait for one word.  A round takes
+  // match_any if the one before had a digit of more than kCrowd lanes, as in short periods and runs; pass 0 begins with
+  // masks (in position order the hashes' low bytes are nearly all different), pass 1 with match_any.  Both passes, ms,
+  // match_any alone / masks by this rule in pass 0 / in both: 1 GiB of lz_mix 9.9 / 9.24 / 9.33, 64 MiB of text 0.77 /
+  // 0.62 / 0.62, 1000 files 1.94 / 1.65 / 1.44.  (Masks alone in pass 0: 9.6, 0.63, 1.68.)
   uint32_t* mask = st_e + 256 * w;
-  bool crowded = false;
+  bool crowded = PASS == 1;
 #pragma unroll
   for (uint32_t j = 0; j < kSortPer; ++j) {
     const bool on = l0 + j * 32 < tn;
     const uint32_t d = on ? sort_digit<PASS>(kh[j]) : 256u;
     uint32_t peers;
-    if (PASS == 0) {
-      if (crowded) {
-        peers = __match_any_sync(kFull, d);
-      } else {
-        if (on) atomicOr(&mask[d], 1u << lane);
-        __syncwarp();
-        peers = on ? mask[d] : 0u;
-      }
-    } else {
+    if (crowded) {
       peers = __match_any_sync(kFull, d);
+    } else {
+      if (on) mask[d] = 0;
+      __syncwarp();
+      if (on) atomicOr(&mask[d], 1u << lane);
+      __syncwarp();
+      peers = on ? mask[d] : 0u;
     }
     const uint32_t lower = peers & ((1u << lane) - 1u), c = on ? cw[w][d] : 0u;
     __syncwarp();
-    if (on && !lower) {
-      cw[w][d] = (uint16_t)(c + __popc(peers));
-      if (PASS == 0 && !crowded) mask[d] = 0;
-    }
-    if (PASS == 0) crowded = __any_sync(kFull, __popc(peers) > kCrowd);
+    if (on && !lower) cw[w][d] = (uint16_t)(c + __popc(peers));
+    crowded = __any_sync(kFull, __popc(peers) > kCrowd);
     __syncwarp();
     kh[j] |= (c + __popc(lower)) << 16;
   }
@@ -476,7 +469,7 @@ __device__ __forceinline__ void finish_lists(const ParseBlock& P, Finish& W, uin
   // there differs.  (Eight at a time, four lanes each: the walks took 10.3 ms for 1 GiB of lz_mix against 9.2, 7.6
   // against 6.6 for 256 MiB at depth 256.)
   while (n3) {
-    uint32_t m = 0, nb = 0, carry = 32;  // kept ones, this round's, the last kept one's slot
+    uint32_t m = 0, nb = 0, carry = 32;  // kept ones, those of this turn, the last kept one's slot
     const uint32_t* batch = W.batch;
     if (n3 <= kBatch) {  // (so few that all are extended)
       batch = far;
