@@ -15,8 +15,8 @@
 //                  of every segment of every block; a warp's walks step together, and the exact matches that
 //                  a step needs are computed by the warp for all its walks at once (warp_finish), only at
 //                  positions that a walk visits
-//   k_enc_parse    one CTA per block: segments re-walked from where the chain before them leaves until they
-//                  meet the first walk (rounds until no segment exit moves), then the tokens written
+//   k_enc_parse    one CTA per block: the segments that the chain enters, found over the walks' exits, re-walked from
+//                  there until they meet the first walk (rounds until no exit moves), then the tokens written
 //   k_enc_streams  one CTA per block, a lane a token: group starts from a running maximum of per-token thresholds
 //                  and next-start chains, recent offsets from each group's start, tok / ext / sym / group streams
 //                  placed by scans, offset bits gathered in shared memory, literals
@@ -408,7 +408,7 @@ struct ParseBlock {
 // memory.  A candidate is slot << 20 | its position.
 constexpr uint32_t kTasks = 4;                        // chain loads in flight together
 constexpr uint32_t kItems = 32 + 32 * kTasks;         // the most candidates that wait at a time
-constexpr uint32_t kBatch = 32;
+constexpr uint32_t kBatch = 32, kPause = 256;
 struct Finish {
   uint4 xw[32];                                       // the first 16 bytes at the request's position
   uint32_t x[32], key[32];                            // its position; best so far
@@ -421,9 +421,15 @@ struct Finish {
 // key: (length - 1) << 20 | the candidate's position: the longest match, the nearest on a tie, is the largest
 __device__ __forceinline__ uint32_t k_len(uint32_t key) { return (key >> 20) + 1u; }
 
+// What a walk knows of the bytes that it comes to: up to position `end` they equal those `dist` before them (0: nothing).
+struct Known {
+  uint32_t end = 0, dist = 0;
+};
+
 // Works the lists off: cnt candidates not compared (W.it), n2 equal for 16 bytes (W.deep), into the slots' keys.
-// (One of the two counts is 0, so no list grows over kItems.)
-__device__ __forceinline__ void finish_lists(const ParseBlock& P, Finish& W, uint32_t cnt, uint32_t n2) {
+// (One of the two counts is 0, so no list grows over kItems.)  With KNOW, each lane brings its request's `kn`.
+template <bool KNOW>
+__device__ __forceinline__ void finish_lists(const ParseBlock& P, Finish& W, uint32_t cnt, uint32_t n2, const Known& kn) {
   const uint32_t lane = lane_id(), below = (1u << lane) - 1u;
   const uint64_t base = P.base;
   uint32_t* const far = W.it;  // (equal for 32 bytes: written when W.it has been worked off)
@@ -447,31 +453,46 @@ __device__ __forceinline__ void finish_lists(const ParseBlock& P, Finish& W, uin
   __syncwarp();
   // the next 16, a lane a candidate
   uint32_t n3 = 0;
+  bool one = false;  // of each request, one candidate is extended at a time
   for (uint32_t k = 0; k < n2; k += 32) {
     const bool on = k + lane < n2;
     const uint32_t c = on ? W.deep[k + lane] : 0u, i = c >> 20, j = c & 0xFFFFFu;
     const uint32_t x = W.x[i], key = W.key[i], lim = min(kMaxMatch, P.n - x);
+    uint32_t known = 0;
+    if (KNOW) {
+      const uint32_t ke = __shfl_sync(kFull, kn.end, i), kd = __shfl_sync(kFull, kn.dist, i);
+      if (kd == x - j && ke > x + 32) known = ke - x;
+      one |= __any_sync(kFull, on && known);
+    }
     bool more = false;
     if (on && !(k_len(key) == lim && j < (key & 0xFFFFFu))) {  // (a nearer match of the whole length cannot be beaten)
-      const uint32_t l = lcp16(load16(P.in, base + j + 16), load16(P.in, base + x + 16));
-      const uint32_t len = min(16u + l, lim);
+      const uint32_t l = known ? 16u : lcp16(load16(P.in, base + j + 16), load16(P.in, base + x + 16));
+      const uint32_t len = min(known ? known : 16u + l, lim);
       if (len > 16u) atomicMax(&W.key[i], (len - 1u) << 20 | j);
-      more = l == 16u && lim > 32u;
+      more = l == 16u && lim > max(known, 32u);
     }
     const unsigned mm = __ballot_sync(kFull, more);
     if (more) far[n3 + __popc(mm & below)] = c;
     n3 += (uint32_t)__popc(mm);
   }
   __syncwarp();
-  // The rest are extended, up to 32 at a time, 32 lanes / their number each (four lanes take 64 bytes a step), until
-  // none is left.  Of more than 32, those that can still win, the first one of each request: one that is nearer than
-  // its request's best wins with the best's length, a farther one only with more, so it is dropped when its byte
-  // there differs.  (Eight at a time, four lanes each: the walks took 10.3 ms for 1 GiB of lz_mix against 9.2, 7.6
-  // against 6.6 for 256 MiB at depth 256.)
+  // The rest are extended, up to 32 at a time, 32 lanes / their number each and 16 bytes a lane a step, until none is
+  // left.  Of more than 32, those that can still win, the first one of each request: one that is nearer than its request's
+  // best wins with the best's length, a farther one only with more, so it is dropped when its byte there differs.
+  // (Eight at a time, four lanes each: the walks took 10.3 ms for 1 GiB of lz_mix against 9.2, 7.6 against 6.6 for
+  // 256 MiB at depth 256.  Four lanes each at most: the whole call 27.1 ms against 26.2, and 25 us for one match of 4096
+  // bytes.)
+  // In runs and periods the matches of all the warp's requests go on to the longest length or the run's end, at one
+  // distance.  So a candidate at the distance of the one after it is compared only up to that one's position: it
+  // ends where that one ends.  The parse's walks also bring what they know of the bytes before them (Known), and where
+  // two candidates of a request go on after kPause bytes, one of each request is extended at a time from there on.
+  // Walks and parse, ms, before all this / now: 256 MiB of one value at block 18 22.2 / 3.7, at block 20 and depth 256
+  // 19.1 / 3.1; of a period of 5000 bytes 61.1 / 8.4 and 69.7 / 6.6; one such block of 1 MiB 30.1 / 2.1.
   while (n3) {
     uint32_t m = 0, nb = 0, carry = 32;  // kept ones, those of this turn, the last kept one's slot
     const uint32_t* batch = W.batch;
-    if (n3 <= kBatch) {  // (so few that all are extended)
+    const bool few = n3 <= kBatch && !one;
+    if (few) {  // (so few that all are extended)
       batch = far;
       nb = n3;
       n3 = 0;
@@ -501,27 +522,55 @@ __device__ __forceinline__ void finish_lists(const ParseBlock& P, Finish& W, uin
     }
     n3 = m;
     if (!nb) break;  // (none was kept)
-    const uint32_t sh = nb <= 8 ? 2u : nb <= 16 ? 1u : 0u;  // 4 lanes each for a few (64 bytes a step), else fewer
+    const uint32_t sh = (uint32_t)__clz(nb - 1u) - 27u;  // 2^sh lanes each
     const uint32_t g = lane >> sh, gl = lane & ((1u << sh) - 1u);
-    bool act = g < nb;
+    bool act = g < nb, back = false;
     const uint32_t c = act ? batch[g] : 0u, i = c >> 20, j = c & 0xFFFFFu;
     const uint32_t x = W.x[i], lim = min(kMaxMatch, P.n - x);
     const bool mine = act && gl == 0;
-    uint32_t len = 32;
-    for (uint32_t o = 32; __any_sync(kFull, act); o += 16u << sh) {
-      const uint32_t q = o + 16u * gl;
-      uint32_t e = lim;  // the match's end, if it lies in this lane's 16 bytes
-      bool stop = act;
-      if (act && q < lim) {
-        const uint32_t l = lcp16(load16(P.in, base + j + q), load16(P.in, base + x + q));
-        e = min(q + l, lim);
-        stop = l < 16u || q + 16u >= lim;
+    // the next candidate, if it is at this distance too, and the bytes before it (requests rise in position)
+    uint32_t next = min((g + 1u) << sh, 31u);
+    const uint32_t gap = __shfl_sync(kFull, x, next) - x, step = __shfl_sync(kFull, x - j, next);
+    if (g + 1u >= nb || step != x - j) next = lane;
+    const uint32_t upto = next != lane ? min(lim, gap) : lim;
+    uint32_t len = 32, o = 32;
+    if (KNOW) {
+      const uint32_t ke = __shfl_sync(kFull, kn.end, i), kd = __shfl_sync(kFull, kn.dist, i);
+      if (kd == x - j && ke > x + 32) o = ke - x;
+    }
+    for (uint32_t done = 32; __any_sync(kFull, act); o += 16u << sh, done += 16u << sh) {
+      if (KNOW && few && done - kPause < 16u << sh) {  // (once)
+        const uint32_t peers = __match_any_sync(kFull, mine && act ? i : 32u + lane);
+        if (__any_sync(kFull, peers & below)) { back = act; act = false; }
       }
-      const unsigned sm = __ballot_sync(kFull, stop) >> (g << sh) & ((1u << (1u << sh)) - 1u);
+      const uint32_t q = o + 16u * gl;
+      uint32_t e = upto;  // the match's end, if it lies in this lane's 16 bytes
+      bool stop = act;
+      if (act && q < upto) {
+        const uint32_t l = lcp16(load16(P.in, base + j + q), load16(P.in, base + x + q));
+        e = min(q + l, upto);
+        stop = l < 16u || q + 16u >= upto;
+      }
+      const unsigned sm = __ballot_sync(kFull, stop) >> (g << sh) & 0xFFFFFFFFu >> (32u - (1u << sh));
       const uint32_t v = __shfl_sync(kFull, e, (g << sh) + (sm ? (uint32_t)__ffs(sm) - 1u : 0u));
       if (act && sm) { len = v; act = false; }
     }
-    if (mine) atomicMax(&W.key[i], (len - 1u) << 20 | j);
+    if (back || len != gap) next = lane;
+    if (__any_sync(kFull, next != lane)) {  // a match that reaches the next candidate's position ends where that one does
+      uint32_t end = x + len;
+#pragma unroll
+      for (uint32_t k = 0; k < 5; ++k) next = __shfl_sync(kFull, next, next);
+      end = __shfl_sync(kFull, end, next);
+      back = __shfl_sync(kFull, back, next);
+      len = min(end - x, lim);
+    }
+    if (mine && !back) atomicMax(&W.key[i], (len - 1u) << 20 | j);
+    const unsigned bm = __ballot_sync(kFull, mine && back);
+    if (bm) {  // (far is empty)
+      if (mine && back) far[__popc(bm & below)] = c;
+      n3 = (uint32_t)__popc(bm);
+      one = true;
+    }
     __syncwarp();
   }
   __syncwarp();
@@ -544,8 +593,9 @@ __device__ __forceinline__ void finish_lists(const ParseBlock& P, Finish& W, uin
 // (One request after the other by the whole warp, its 32 candidates a lane each, waited for three to six
 // dependent loads a request: 5.4 us each with 64 warps an SM.  Comparing every candidate of the tag, 16 bytes and
 // on, took 530 warp instructions a token of lz_mix at block 18, level 5.)
+template <bool KNOW>
 __device__ __forceinline__ void warp_finish(const ParseBlock& P, Finish& W, bool act, uint32_t p, uint32_t& v,
-                                            uint32_t& v2) {
+                                            uint32_t& v2, const Known& kn) {
   const uint32_t lane = lane_id(), below = (1u << lane) - 1u;
   const uint32_t G = min(32u, P.depth);  // lanes a request: 32, or 8 at depth 8
   const uint32_t gl = lane & (G - 1u), NR = 32u / G;
@@ -579,7 +629,7 @@ __device__ __forceinline__ void warp_finish(const ParseBlock& P, Finish& W, bool
     if (more) W.deep[__popc(mm & below)] = c;
     n2 = (uint32_t)__popc(mm);
   }
-  finish_lists(P, W, 0, n2);
+  finish_lists<KNOW>(P, W, 0, n2, kn);
   const uint32_t subs = P.depth > 32 ? 3u : 1u;  // chains are scanned 32 entries first, then the next 128, then the rest
   uint32_t need = 0;
 #pragma unroll 1
@@ -662,7 +712,7 @@ __device__ __forceinline__ void warp_finish(const ParseBlock& P, Finish& W, bool
           }
           t += kTasks;
         }
-        finish_lists(P, W, cnt, 0);
+        finish_lists<KNOW>(P, W, cnt, 0, kn);
       } while (t < nt);
       ask = ask && !(ended >> mine & 1u);
     }
@@ -683,8 +733,10 @@ __device__ __forceinline__ void warp_finish(const ParseBlock& P, Finish& W, bool
 // Positions without a match are literal steps to the next one: a run of them is taken together with the token
 // after it, up to `lim` (the walk's end), where the walk lands if the run reaches it.  A position whose
 // finished record turns out to be NONE is a literal step by itself.
+template <bool KNOW>
 __device__ __forceinline__ uint32_t warp_step(const ParseBlock& P, Finish& W, uint32_t p, uint32_t lim, bool act,
-                                              bool& tok, uint32_t& ti, uint32_t& tm, uint32_t& td) {
+                                              bool& tok, uint32_t& ti, uint32_t& tm, uint32_t& td,
+                                              const Known& kn = Known()) {
   uint32_t v = M_NONE, v2 = M_NONE;
   if (act) {
     // eight records at a time, from two aligned loads: the first that is not NONE ends the run (a load a record, or
@@ -709,7 +761,7 @@ __device__ __forceinline__ uint32_t warp_step(const ParseBlock& P, Finish& W, ui
     if (v != M_NONE && p + 1 < P.n) v2 = m[p + 1];
     if (m_is_below(v2)) v2 = M_NONE;  // (of no use to p's lazy test)
   }
-  if (__any_sync(kFull, m_is_sat(v) || m_is_sat(v2))) warp_finish(P, W, act, p, v, v2);
+  if (__any_sync(kFull, m_is_sat(v) || m_is_sat(v2))) warp_finish<KNOW>(P, W, act, p, v, v2, kn);
   tok = false;
   if (!act) return p;
   if (v == M_NONE) return p < lim ? p + 1 : p;
@@ -751,33 +803,27 @@ __global__ void __launch_bounds__(64, 16) k_enc_walk(EncArgs A, uint32_t walks) 
   const uint32_t e = min(p + S, n);
   bool t; uint32_t ta, tc, td;
   while (__any_sync(kFull, p < e)) {
-    p = warp_step(P, W, p, e, p < e, t, ta, tc, td);
+    p = warp_step<false>(P, W, p, e, p < e, t, ta, tc, td);
     if (t) toks[cnt++] = tk_pack(ta, tc, td);
   }
   if (mine) A.seg_exit[(size_t)b * A.nseg + q] = make_uint2(p, cnt);
 }
 
-// how many of a walk's n tokens lie before position c
-__device__ __forceinline__ uint32_t tk_after(const uint2* toks, uint32_t n, uint32_t c) {
-  uint32_t lo = 0;
-  while (lo < n) {
-    const uint32_t mid = (lo + n) >> 1;
-    if (tk_i(toks[mid]) < c) lo = mid + 1; else n = mid;
-  }
-  return lo;
-}
-
-// One CTA per block, a lane a segment.  Rounds re-walk each segment from where the chain before it leaves, until
-// that walk meets the previous one (a two-pointer merge), and end when no segment's exit moves.  Then every
-// segment's tokens are its first walk's (k_enc_walk) from where the walk from its true entry meets that one, after
-// those of the steps before; a walk that starts at the wrong place meets the right one within a step or two.  (A whole
-// walk from the true entry for the tokens: 2.26 ms per GiB of lz_mix at block 18, 0.52 for 64 MiB of text.)
+// One CTA per block, a lane a segment.  Each round follows the chain over the segments' exits as far as they are known,
+// and a segment that it enters elsewhere than before is walked from there until that walk comes to a position of
+// the first one (k_enc_walk's: its start, its tokens' ends, its exit); the segment's tokens are those of the steps
+// before, then the first walk's.  A walk that starts at the wrong place meets the right one within a step or two.  The
+// rounds end when no exit moves; a warp takes its part of the chain to its end before the next one.  (A whole walk from
+// the true entry for the tokens: 2.26 ms per GiB of lz_mix at block 18, 0.52 for 64 MiB of text; now 0.35 and 0.17.)
+// Where a match covers many segments, as in runs and periods, whose walks never meet, a step of the chain settles a
+// match.  (Exits handed from each segment to the next, skipped ones among them, settled one segment a round: one block
+// of 1 MiB of one value 6.5 ms, now 1.0; of 256 KiB 2.0, now 0.28.)
 template <uint32_t T>
 __global__ void __launch_bounds__(T, 1024 / T) k_enc_parse(EncArgs A) {
-  const uint32_t b = blockIdx.x, q = threadIdx.x;
+  const uint32_t b = blockIdx.x, q = threadIdx.x, lane = lane_id(), below = (1u << lane) - 1u;
   const uint32_t n = A.in_len[b];
   const size_t so = (size_t)b * A.B;
-  __shared__ uint32_t ent[T], ex[T], wsum[T / 32];
+  __shared__ uint32_t hop[T], wsum[T / 32];
   extern __shared__ uint4 parse_sm[];
   Finish& W = reinterpret_cast<Finish*>(parse_sm)[q >> 5];
   ParseBlock P;
@@ -786,89 +832,99 @@ __global__ void __launch_bounds__(T, 1024 / T) k_enc_parse(EncArgs A) {
   const uint32_t S = seg_bytes(n, T);
   const uint32_t s = min(q * S, n), e = min(s + S, n);
   bool t; uint32_t ta, tc, td;
-  ent[q] = s;
   const uint2 first = A.seg_exit[(size_t)b * T + q];  // the first walk's exit, its tokens
-  ex[q] = first.x;
+  uint32_t ent = s, ex = first.x;
   // the segment's tokens: cnt of its own slots, then the first walk's from the from-th on
   const uint32_t slots = S / 4 + 2;
   const uint2* old = A.tk_seg + (size_t)b * 2 * seg_tok_cap(A.B) + (size_t)q * slots;
   uint2* own = A.tk_seg + ((size_t)b * 2 + 1) * seg_tok_cap(A.B) + (size_t)q * slots;
   uint32_t cnt = 0, from = 0;
-  bool again = false;  // the entry moved twice: the tokens are taken after the rounds
-  // rounds: each segment re-walked from where the chain before it leaves, until it meets its old walk
+  // from each lane on, the warp's segments that the chain enters, the last of them, and the segment it enters after each
+  uint32_t follow, far, goes;
+  auto chain = [&]() {
+    goes = ex >= n ? T : ex / S;  // (an exit lies past its segment)
+    uint32_t nx = min(goes - (q & ~31u), 32u);
+    follow = 1u << lane;
+    far = lane;
+#pragma unroll
+    for (uint32_t o = 0; o < 5; ++o) {
+      const uint32_t f = __shfl_sync(kFull, follow, nx & 31u), l = __shfl_sync(kFull, far, nx & 31u),
+                     x = __shfl_sync(kFull, nx, nx & 31u);
+      if (nx < 32u) { follow |= f; far = l; nx = x; }
+    }
+  };
+  chain();
+  bool entered;
   for (;;) {
+    hop[q] = __shfl_sync(kFull, goes, far) | __shfl_sync(kFull, ex, far) << 11;  // (segment <= 1024, exit <= 2^20)
     __syncthreads();
-    const uint32_t want = q == 0 ? 0u : ex[q - 1];
-    __syncthreads();
-    bool changed = false;
-    const uint32_t old_ent = ent[q], old_ex = ex[q];
-    // mode 0: settled; 1: walk a until it leaves the segment; 2: advance the lower of a (new walk) and
-    // c (old walk) until they meet or both leave
-    int mode = 0;
-    uint32_t a = want, c = old_ent, nx = old_ex;
-    if (want != old_ent) {
-      again = old_ent != s;  // (its path was the first walk's: the tokens until the walks meet are taken here)
-      cnt = 0;
-      from = first.y;
-      if (want >= e) nx = want;
-      else mode = old_ent >= e ? 1 : 2;
+    uint32_t g = 0, at = 0;  // the segment where the chain enters this warp, or a later one's, and its entry
+    while (g < (q & ~31u)) {
+      const uint32_t h = hop[g];
+      g = h & 0x7FFu;
+      at = h >> 11;
     }
-    while (__any_sync(kFull, mode != 0)) {
-      const bool adv_a = mode == 1 || (mode == 2 && a < c);
-      const uint32_t y = warp_step(P, W, adv_a ? a : c, e, mode != 0, t, ta, tc, td);
-      if (t && adv_a && !again) own[cnt++] = tk_pack(ta, tc, td);
-      if (mode == 1) {
-        a = y;
-        if (a >= e) { nx = a; mode = 0; }
-      } else if (mode == 2) {
-        if (adv_a) a = y; else c = y;
-        if (a == c) {
-          nx = old_ex;
-          mode = 0;
-          if (!again) from = tk_after(old, first.y, c);
-        }
-        else if (a >= e && c >= e) { nx = a; mode = 0; }
-      }
-    }
-    if (want != old_ent) {
-      ent[q] = want;
-      if (nx != old_ex) { ex[q] = nx; changed = true; }
-    }
-    if (!__syncthreads_or(changed)) break;
-  }
-  {
-    uint32_t a = ent[q], c = s;
-    if (again) { cnt = 0; from = a == c ? 0u : first.y; }
-    bool on = again && a != c && a < e;
-    while (__any_sync(kFull, on)) {
-      const bool adv_a = a < c;
-      const uint32_t y = warp_step(P, W, adv_a ? a : c, e, on, t, ta, tc, td);
+    bool moved = false;
+    for (;;) {  // (the warp's part of the chain to its end, then the next round)
+      const uint32_t in = __shfl_sync(kFull, follow, g & 31u), prev = in & below;
+      entered = (g & ~31u) == (q & ~31u) && (in >> lane & 1u);
+      const uint32_t px = __shfl_sync(kFull, ex, prev ? 31u - __clz(prev) : 0u), want = prev ? px : at;
+      const bool on = entered && want != ent;
+      if (!__any_sync(kFull, on)) break;
+      // the walk from there, and the first one's positions: its start, its tokens' ends, its exit
+      uint32_t a = want, c = s, k = 0;
+      Known kn;
       if (on) {
-        if (adv_a) {
+        ent = want;
+        cnt = 0;
+      }
+      bool go = on;
+      for (;;) {
+        if (go) {
+          while (c < a && k < first.y) {
+            const uint2 f = old[k++];
+            c = tk_i(f) + tk_m(f);
+            kn.end = c;
+            kn.dist = tk_i(f) <= a ? f.y : 0u;
+          }
+          if (c < a) { c = first.x; kn.end = 0; }
+          go = a != c && a < e;
+        }
+        if (!__any_sync(kFull, go)) break;
+        const uint32_t y = warp_step<true>(P, W, a, e, go, t, ta, tc, td, kn);
+        if (go) {
           a = y;
           if (t) own[cnt++] = tk_pack(ta, tc, td);
-        } else {
-          c = y;
         }
-        on = a != c && (a < e || c < e);
-        if (a == c) from = tk_after(old, first.y, c);
       }
+      bool now = false;
+      if (on) {
+        from = a == c ? k : first.y;
+        const uint32_t x = a == c ? first.x : a;
+        now = x != ex;
+        ex = x;
+      }
+      if (!__any_sync(kFull, now)) break;
+      moved |= now;
+      chain();
     }
+    if (!__syncthreads_or(moved)) break;
   }
+  if (!entered) { cnt = 0; from = first.y; }
   const uint32_t rest = first.y - from;
   const uint32_t incl = warp_incl_scan(cnt + rest);
-  if (lane_id() == 31) wsum[q >> 5] = incl;
+  if (lane == 31) wsum[q >> 5] = incl;
   __syncthreads();
   // the warp's 32 segments' tokens lie one after another in the list: a lane a token, whose segment is the first with
   // a higher inclusive count
-  uint32_t off = warp_sum(lane_id() < (q >> 5) ? wsum[lane_id()] : 0u);
+  uint32_t off = warp_sum(lane < (q >> 5) ? wsum[lane] : 0u);
   uint2* to = A.tk + (size_t)b * tok_cap(A.B) + off;
   const uint32_t all = __shfl_sync(kFull, incl, 31);
-  const uint2* own0 = own - (size_t)lane_id() * slots;
-  const uint2* old0 = old - (size_t)lane_id() * slots;
+  const uint2* own0 = own - (size_t)lane * slots;
+  const uint2* old0 = old - (size_t)lane * slots;
 #pragma unroll 4
   for (uint32_t k0 = 0; k0 < all; k0 += 32) {
-    const uint32_t k = k0 + lane_id();
+    const uint32_t k = k0 + lane;
     uint32_t l = 0;
 #pragma unroll
     for (uint32_t h = 16; h; h >>= 1) l += __shfl_sync(kFull, incl, l + h - 1) <= k ? h : 0u;
