@@ -625,6 +625,7 @@ int write_host(zc_ctx* c, const uint8_t* solid, uint32_t bl, int level, zc_entry
   put_header(out, n, nb64, bl);
   uint64_t at = kArchHdr;
   const uint32_t per_launch = enc_blocks_per_launch(bl);
+  if (int r = reserve_host(c, bl, per_launch, nb, true)) return r;
   struct Chunk {
     uint32_t b0 = 0, k = 0;
     size_t len_at = 0;  // where the chunk's records length lies in its stage's descriptors
@@ -767,6 +768,7 @@ int extract_host(zc_ctx* c, const uint8_t* arch, uint64_t len, uint8_t* out, uin
   uint32_t* d_err = reinterpret_cast<uint32_t*>(X + o_err);
   uint32_t* d_pcrc = reinterpret_cast<uint32_t*>(X + o_pcrc);
   const uint32_t per_launch = dec_blocks_per_launch(bl);
+  if (int r = reserve_host(c, bl, per_launch, nb, false)) return r;
   struct Chunk {
     uint32_t b0 = 0, k = 0;
     uint64_t raw_at = 0, raw_total = 0;

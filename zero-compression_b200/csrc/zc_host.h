@@ -121,6 +121,8 @@ cudaError_t grow(DevBuf& b, size_t bytes);
 cudaError_t grow_host(HostBuf& b, size_t bytes);  // pinned
 // blocks in chunk `i` of a host-pointer call: 64, 128, then 256 MiB (at most per_launch)
 uint32_t host_chunk_blocks(uint32_t block_log, uint32_t per_launch, uint32_t i);
+// scratch for the largest chunk of a host-pointer call over nb blocks
+int reserve_host(zc_ctx* c, uint32_t block_log, uint32_t per_launch, uint32_t nb, bool encode);
 bool bad_block_log(uint32_t bl);
 uint32_t enc_blocks_per_launch(uint32_t block_log);
 uint32_t dec_blocks_per_launch(uint32_t block_log);
