@@ -80,7 +80,9 @@ int zc_compress_batch(zc_ctx *ctx, const uint8_t *in, const uint64_t *in_offs, c
  * Block b is comp_lens[b] bytes at comp + comp_offs[b] with method methods[b] and raw length raw_lens[b].
  * Writes the raw bytes of all blocks back to back into out (sum of raw_lens bytes).
  * crcs_out[b] (may be NULL) gets the CRC-32 of block b's output; block_err[b] (may be NULL) a nonzero
- * code for a damaged block.  Returns ZC_E_DATA when any block is damaged. */
+ * code for a damaged block, or ZC_BLOCK_GAVE_UP.  Returns ZC_E_DATA when any block is damaged, ZC_E_DEVICE when the
+ * decoder gave up on one. */
+#define ZC_BLOCK_GAVE_UP 11u /* a wait inside the decoder ran out: the GPU failed, the block may be good */
 int zc_decompress(zc_ctx *ctx, const uint8_t *comp, const uint64_t *comp_offs, const uint32_t *comp_lens,
                   const uint8_t *methods, const uint32_t *raw_lens, uint32_t nb, uint8_t *out, uint32_t *crcs_out,
                   uint32_t *block_err);
@@ -102,7 +104,8 @@ int zc_compress_device(zc_ctx *ctx, const uint8_t *d_in, const uint64_t *d_in_of
                        void *stream);
 
 /* zc_decompress_device: block b is d_comp_lens[b] bytes at d_comp + d_comp_offs[b]; its raw bytes go to
- * d_out + d_out_offs[b].  d_crcs (may be NULL) gets each output's CRC-32, d_err each block's status.
+ * d_out + d_out_offs[b].  d_crcs (may be NULL) gets each output's CRC-32, d_err each block's status (0; a code for
+ * a damaged block; ZC_BLOCK_GAVE_UP).
  * block_log bounds the raw lengths (a block longer than 2^block_log is damaged). */
 int zc_decompress_device(zc_ctx *ctx, const uint8_t *d_comp, const uint64_t *d_comp_offs, const uint32_t *d_comp_lens,
                          const uint8_t *d_methods, const uint32_t *d_raw_lens, uint32_t nb, uint32_t block_log,

@@ -233,6 +233,7 @@ int decode_device(zc_ctx* c, const uint8_t* d_comp, const uint64_t* d_comp_offs,
   const Shape& sh = c->shape[block_log - zc::kMinBlockLog][level_class(c->level)];
   A.ring_log = sh.ring_log; A.fill_warps = sh.fill_warps; A.fill_words = sh.fill_words;
   A.work = c->work.as<uint32_t>() + 1;
+  A.polls = c->fill_polls;
   zc::launch_decode_fill(A, st, c->stages);
   if (d_crcs && nb) {
     zc::CrcArgs C{};
@@ -250,6 +251,17 @@ int decode_device(zc_ctx* c, const uint8_t* d_comp, const uint64_t* d_comp_offs,
 uint32_t host_chunk_blocks(uint32_t block_log, uint32_t per_launch, uint32_t i) {
   const size_t bytes = (size_t)(i == 0 ? 64 : i == 1 ? 128 : 256) << 20;
   return std::max<uint32_t>(1, std::min<uint32_t>(per_launch, (uint32_t)(bytes >> block_log)));
+}
+
+void note_block(zc_ctx* c, uint64_t block, uint32_t code, int& status) {
+  static_assert(zc::E_GAVE_UP == ZC_BLOCK_GAVE_UP, "the public code");
+  const int s = code == zc::E_GAVE_UP ? ZC_E_DEVICE : ZC_E_DATA;
+  if (s == status || status == ZC_E_DEVICE) return;
+  status = s;
+  char m[128];
+  snprintf(m, sizeof m, s == ZC_E_DATA ? "block %llu damaged (GPU decoder, code %u)" : "the GPU decoder gave up on block %llu (code %u)",
+           (unsigned long long)block, code);
+  c->err = m;
 }
 
 // Before the first chunk: scratch that grew with the chunks would be freed and allocated again between them, each time
@@ -424,6 +436,7 @@ int zc_open(zc_ctx** out, int device) {
   c->device = device;
   c->stages.impl = &c->records;
   if (const char* fa = getenv("ZC_FAIL_AFTER")) c->fail_after = atoll(fa);
+  if (const char* fp = getenv("ZC_FILL_POLLS")) c->fill_polls = (uint32_t)std::min<unsigned long long>(strtoull(fp, nullptr, 10), zc::kFillPolls);
   cudaError_t e = cudaSetDevice(device);
   cudaDeviceProp prop;
   if (e == cudaSuccess) e = cudaGetDeviceProperties(&prop, device);
@@ -779,12 +792,7 @@ int zc_decompress(zc_ctx* c, const uint8_t* comp, const uint64_t* comp_offs, con
     for (uint32_t b = 0; b < q.k; ++b) {
       if (crcs_out) crcs_out[q.b0 + b] = h_crc[b];
       if (block_err) block_err[q.b0 + b] = h_err[b];
-      if (h_err[b] && status == ZC_OK) {
-        status = ZC_E_DATA;
-        char m[128];
-        snprintf(m, sizeof m, "block %u damaged (GPU decoder, code %u)", q.b0 + b, h_err[b]);
-        c->err = m;
-      }
+      if (h_err[b]) note_block(c, q.b0 + b, h_err[b], status);
     }
     return ZC_OK;
   };

@@ -852,8 +852,9 @@ int extract_host(zc_ctx* c, const uint8_t* arch, uint64_t len, uint8_t* out, uin
   char m[512];
   for (uint32_t b = 0; b < nb; ++b) {
     if (err[b]) {
-      snprintf(m, sizeof m, "block %u damaged (GPU decoder, code %u)", b, err[b]);
-      return fail(c, ZC_E_DATA, m);
+      int status = ZC_OK;
+      note_block(c, b, err[b], status);
+      return status;
     }
     if (got[b] != rcrc[b]) {
       snprintf(m, sizeof m, "block %u does not match its checksum: the archive is damaged", b);

@@ -517,7 +517,6 @@ __global__ void __maxnreg__(72) k_dec_fill(DecArgs A) {  // (72 registers: 28 wa
 // (kMultiRing - kMultiAhead) * NW lines back is read from the ring, a farther one from the output itself, which
 // its warp stored before it published its next line).
 constexpr uint32_t kMultiWarps = 16, kMultiRing = 16, kMultiAhead = 4;
-constexpr uint32_t kMultiPoll = 1u << 24;  // polls before a warp gives up
 __host__ __device__ constexpr size_t multi_smem(uint32_t nw) { return nw * kMultiRing * 128; }
 
 // a warp's state, read and published in the order of the CTA's memory: what was stored before it was published is
@@ -591,7 +590,7 @@ __global__ void __launch_bounds__(32 * kMultiWarps, 2) k_dec_fill_multi(DecArgs 
       for (uint32_t k = 0;; ++k) {
         low = __reduce_min_sync(kFull, lane < NW ? (uint32_t)(load_state(&state[lane]) >> 32) : 0xFFFFFFFFu);
         if (ln < low + kMultiAhead * NW) break;
-        if (k > kMultiPoll) { dead = true; break; }
+        if (k > A.polls) { dead = true; break; }
       }
       if (dead) break;
       __syncwarp();
@@ -707,7 +706,7 @@ __global__ void __launch_bounds__(32 * kMultiWarps, 2) k_dec_fill_multi(DecArgs 
           }
         }
         done = __ballot_sync(kFull, !wait);
-        if (k > kMultiPoll) { dead = true; break; }
+        if (done != kFull && k > A.polls) { dead = true; break; }
       }
       if (dead) break;
       __syncwarp();
@@ -722,7 +721,7 @@ __global__ void __launch_bounds__(32 * kMultiWarps, 2) k_dec_fill_multi(DecArgs 
     }
     __syncwarp();
     if (lane == 0) store_state(&state[w], (uint64_t)0x7FFFFFFFu << 32);
-    if (dead && lane == 0) flag(A.err, b, E_TOKEN);
+    if (dead && lane == 0) flag(A.err, b, E_GAVE_UP);
   }
 }
 

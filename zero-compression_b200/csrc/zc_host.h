@@ -111,6 +111,7 @@ struct zc_ctx {
   // the test injector of device failures: ZC_FAIL_AFTER=n at open fails the (n+1)-th codec call
   int64_t fail_after = -1;
   bool lost = false;
+  uint32_t fill_polls = zc::kFillPolls;  // (ZC_FILL_POLLS=n at open: a wait of the decoder's fill runs out sooner)
 };
 
 namespace zch {
@@ -129,6 +130,9 @@ uint32_t dec_blocks_per_launch(uint32_t block_log);
 int check_launch(zc_ctx* c, const char* what);
 // ZC_E_DEVICE when the injector fails this call (or failed an earlier one); counts the call otherwise
 int gate(zc_ctx* c);
+// a decoder status code of a block: `status` becomes ZC_E_DATA for a damaged block, ZC_E_DEVICE (which stays) when the
+// decoder gave up, with the context's message
+void note_block(zc_ctx* c, uint64_t block, uint32_t code, int& status);
 // the slice-by-8 tables and x^(8 * 2^e) powers of the CRC-32 (host copy; the context uploads one)
 void build_crc_tables(zc::CrcTables& T);
 // uniform blocks: block b of an n-byte span starts at b * B and holds min(B, n - b * B) bytes

@@ -22,9 +22,9 @@ constexpr uint32_t kRecHdr = 16;           // block record header in the archive
 __host__ __device__ inline uint32_t tok_cap(uint32_t B) { return B / 4 + 16; }
 __host__ __device__ inline uint32_t ext_cap(uint32_t B) { return B / 5 + 64; }
 
-// decoder status codes per block (0 = good)
+// decoder status codes per block (0 = good; E_GAVE_UP: a wait of the fill ran out, which says nothing of the block)
 enum : uint32_t { E_HDR = 1, E_COUNTS = 2, E_STREAM = 3, E_TABLE = 4, E_LANE = 5, E_TOKEN = 6, E_METHOD = 7,
-                  E_STORED = 8, E_RAWLEN = 9, E_CRC = 10 };
+                  E_STORED = 8, E_RAWLEN = 9, E_CRC = 10, E_GAVE_UP = 11 };
 
 // ---- little-endian byte access
 __device__ __forceinline__ uint32_t ld32(const uint8_t* p) {

@@ -50,10 +50,12 @@ struct DecArgs {
   // fill_words output words a lane a round (1, 2 or 4)
   uint32_t ring_log, fill_warps, fill_words;
   uint32_t* work;             // the fill's device work counter (zeroed by the launcher)
+  uint32_t polls;             // several warps a block: polls of another warp's progress before a warp gives up
 };
 
 __host__ __device__ inline uint32_t line_cap(uint32_t B) { return B / 128 + 2; }
 
+constexpr uint32_t kFillPolls = 1u << 24;
 constexpr uint32_t kMinFillRingLog = 11, kMaxFillRingLog = 15, kMaxFillWarps = 8;
 constexpr size_t kMaxFillSmem = 227 * 1024;
 size_t fill_smem_bytes(uint32_t ring_log, uint32_t warps, uint32_t words);

@@ -144,6 +144,7 @@ extern "C" int zc_decompress_noalloc(const uint8_t* d_comp, const uint64_t* d_co
   A.ring_log = 12;
   A.fill_warps = 4;
   A.fill_words = 1;
+  A.polls = zc::kFillPolls;
   zc::Stages stages;  // (no timing; nothing to record)
   zc::launch_decode_fill(A, st, stages);
   if (d_crcs) {

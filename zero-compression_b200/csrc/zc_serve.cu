@@ -345,7 +345,8 @@ void complete_batch(zc_server* S, Slot& L) {
       Job* J = L.take[i].first;
       const uint32_t b = L.take[i].second;
       if (J->j.out_crcs) J->j.out_crcs[b] = v.r_crc[i];
-      if (v.r_err[i]) J->status = ZC_E_DATA;
+      if (J->status == ZC_E_DEVICE) continue;
+      if (v.r_err[i]) J->status = v.r_err[i] == ZC_BLOCK_GAVE_UP ? ZC_E_DEVICE : ZC_E_DATA;
       else if (J->j.kind == ZC_JOB_TEST && J->j.crcs_expected && J->j.crcs_expected[b] != v.r_crc[i]) J->status = ZC_E_DATA;
     }
   }
