@@ -706,7 +706,7 @@ __global__ void __launch_bounds__(32 * kMultiWarps, 2) k_dec_fill_multi(DecArgs 
           }
         }
         done = __ballot_sync(kFull, !wait);
-        if (done != kFull && k > A.polls) { dead = true; break; }
+        if (k > A.polls) { dead = true; break; }
       }
       if (dead) break;
       __syncwarp();
