@@ -147,20 +147,20 @@ int ensure_dec(zc_ctx* c, uint32_t nb, uint32_t block_log) {
 
 bool bad_block_log(uint32_t bl) { return bl < zc::kMinBlockLog || bl > zc::kMaxBlockLog; }
 
-// blocks per encoder launch: 1 GiB of input (about 25 GiB of scratch: several waves of every stage on
+// blocks per encoder launch: 1 GiB of input (about 27 GiB of scratch: several waves of every stage on
 // 148 SMs), and the grid's y limit
 uint32_t enc_blocks_per_launch(uint32_t block_log) {
   return (uint32_t)std::min<size_t>(((size_t)1 << 30) >> block_log, 65535);
 }
 // blocks per decoder launch: 4 GiB of output (the fill runs one warp per block, so large launches keep
-// every SM busy; about 6 bytes of scratch per output byte)
+// every SM busy; about 5 bytes of scratch per output byte)
 uint32_t dec_blocks_per_launch(uint32_t block_log) {
   return (uint32_t)std::min<size_t>(((size_t)4 << 30) >> block_log, 1u << 20);
 }
 
-// segments a block is parsed in: 512 bytes each, a lane's walk; 256 in launches whose 256-byte segments would not
-// keep every SM's 1024 walks busy eight times over, so that the walks end sooner.  Shorter ones cost more re-walked
-// steps.  ms of walks and parse: 1 GiB of lz_mix, block 18, in 1024 / 512 / 256 bytes 11.7 / 11.0 / 11.6; 571 blocks of
+// segments a block is parsed in, a lane's walk each: 512 bytes, or 256 in launches whose 256-byte segments would not
+// keep every SM's 1024 walks busy eight times over, so that the walks end sooner; but 256 to 1024 segments a block, so
+// always 256 bytes at block 16, 512 at 19 and 1024 at 20.  Shorter ones cost more re-walked steps.  ms of walks and parse: 1 GiB of lz_mix, block 18, in 1024 / 512 / 256 bytes 11.7 / 11.0 / 11.6; 571 blocks of
 // files 6.0 / 3.0 / 2.5; 256 blocks of text 5.4 / 2.2 / 2.0.
 uint32_t enc_segments(uint32_t nb, uint32_t block_log) {
   const uint32_t bytes = ((uint64_t)nb << block_log) < 8ull * 148 * 1024 * 256 ? 256 : 512;
@@ -197,7 +197,7 @@ int encode_device(zc_ctx* c, const uint8_t* d_in, const uint64_t* d_off, const u
   if (int r = ensure_enc(c, nb, block_log)) return r;
   zc::EncArgs A{};
   A.in = d_in; A.in_off = d_off; A.in_len = d_len; A.nb = nb;
-  A.B = 1u << block_log; A.block_log = block_log; A.depth = depth_for_level(level);
+  A.B = 1u << block_log; A.depth = depth_for_level(level);
   A.tmp_e = c->e_tmp.as<uint32_t>(); A.tmp_d = c->e_tmp_d.as<uint8_t>(); A.srt = c->e_srt.as<uint32_t>();
   A.minfo = c->e_minfo.as<uint32_t>(); A.scnt = c->e_scnt.as<uint32_t>();
   A.tk_seg = c->e_tk_seg.as<uint2>(); A.seg_exit = c->e_seg.as<uint2>();

@@ -6,8 +6,8 @@
 // chain is exactly the run of i's predecessors in a stable sort of the positions by hash, so:
 //
 //   k_sort_*       stable two-pass LSD radix sort of each block's positions by hash (8 + 8 bits), a
-//                  CTA per 4096-position tile: digit counts, per-block scan, ranked scatter (warp
-//                  match_any ranks, the tile reordered in shared memory, digit runs written together).
+//                  CTA per 4096-position tile: digit counts, per-block scan, ranked scatter (ranks by shared
+//                  masks or match_any, the tile reordered in shared memory, digit runs written together).
 //                  An entry is one word: the position and 12 more bits of its 4 bytes' product
 //   k_enc_chain    per sorted entry: does its chain hold an entry with the same 12 bits (a candidate of 4
 //                  equal bytes)?  No: no match.  Yes: the position is marked with its place in the order
@@ -89,11 +89,10 @@ __device__ __forceinline__ uint32_t lcp16(const uint4& a, const uint4& b) {
 // Two stable LSD passes over the 16-bit hash (low byte, then high byte), each as three kernels over
 // tiles of 4096 positions, every tile its own CTA: k_sort_count (the tile's digit counts), k_sort_scan
 // (per block: each tile's start for each digit, digit-major), k_sort_scatter (ranks the tile's entries
-// per digit in order with warp match_any, reorders the tile by digit in shared memory, and writes each
-// digit's run to its place).  Pass 0 reads positions in order and hashes them; it writes each entry's word
-// and, in a byte array, its digit of pass 1, which reads both and writes words alone: 16 bytes moved a
-// position in all (22 with the hash beside the position in both passes).  The counts array holds
-// tiles_per_block(B) * 256 words per block.
+// per digit in order, reorders the tile by digit in shared memory, and writes each digit's run to its place).
+// Pass 0 reads positions in order and hashes them; it writes each entry's word and, in a byte array, its digit of
+// pass 1, which reads both and writes words alone: 16 bytes moved a position in all (22 with the hash beside the
+// position in both passes).  The counts array holds tiles_per_block(B) * 256 words per block.
 constexpr uint32_t kSortTile = 4096, kSortThreads = 512, kSortPer = kSortTile / kSortThreads;
 constexpr int kCrowd = 3;
 

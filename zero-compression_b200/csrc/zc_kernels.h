@@ -80,7 +80,7 @@ struct EncArgs {
   const uint8_t* in;          // block b: in_len[b] bytes at in + in_off[b]; 16-aligned, >= 64 readable bytes after the last
   const uint64_t* in_off;
   const uint32_t* in_len;
-  uint32_t nb, B, block_log;
+  uint32_t nb, B;
   int depth;                  // hash chain steps (8 / 32 / 256)
   // scratch, per block slot (capacity B positions)
   uint32_t *tmp_e, *srt, *minfo;  // sort entries after pass 0 and in order; match records
@@ -138,7 +138,7 @@ __host__ __device__ inline uint32_t seg_bytes(uint32_t n, uint32_t nseg) {
 __host__ __device__ inline uint32_t seg_tok_cap(uint32_t B) { return B / 4 + 2 * kMaxSegs; }
 
 void launch_encode(const EncArgs& A, const CrcArgs& crc_in, cudaStream_t st, Stages& S);
-cudaError_t prepare_kernels();
-cudaError_t prepare_fill();  // per-kernel attributes (the sort's shared memory), the device current
+cudaError_t prepare_kernels();  // per-kernel attributes (dynamic shared memory), the device current
+cudaError_t prepare_fill();     // (the fill's part)
 
 }  // namespace zc
