@@ -33,7 +33,7 @@ sys.path.insert(0, os.path.join(ROOT, "zero-compression_b200"))
 METRIC = "compress/decompress GB/s on 1 B200, bit-exact round-trip; served p50/p99 latency"
 # dram__bytes_read.sum + dram__bytes_write.sum per raw byte of one launch (block 18, level 5 lz_mix), from
 # the ncu capture summarised in profiles/kernels_lz240m_b18_l5.md (k_sort_scatter: the mean of its two passes)
-DRAM_BYTES_PER_RAW_BYTE = {"k_enc_walk": 15.74, "k_sort_scatter": 7.96, "k_enc_chain": 7.86, "k_enc_parse": 1.34,
+DRAM_BYTES_PER_RAW_BYTE = {"k_enc_walk": 15.86, "k_sort_scatter": 8.09, "k_enc_chain": 7.86, "k_enc_parse": 0.95,
                            "k_dec_fill": 1.518, "k_dec_tokens": 0.109, "k_dec_streams": 0.182}
 GB = 1e9
 
