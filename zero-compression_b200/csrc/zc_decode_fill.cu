@@ -105,6 +105,13 @@ __device__ __forceinline__ uint32_t bits_at(const uint8_t* p, uint32_t at, uint3
 // gs - 1 - r (the last three offsets before the group, nearest first), or the initial 1, 4, 8 when r >= gs.  The group
 // counts' scan sets a bit for each group's first token; the maximum of those up to a token is its gs.  A token named
 // in an earlier tile is resolved; within the tile, by pointer jumping in shared memory (a chain halves each round).
+//
+// Many near copies and hardly a literal make one long chain of the output, which several warps only hand to one another,
+// 0.85 us a hop: such a block's line table says in its last row that one warp is to fill it.  Two values at random, ms
+// shared / by one warp: at level 1, 13 near copies a 128-byte line and 3.2 hops, one block of 256 KiB 5.53 / 2.65, 256
+// blocks 7.42 / 3.01; at level 5, 4 a line and one hop, 1.74 / 1.83 and 2.44 / 2.13.  Four symbols at level 1, 2.4 a
+// line, 0.92 / 2.01 and 1.36 / 2.51.  So the line lies at 8.
+constexpr uint32_t kNearOffset = 128, kNearBytes = 16;  // more than one copy from at most 128 back in 16 bytes
 constexpr uint32_t kTokThreads = 512, kTokPer = 4, kTokTile = kTokThreads * kTokPer;
 
 __global__ void __launch_bounds__(kTokThreads, 2) k_dec_tokens(DecArgs A) {
@@ -115,6 +122,7 @@ __global__ void __launch_bounds__(kTokThreads, 2) k_dec_tokens(DecArgs A) {
   __shared__ uint32_t maxs[2][NW];
   __shared__ uint32_t gbits[(1u << kMaxBlockLog) / 4 / 32 + 1];  // a bit for each group's first token
   __shared__ __align__(16) uint32_t jump[kTokTile];
+  __shared__ uint32_t nears;
   const DecMeta m = A.meta[b];
   const uint32_t raw = A.raw_len[b], B = A.B;
   const size_t TC = tok_cap(B), EC = ext_cap(B);
@@ -134,6 +142,7 @@ __global__ void __launch_bounds__(kTokThreads, 2) k_dec_tokens(DecArgs A) {
   if (line)
     for (uint32_t k = tid; k < (raw + al + 127u) >> 7; k += kTokThreads) line[k] = make_uint2(0, 0);
   for (uint32_t k = tid; k < (m.nt >> 5) + 1; k += kTokThreads) gbits[k] = 0;
+  if (tid == 0) nears = 0;
   __syncthreads();
   // ---- the groups' first tokens
   {
@@ -161,7 +170,7 @@ __global__ void __launch_bounds__(kTokThreads, 2) k_dec_tokens(DecArgs A) {
   }
   __syncthreads();
   // ---- the tokens
-  uint32_t ei = 0, bp = 0, op = 0, li = 0, carry = 0;
+  uint32_t ei = 0, bp = 0, op = 0, li = 0, carry = 0, near = 0;
   uint32_t ntv = 0, nsv = 0;  // the next tile's tokens and symbols
   if (kTokPer * tid < m.nt) { ntv = tok[tid]; nsv = sym[tid]; }
   for (uint32_t t0 = 0; t0 < m.nt; t0 += kTokTile) {
@@ -247,12 +256,17 @@ __global__ void __launch_bounds__(kTokThreads, 2) k_dec_tokens(DecArgs A) {
     if (n) {
 #pragma unroll
       for (uint32_t j = 0; j < kTokPer; ++j)
-        if (j < n && (D[j] == 0 || D[j] > ms[j])) bad = true;
+        if (j < n) {
+          if (D[j] == 0 || D[j] > ms[j]) bad = true;
+          near += D[j] <= kNearOffset;
+        }
       *reinterpret_cast<uint4*>(Tp + t) = make_uint4(row[0].x, row[0].y, row[1].x, row[1].y);
       *reinterpret_cast<uint4*>(Tp + t + 2) = make_uint4(row[2].x, row[2].y, row[3].x, row[3].y);
       *reinterpret_cast<uint4*>(Td + t) = make_uint4(D[0], D[1], D[2], D[3]);
     }
   }
+  near = warp_sum(near);
+  if (lane_id() == 0) atomicAdd(&nears, near);
   const int any_bad = __syncthreads_or(bad);
   if (tid == 0) {
     Tp[m.nt] = tok_row(op, raw - op, li);  // token nt: the literal tail
@@ -260,6 +274,7 @@ __global__ void __launch_bounds__(kTokThreads, 2) k_dec_tokens(DecArgs A) {
     if (any_bad || op + (m.nl - li) != raw) flag(A.err, b, E_TOKEN);
     A.meta[b].op_total = op;
     A.meta[b].li_total = li;
+    if (line) line[line_cap(B) - 1].x = nears > raw / kNearBytes && m.nl <= raw / kNearBytes;
   }
   if (line && !any_bad && op < raw) {  // the literal tail's lines and start (a line 0 that starts before the output: token 0)
     for (uint32_t k = ((op + al + 127u) >> 7) + tid; k < (raw + al + 127u) >> 7; k += kTokThreads) line[k].x = m.nt;
@@ -322,9 +337,9 @@ __device__ inline void copy_bytes(uint8_t* d, const uint8_t* s, uint32_t n, uint
 // D) (src/codec2.h:194-197: an overlapping match repeats its D bytes before it), the quotient from a
 // multiply-high by the reciprocal, exact to one step, which a compare corrects.
 template <uint32_t WPL, uint32_t TR>
-__device__ __forceinline__ void fill_block(const DecArgs& A, uint32_t b, FillTable<TR>& T, uint8_t* ring,
+__device__ __forceinline__ void fill_block(const DecArgs& A, uint32_t b, FillTable<TR>& T, uint8_t* ring, uint32_t R,
                                            uint16_t* stage) {
-  const uint32_t R = 1u << A.ring_log, rmask = R - 1u;
+  const uint32_t rmask = R - 1u;
   const uint32_t lane = lane_id();
   const uint32_t raw = A.raw_len[b], method = A.method[b], clen = A.comp_len[b], B = A.B;
   uint8_t* o = A.out + A.out_off[b];
@@ -497,7 +512,7 @@ __global__ void __maxnreg__(72) k_dec_fill(DecArgs A) {  // (72 registers: 28 wa
     if (lane_id() == 0) b = atomicAdd(A.work, 1u);
     b = __shfl_sync(kFull, b, 0);
     if (b >= A.nb) break;
-    fill_block<WPL>(A, b, T, ring, stage);
+    fill_block<WPL>(A, b, T, ring, R, stage);
     __syncwarp();
   }
 }
@@ -530,10 +545,19 @@ __device__ __forceinline__ void store_state(uint64_t* p, uint64_t v) {
   asm volatile("st.release.cta.shared.u64 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(p)), "l"(v) : "memory");
 }
 
+// a block by one warp, out of line: the shared form's registers stay its own
+constexpr uint32_t kAloneRing = 4096;
+static_assert(fill_table_bytes(1) + kAloneRing + fill_stage_bytes(1) <= 4 * kMultiRing * 128, "what four warps have");
+__device__ __noinline__ void fill_alone(const DecArgs& A, uint32_t b, uint8_t* sm) {
+  uint8_t* ring = sm + fill_table_bytes(1);
+  fill_block<1>(A, b, *reinterpret_cast<FillTable<fill_rows(1)>*>(sm), ring, kAloneRing,
+                reinterpret_cast<uint16_t*>(ring + kAloneRing));
+}
+
 // (Hasty: the polls' limit is A.polls, lowered for a test; read from there in every poll it cost all blocks 1 to 2 %, two
 // values at random 22.1 -> 22.5 ms for 1 MiB, records 8.66 -> 8.86)
 template <bool Hasty>
-__global__ void __launch_bounds__(32 * kMultiWarps, 2) k_dec_fill_multi(DecArgs A) {
+__global__ void __launch_bounds__(32 * kMultiWarps, 2) k_dec_fill_multi(const __grid_constant__ DecArgs A) {
   extern __shared__ __align__(16) uint8_t fsm[];
   __shared__ uint32_t next;
   __shared__ uint64_t state[kMultiWarps];
@@ -549,6 +573,7 @@ __global__ void __launch_bounds__(32 * kMultiWarps, 2) k_dec_fill_multi(DecArgs 
     const uint32_t b = next;
     if (b >= A.nb) break;
     const uint32_t raw = A.raw_len[b], method = A.method[b], clen = A.comp_len[b], B = A.B;
+    const uint32_t alone = A.line[(size_t)(b + 1) * line_cap(B) - 1].x;  // (k_dec_tokens' choice, of a good block)
     uint8_t* o = A.out + A.out_off[b];
     if (raw > B || method > 1 || (method == 0 && clen != raw)) {
       if (threadIdx.x == 0) flag(A.err, b, raw > B ? E_RAWLEN : method > 1 ? E_METHOD : E_STORED);
@@ -559,6 +584,10 @@ __global__ void __launch_bounds__(32 * kMultiWarps, 2) k_dec_fill_multi(DecArgs 
       continue;
     }
     if (A.err[b]) continue;
+    if (alone) {
+      if (w == 0) fill_alone(A, b, fsm);
+      continue;
+    }
     const DecMeta& m = A.meta[b];
     const size_t TC = tok_cap(B);
     const uint8_t* lit = A.s_lit + (size_t)b * B;

@@ -44,7 +44,7 @@ struct DecArgs {
   uint2* tk_pos;
   uint32_t* tk_d;
   // per 128-byte line of the output address (line_cap(B) per block): the token that holds its first byte, and a bit
-  // for each of its words in which another token starts
+  // for each of its words in which another token starts; the last row says whether one warp fills the block
   uint2* line;
   // the fill's shape: a ring of 2^ring_log recent output bytes per warp, fill_warps warps (blocks) per CTA,
   // fill_words output words a lane a round (1, 2 or 4)
