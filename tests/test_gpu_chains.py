@@ -23,11 +23,24 @@ def records(codec, raw, block_log):
     return [(int(m[b]), pay[int(at[b]): int(at[b]) + int(n[b])] if m[b] else raw[b]) for b in range(len(raw))], crc
 
 
+def chain(kind, n, r):
+    if kind == "bits":
+        return r.integers(0, 2, n, dtype=np.uint8)
+    if kind == "counter":
+        return (np.arange(n // 8 + 1, dtype=np.uint64) * 24 + 0x7F0000000000).view(np.uint8)[:n]
+    a, b = np.array([0], np.uint8), np.array([0, 1], np.uint8)
+    while b.size < n:
+        a, b = b, np.concatenate([b, a])
+    return b[:n].copy()
+
+
 # ms of a call when every block had one warp (B200)
-@pytest.mark.parametrize("block_log,nb,limit", [(16, 1, 0.92), (18, 1, 3.58), (18, 256, 4.13), (20, 1, 14.1), (20, 64, 15.8)])
-def test_time(codec, block_log, nb, limit):
+@pytest.mark.parametrize("kind,block_log,nb,limit", [
+    ("bits", 16, 1, 0.92), ("bits", 18, 1, 3.58), ("bits", 18, 256, 4.13), ("bits", 20, 1, 14.1), ("bits", 20, 64, 15.8),
+    ("counter", 16, 1, 2.53), ("counter", 18, 1, 9.99), ("counter", 18, 256, 10.6), ("counter", 20, 64, 41.7)])
+def test_time(codec, kind, block_log, nb, limit):
     import torch
-    raw = [np.random.default_rng(7).integers(0, 2, 1 << block_log, dtype=np.uint8)]
+    raw = [chain(kind, 1 << block_log, np.random.default_rng(7))]
     launch = device_launch(raw, *records(codec, raw, block_log), nb, 0)
     check(codec, launch, block_log)
     args, out, out_at = launch[:3]
@@ -46,9 +59,15 @@ def test_time(codec, block_log, nb, limit):
 @pytest.mark.parametrize("nb", [1, 7, 296, 592, 888, 889])
 @pytest.mark.parametrize("block_log", [16, 18])
 def test_bytes(codec, block_log, nb):
-    """From no literal to one byte in eight, one to six bits a symbol, whole and short: both sides of the rule's lines."""
+    """From no literal to one byte in eight, one to six bits a symbol, whole and short; chains between text and noise."""
+    import datagen as G
     r = np.random.default_rng(nb)
     raw = []
+    for n in (1 << block_log, (1 << block_log) - 1234):
+        for kind in ("bits", "fibonacci", "counter"):
+            for piece in (9000, 20000, 70000):
+                parts = [chain(kind, piece, r), G.text_mix(piece, nb), chain(kind, 2 * piece + 77, r), G.random_bytes(piece // 3, nb)]
+                raw.append(np.resize(np.concatenate(parts), n))
     for n in (1 << block_log, (1 << block_log) - 77, 5000, 300, 33):
         for share in (0, 40, 18, 16, 14, 8):
             for symbols in (2, 4, 16, 64):

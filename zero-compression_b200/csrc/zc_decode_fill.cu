@@ -106,11 +106,13 @@ __device__ __forceinline__ uint32_t bits_at(const uint8_t* p, uint32_t at, uint3
 // counts' scan sets a bit for each group's first token; the maximum of those up to a token is its gs.  A token named
 // in an earlier tile is resolved; within the tile, by pointer jumping in shared memory (a chain halves each round).
 //
-// Many near copies and hardly a literal make one long chain of the output, which several warps only hand to one another,
-// 0.85 us a hop: such a block's line table says in its last row that one warp is to fill it.  Two values at random, ms
-// shared / by one warp: at level 1, 13 near copies a 128-byte line and 3.2 hops, one block of 256 KiB 5.53 / 2.65, 256
-// blocks 7.42 / 3.01; at level 5, 4 a line and one hop, 1.74 / 1.83 and 2.44 / 2.13.  Four symbols at level 1, 2.4 a
-// line, 0.92 / 2.01 and 1.36 / 2.51.  So the line lies at 8.
+// Many near copies make one long chain of the output if hardly a literal or hardly a farther copy ends it.  Several warps
+// only hand such a chain's words to one another, 0.4 to 0.9 us a hop, so the block's line table says in its last row that
+// one warp is to fill it.  ms shared / by one warp, one block of 256 KiB and 256: two values at random at level 1, 13
+// near copies a 128-byte line and 3.2 hops, 5.53 / 2.65 and 7.42 / 3.01, at level 5, 4 a line and one hop, 1.74 / 1.83 and
+// 2.44 / 2.13; four symbols at level 1, 2.4 a line, 0.92 / 2.01 and 1.36 / 2.51: so the line lies at 8.  Counters 8
+// bytes apart at level 1, 16 a line, none farther and 14 hops, 10.5 / 8.0 and 16.4 / 8.5; at level 5, where one in twelve is
+// farther and there are 0.6 hops, 0.96 / 5.5 and 1.55 / 5.9.
 constexpr uint32_t kNearOffset = 128, kNearBytes = 16;  // more than one copy from at most 128 back in 16 bytes
 constexpr uint32_t kTokThreads = 512, kTokPer = 4, kTokTile = kTokThreads * kTokPer;
 
@@ -274,7 +276,8 @@ __global__ void __launch_bounds__(kTokThreads, 2) k_dec_tokens(DecArgs A) {
     if (any_bad || op + (m.nl - li) != raw) flag(A.err, b, E_TOKEN);
     A.meta[b].op_total = op;
     A.meta[b].li_total = li;
-    if (line) line[line_cap(B) - 1].x = nears > raw / kNearBytes && m.nl <= raw / kNearBytes;
+    if (line)
+      line[line_cap(B) - 1].x = nears > raw / kNearBytes && (m.nl <= raw / kNearBytes || m.nt - nears <= nears / 64);
   }
   if (line && !any_bad && op < raw) {  // the literal tail's lines and start (a line 0 that starts before the output: token 0)
     for (uint32_t k = ((op + al + 127u) >> 7) + tid; k < (raw + al + 127u) >> 7; k += kTokThreads) line[k].x = m.nt;
