@@ -476,19 +476,21 @@ __device__ __forceinline__ void finish_lists(const ParseBlock& P, Finish& W, uin
   }
   __syncwarp();
   // The rest are extended, up to 32 at a time, 32 lanes / their number each and 16 bytes a lane a step, until none is
-  // left.  Of more than 32, those that can still win, the first one of each request: one that is nearer than its request's
-  // best wins with the best's length, a farther one only with more, so it is dropped when its byte there differs.
-  // (Eight at a time, four lanes each: the walks took 10.3 ms for 1 GiB of lz_mix against 9.2, 7.6 against 6.6 for
-  // 256 MiB at depth 256.  Four lanes each at most: the whole call 27.1 ms against 26.2, and 25 us for one match of 4096
+  // left.  Of more than 32, those that can still win, of each request the first one, then the next two, four and so on:
+  // one that is nearer than its request's best wins with the best's length, a farther one only with more, so it is dropped
+  // when its byte there differs.  (Always the first one alone: where lengths rise with the distance, as in runs of one value
+  // among few others, a request took a turn for each of its candidates.  Walks, ms, 64 MiB with a byte in 100 not zero,
+  // block 16, depth 256, 13.3 / 4.5; 256 MiB of lz_mix at block 20, depth 256, 6.6 / 5.5.)
+  // (Eight at a time, four lanes each: the walks took 10.3 ms for 1 GiB of lz_mix against 9.2.  Four lanes each at most: the whole call 27.1 ms against 26.2, and 25 us for one match of 4096
   // bytes.)
   // In runs and periods the matches of all the warp's requests go on to the longest length or the run's end, at one
   // distance.  So a candidate at the distance of the one after it is compared only up to that one's position: it
   // ends where that one ends.  The parse's walks also bring what they know of the bytes before them (Known), and where
   // two candidates of a request go on after kPause bytes, one of each request is extended at a time from there on.
-  // Walks and parse, ms, before all this / now: 256 MiB of one value at block 18 22.2 / 3.7, at block 20 and depth 256
-  // 19.1 / 3.1; of a period of 5000 bytes 61.1 / 8.4 and 69.7 / 6.6; one such block of 1 MiB 30.1 / 2.1.
-  while (n3) {
-    uint32_t m = 0, nb = 0, carry = 32;  // kept ones, those of this turn, the last kept one's slot
+  // Walks and parse, ms, before all this / now: 256 MiB of one value at block 18 22.2 / 3.8, at block 20 and depth 256
+  // 19.1 / 3.2; of a period of 5000 bytes 61.1 / 8.6 and 69.7 / 6.8; one such block of 1 MiB 30.1 / 2.2.
+  for (uint32_t quota = 1; n3; quota = min(2 * quota, kBatch)) {
+    uint32_t m = 0, nb = 0, carry = 32, run = 0;  // kept ones, those of this turn, the last kept one's slot and its count
     const uint32_t* batch = W.batch;
     const bool few = n3 <= kBatch && !one;
     if (few) {  // (so few that all are extended)
@@ -507,16 +509,20 @@ __device__ __forceinline__ void finish_lists(const ParseBlock& P, Finish& W, uin
       const unsigned km = __ballot_sync(kFull, keep);
       const unsigned pm = km & below;
       const uint32_t pi = __shfl_sync(kFull, i, pm ? 31u - __clz(pm) : 0u);
-      const bool first = keep && (pm ? pi : carry) != i;
-      const unsigned fm = __ballot_sync(kFull, first);
+      const unsigned hm = __ballot_sync(kFull, keep && (pm ? pi : carry) != i) & (below | 1u << lane);  // first ones so far
+      const uint32_t rank = hm ? __popc(pm >> (31u - __clz(hm))) : run + __popc(pm);  // among its request's
+      const unsigned fm = __ballot_sync(kFull, keep && rank < quota);
       const uint32_t fk = nb + __popc(fm & below);
-      const bool sel = first && fk < kBatch;
+      const bool sel = keep && rank < quota && fk < kBatch;
       if (sel) W.batch[fk] = c;
       const unsigned rm = km & ~__ballot_sync(kFull, sel);
       if (rm >> lane & 1u) far[m + __popc(rm & below)] = c;
       m += (uint32_t)__popc(rm);
       nb = min(kBatch, nb + (uint32_t)__popc(fm));
-      if (km) carry = __shfl_sync(kFull, i, 31u - __clz(km));
+      if (km) {
+        carry = __shfl_sync(kFull, i, 31u - __clz(km));
+        run = __shfl_sync(kFull, rank, 31u - __clz(km)) + 1u;
+      }
       __syncwarp();
     }
     n3 = m;
@@ -782,7 +788,7 @@ __device__ __forceinline__ uint32_t warp_step(const ParseBlock& P, Finish& W, ui
 // Text in 512-byte segments is bound by L2 misses: 32 warps an SM are then in 296 blocks' candidate orders, 1.25 MiB
 // each, 103 bytes read from memory a byte of input; lz_mix has few candidates and does not mind.
 // The walks' own loads live on the L1, which has what 32 warps' lists leave of an SM's 256 KiB: two warps a CTA and
-// 2688 bytes of lists a warp leave 128 KiB (1 GiB of lz_mix 8.7 ms, 64 MiB of text 1.62, 256 MiB at depth 256 6.5);
+// 2688 bytes of lists a warp leave 128 KiB (1 GiB of lz_mix 8.7 ms, 64 MiB of text 1.62, 256 MiB at depth 256, then, 6.5);
 // one, and 3584 bytes, left 64 (8.8, 1.68, 6.8).  40 or 48 warps in as many registers as that leaves: 8.9 and 9.4, text
 // 1.9 and 2.5.
 __global__ void __launch_bounds__(64, 16) k_enc_walk(EncArgs A, uint32_t walks) {
@@ -816,7 +822,7 @@ __global__ void __launch_bounds__(64, 16) k_enc_walk(EncArgs A, uint32_t walks) 
 // the true entry for the tokens: 2.26 ms per GiB of lz_mix at block 18, 0.52 for 64 MiB of text; now 0.35 and 0.17.)
 // Where a match covers many segments, as in runs and periods, whose walks never meet, a step of the chain settles a
 // match.  (Exits handed from each segment to the next, skipped ones among them, settled one segment a round: one block
-// of 1 MiB of one value 6.5 ms, now 1.0; of 256 KiB 2.0, now 0.28.)
+// of 1 MiB of one value 6.5 ms, now 1.1; of 256 KiB 2.0, now 0.29.)
 template <uint32_t T>
 __global__ void __launch_bounds__(T, 1024 / T) k_enc_parse(EncArgs A) {
   const uint32_t b = blockIdx.x, q = threadIdx.x, lane = lane_id(), below = (1u << lane) - 1u;
