@@ -481,12 +481,12 @@ __device__ __forceinline__ void finish_lists(const ParseBlock& P, Finish& W, uin
   // when its byte there differs.  (Always the first one alone: where lengths rise with the distance, as in runs of one value
   // among few others, a request took a turn for each of its candidates.  Walks, ms, 64 MiB with a byte in 100 not zero,
   // block 16, depth 256, 13.3 / 4.5; 256 MiB of lz_mix at block 20, depth 256, 6.6 / 5.5.)
-  // (Eight at a time, four lanes each: the walks took 10.3 ms for 1 GiB of lz_mix against 9.2.  Four lanes each at most: the whole call 27.1 ms against 26.2, and 25 us for one match of 4096
-  // bytes.)
+  // (Eight at a time, four lanes each: the walks took 10.3 ms for 1 GiB of lz_mix against 9.2.  Four lanes each at most: the
+  // whole call 27.1 ms against 26.2, and 25 us for one match of 4096 bytes.)
   // In runs and periods the matches of all the warp's requests go on to the longest length or the run's end, at one
   // distance.  So a candidate at the distance of the one after it is compared only up to that one's position: it
   // ends where that one ends.  The parse's walks also bring what they know of the bytes before them (Known), and where
-  // two candidates of a request go on after kPause bytes, one of each request is extended at a time from there on.
+  // two candidates of a request go on after kPause bytes, the turns begin with one of each request again.
   // Walks and parse, ms, before all this / now: 256 MiB of one value at block 18 22.2 / 3.8, at block 20 and depth 256
   // 19.1 / 3.2; of a period of 5000 bytes 61.1 / 8.6 and 69.7 / 6.8; one such block of 1 MiB 30.1 / 2.2.
   for (uint32_t quota = 1; n3; quota = min(2 * quota, kBatch)) {

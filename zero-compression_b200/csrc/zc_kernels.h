@@ -129,8 +129,11 @@ __host__ __device__ inline uint64_t lane_base(uint32_t B, uint32_t s) {
 __host__ __device__ inline uint64_t lanes_per_block(uint32_t B) { return lane_base(B, 5); }
 __host__ __device__ inline uint32_t bits_cap(uint32_t B) { return 5 * B / 8 + 64; }
 // the parse's segments: ceil(n / nseg) bytes each, at least kMinSeg; their token slots per block: a token takes at
-// least 4 bytes, so a segment of S bytes has at most S / 4 + 1, S / 4 + 2 slots are kept for it, and nseg <= 1024
-constexpr uint32_t kMaxSegs = 1024, kMinSeg = 64;
+// least 4 bytes, so a segment of S bytes has at most S / 4 + 1, S / 4 + 2 slots are kept for it, and nseg <= 1024.  Short
+// blocks end sooner in short segments, whose walks meet the right ones later; compress at block 18, level 5, ms, with at
+// least 128 / 64 / 32 / 16 bytes: 600 blocks of 3000 bytes of text 0.59 / 0.51 / 0.48 / 0.46, of one value 0.31 / 0.34 /
+// 0.37 / 0.40; one text block of 1000 bytes 0.128 / 0.117 / 0.109 / 0.103, of 16 000 0.175 / 0.156 / 0.140 / 0.144.
+constexpr uint32_t kMaxSegs = 1024, kMinSeg = 32;
 __host__ __device__ inline uint32_t seg_bytes(uint32_t n, uint32_t nseg) {
   const uint32_t s = (n + nseg - 1) / nseg;
   return s > kMinSeg ? s : kMinSeg;
