@@ -112,7 +112,7 @@ __device__ __forceinline__ uint32_t bits_at(const uint8_t* p, uint32_t at, uint3
 // near copies a 128-byte line and 3.2 hops, 5.53 / 2.65 and 7.42 / 3.01, at level 5, 4 a line and one hop, 1.74 / 1.83 and
 // 2.44 / 2.13; four symbols at level 1, 2.4 a line, 0.92 / 2.01 and 1.36 / 2.51: so the line lies at 8.  Counters 8
 // bytes apart at level 1, 16 a line, none farther and 14 hops, 10.5 / 8.0 and 16.4 / 8.5; at level 5, where one in twelve is
-// farther and there are 0.6 hops, 0.96 / 5.5 and 1.55 / 5.9.
+// farther and there are 0.6 hops, 0.96 / 5.5 and 1.55 / 5.9.  (Others pay 1 % of this kernel and 0.5 % of the fill for it.)
 constexpr uint32_t kNearOffset = 128, kNearBytes = 16;  // more than one copy from at most 128 back in 16 bytes
 constexpr uint32_t kTokThreads = 512, kTokPer = 4, kTokTile = kTokThreads * kTokPer;
 
